@@ -3,7 +3,7 @@
 Each translation unit is compiled by nvcc for sm_103a only, in parallel, then
 linked into one shared library that exports the C ABI of include/mara_gpu.h.
 
-* plain_fp64.cu  --fmad=false: the plain FP64 path must round exactly like
+* plain_*.cu     --fmad=false: the plain FP64 path must round exactly like
                  the reference's CPU build, so no multiply-add is contracted;
 * mixed.cu       contraction on: FP32 arithmetic with explicit intrinsics;
 * every host compile uses -ffp-contract=off (the host computes the mesh
@@ -25,6 +25,10 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
           "-I" + os.path.join(HERE, "..", "include")] + ARCH
 UNITS = {
+    "plain_hydro.cu": ["--fmad=false"],
+    "plain_mhd.cu": ["--fmad=false"],
+    "plain_mhd_cool.cu": ["--fmad=false"],
+    "plain_rmhd.cu": ["--fmad=false"],
     "plain_fp64.cu": ["--fmad=false"],
     "mixed.cu": ["--fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
     "batch.cu": ["--fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],

@@ -1,0 +1,597 @@
+// plain_kernels.cuh -- the kernels of the plain FP64 path: one face-flux sweep kernel per
+// fleshed axis, then one fused update kernel per RK stage, plus the Courant
+// reduction.  Compiled with --fmad=false (see mara2_gb300/build.py) so that
+// the arithmetic rounds as the reference's CPU build does.
+//
+// Per stage (MethodOfLinesTVD::advance, SolutionSchemes.cpp:191-274):
+//   flux_kernel<axis>   MeshOperator::godunov (MeshOperator.cpp:443-525):
+//                       gather the 2s-cell stencil along the axis, intercell
+//                       flux (reconstruction + fromPrimitive x2 + Riemann),
+//                       raw flux stored per face.  Faces are those the
+//                       interior update reads: along the axis the interior
+//                       faces, across it the interior rows plus one guard row
+//                       on each side when flux CT needs transverse neighbours.
+//   update_kernel       per interior zone: CellCenteredFieldCT's flux CT on
+//                       the magnetic fluxes of the zone's six faces
+//                       (CellCenteredFieldCT.cpp:14-134), the divergence
+//                       (MeshOperator.cpp:323-381), the RK combine
+//                       (SolutionSchemes.cpp:232-235), fromConserved
+//                       (FieldOperator::recoverPrimitive, FieldOperator.cpp:
+//                       41-82) and the guard fill: boundary conditions are
+//                       copies (periodic, outflow) or mirrored copies
+//                       (reflecting) of interior zones applied axis by axis,
+//                       so every guard zone equals one interior zone (velocity
+//                       components negated on reflecting axes) and the zone
+//                       that owns a value writes all of its guard images.
+#pragma once
+
+#include "../../include/mara_gpu.h"
+#include "internal.h"
+#include "fast64.cuh"
+#include "physics_fp64.cuh"
+
+namespace mara {
+
+template <int RECON> struct ReconInfo;
+template <> struct ReconInfo<RECON_PCM> { static constexpr int S = 1; };
+template <> struct ReconInfo<RECON_PLM> { static constexpr int S = 2; };
+template <> struct ReconInfo<RECON_WENO5> { static constexpr int S = 3; };
+
+__device__ __forceinline__ void record_status(DevStatus* st, int code)
+{
+    atomicCAS(&st->code, 0, code);
+}
+
+// ---------------------------------------------------------------------------
+// The Godunov flux of one face with the general functions, written to F; the
+// cell on its right is P[base].  Returns the status of the face's states.
+template <int LAW, int RECON, int RIEMANN>
+__device__ __noinline__ int face_general(const double* P, long long sP, long long stride, double n0, double n1,
+                                         double n2, const PhysParams* __restrict__ ppp, double* F, long long sF)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ;
+    constexpr int S = ReconInfo<RECON>::S;
+    const PhysParams& pp = *ppp;
+    const double n[3] = {n0, n1, n2};
+    double PL[NQ], PR[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        double v[2 * S];
+#pragma unroll
+        for (int c = 0; c < 2 * S; ++c) v[c] = P[q * sP + (c - S) * stride];
+        if constexpr (RECON == RECON_PCM) {
+            PL[q] = v[0];
+            PR[q] = v[1];
+        } else if constexpr (RECON == RECON_PLM) {
+            PL[q] = v[1] + +1.0 * 0.5 * minmod(pp.plm_theta, v[0], v[1], v[2]);
+            PR[q] = v[2] + -1.0 * 0.5 * minmod(pp.plm_theta, v[1], v[2], v[3]);
+        } else {
+            PL[q] = weno5<true>(&v[2], pp.weno_is, pp.shenzha_A);
+            PR[q] = weno5<false>(&v[3], pp.weno_is, pp.shenzha_A);
+        }
+    }
+    StateD<NQ> L, R;
+    int e = law_prim<LAW>(pp, PL, n, L);
+    if (e == ST_OK) e = law_prim<LAW>(pp, PR, n, R);
+    if (e != ST_OK) return e;
+    double Fh[NQ];
+    if constexpr (RIEMANN == RIEMANN_HLLC) hllc<NQ>(L, R, n, Fh);
+    else hlle<NQ>(L, R, Fh);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) F[q * sF] = Fh[q];
+    return ST_OK;
+}
+
+// laws and solvers that fast64.cuh covers
+template <int LAW, int RIEMANN>
+constexpr bool HAS_FAST = LAW != LAW_RMHD && (RIEMANN == RIEMANN_HLLE || LAW == LAW_HYDRO);
+
+// The faces of one axis, each thread a run of consecutive faces along it: a
+// zone's reconstruction serves the faces on both of its sides.  Bound by the
+// FP64 pipe (fast64.cuh); a face whose operands are not ordinary goes through
+// face_general, as do all faces of the laws without a fast form (AXIS < 0,
+// the axis at run time).
+struct FaceSpace {
+    int lo[3];   // first face (right cell) and row of each axis
+    int nb[3];   // threads per axis: runs along the faces' axis, rows across it
+    int nf, run; // faces along the axis, faces per run
+    int axis;
+};
+
+template <int LAW, int RECON, int RIEMANN, int AXIS>
+__global__ void __launch_bounds__(128) flux_kernel(const double* __restrict__ P, double* __restrict__ F,
+                                                   const __grid_constant__ GridDesc G,
+                                                   const __grid_constant__ PhysParams pp,
+                                                   const __grid_constant__ fast64::Consts C,
+                                                   const __grid_constant__ FaceSpace X, DevStatus* __restrict__ st)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ;
+    constexpr int S = ReconInfo<RECON>::S;
+    if (st->code != 0 || st->done) return;
+    if (st->failures != 0) { st->halt = 1; return; }  // failures are final once the stage ended
+    // the threads of one z-slice as one index space (rows of n + 1 or n + 2
+    // faces would leave a nearly empty block per row)
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin >= (unsigned) X.nb[0] * (unsigned) X.nb[1]) return;
+    const int axis = AXIS < 0 ? X.axis : AXIS;
+    int x[3] = {(int) (lin % (unsigned) X.nb[0]), (int) (lin / (unsigned) X.nb[0]), (int) blockIdx.y};
+    const int row = axis == 0 ? x[0] : axis == 1 ? x[1] : x[2];
+    const int first = row * X.run;
+    const int count = min(X.run, X.nf - first);
+    if (axis == 0) x[0] = first;
+    else if (axis == 1) x[1] = first;
+    else x[2] = first;
+    const int i = X.lo[0] + x[0], j = X.lo[1] + x[1], k = X.lo[2] + x[2];
+    const long long stride = axis == 0 ? 1 : axis == 1 ? (long long) G.N[0] : (long long) G.N[0] * G.N[1];
+    const long long fstride = axis == 0 ? 1 : axis == 1 ? (long long) (G.N[0] + 1) : (long long) (G.N[0] + 1) * (G.N[1] + 1);
+    const double* p = P + ((long long) k * G.N[1] + j) * G.N[0] + i;  // cell on the right of the face
+    double* f = F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
+
+    if constexpr (AXIS < 0) {
+        for (int m = 0; m < count; ++m, p += stride, f += fstride) {
+            const int e = face_general<LAW, RECON, RIEMANN>(p, G.sP, stride, G.nrm[axis][0], G.nrm[axis][1],
+                                                            G.nrm[axis][2], &pp, f, G.sF);
+            if (e != ST_OK) { record_status(st, e); return; }
+        }
+    } else {
+        // PL: the right edge of the zone on the face's left; d (PLM): the
+        // scaled difference across the face; fine: one bit per zone of the
+        // stencil, set where its values are ordinary
+        double PL[NQ], d[RECON == RECON_PLM ? NQ : 1];
+        unsigned fine = 0;
+        bool ok_left = true;
+#pragma unroll
+        for (int z = -S; z < S - 1; ++z) {
+            bool o = true;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const double v = p[q * G.sP + z * stride];
+                o = o && (RECON == RECON_WENO5 ? fast64::weno_ordinary(v) : fast64::ordinary(v));
+            }
+            fine = 2 * fine + o;
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double* v = p + q * G.sP;
+            if constexpr (RECON == RECON_PCM) {
+                PL[q] = v[-stride];
+            } else if constexpr (RECON == RECON_PLM) {
+                const double a = C.theta * (v[-stride] - v[-2 * stride]);
+                d[q] = C.theta * (v[0] - v[-stride]);
+                PL[q] = v[-stride] + fast64::half_slope(a, v[0] - v[-2 * stride], d[q]);
+            } else {
+                const double w[5] = {v[-3 * stride], v[-2 * stride], v[-stride], v[0], v[stride]};
+                double left;
+                fast64::weno5_edges(C, &w[2], left, PL[q], ok_left);
+            }
+        }
+        for (int m = 0; m < count; ++m, p += stride, f += fstride) {
+            double PR[NQ], next[NQ];
+            bool ok = ok_left && C.ok, o = true;
+            ok_left = true;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const double* v = p + q * G.sP;
+                if constexpr (RECON == RECON_PCM) {
+                    PR[q] = next[q] = v[0];
+                    o = o && fast64::ordinary(v[0]);
+                } else if constexpr (RECON == RECON_PLM) {
+                    const double c = v[0], r = v[stride];
+                    const double b = C.theta * (r - c);
+                    const double h = fast64::half_slope(d[q], r - v[-stride], b);
+                    d[q] = b;
+                    PR[q] = c - h;
+                    next[q] = c + h;
+                    o = o && fast64::ordinary(r);
+                } else {
+                    const double w[5] = {v[-2 * stride], v[-stride], v[0], v[stride], v[2 * stride]};
+                    fast64::weno5_edges(C, &w[2], PR[q], next[q], ok_left);
+                    o = o && fast64::weno_ordinary(w[4]);
+                }
+            }
+            fine = 2 * fine + o;
+            ok = ok && ok_left && (fine & ((1u << 2 * S) - 1u)) == (1u << 2 * S) - 1u;
+            fast64::Side<NQ> L, R;
+            double Fh[NQ];
+            fast64::side<LAW, AXIS>(C, PL, L, ok);
+            fast64::side<LAW, AXIS>(C, PR, R, ok);
+            if constexpr (RIEMANN == RIEMANN_HLLC) fast64::hllc<AXIS>(C, PL, PR, L, R, Fh, ok);
+            else fast64::hlle<NQ>(L, R, Fh, ok);
+            if (ok) {
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) f[q * G.sF] = Fh[q];
+            } else {
+                const int e = face_general<LAW, RECON, RIEMANN>(p, G.sP, stride, G.nrm[AXIS][0], G.nrm[AXIS][1],
+                                                                G.nrm[AXIS][2], &pp, f, G.sF);
+                if (e != ST_OK) { record_status(st, e); return; }
+            }
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) PL[q] = next[q];
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+struct FluxView {
+    const double* F[3];
+    long long sF;
+    int M0, M1; // (N0+1), (N1+1)
+    __device__ __forceinline__ double at(int a, int q, int i, int j, int k) const
+    {
+        return F[a][q * sF + ((long long) k * M1 + j) * M0 + i];
+    }
+};
+
+// x 2^k, on the exponent where x and the result are normal
+__device__ __forceinline__ double times_pow2(double x, int k)
+{
+    const unsigned e = fast64::expo(x);
+    if (e - 1u < 2046u && e + (unsigned) k - 1u < 2046u)
+        return fast64::from_bits(fast64::bits(x) + ((unsigned long long) (long long) k << 52));
+    return fast64::is_zero(x) ? x : x * (k == 1 ? 2.0 : k == -1 ? 0.5 : k == -2 ? 0.25 : 0.125);
+}
+
+// Flux of field q through the face of axis a at flux index (i, j, k), after
+// CellCenteredFieldCT::correctGodunovFluxes when ct is on (magnetic index 5):
+// 1/8 of (2 F + ...), its powers of two on the exponents.
+template <int NQ>
+__device__ __forceinline__ double face_flux(const FluxView& V, const GridDesc& G, int a, int q, int i, int j, int k)
+{
+    if ((NQ == 8 || NQ == 9) && G.ct && q >= 5 && q <= 7) {
+        const int B0 = 5, B1 = 6, B2 = 7;
+        const bool fx = G.n[0] > 1, fy = G.n[1] > 1, fz = G.n[2] > 1;
+        if (a == 0) {
+            if (q == B0) return 0.0;
+            if (q == B1 && fy)
+                return times_pow2(times_pow2(V.at(0, B1, i, j, k), 1) + V.at(0, B1, i, j + 1, k) + V.at(0, B1, i, j - 1, k)
+                                - V.at(1, B0, i, j + 1, k) - V.at(1, B0, i - 1, j + 1, k)
+                                - V.at(1, B0, i, j, k) - V.at(1, B0, i - 1, j, k), -3);
+            if (q == B2 && fz)
+                return times_pow2(times_pow2(V.at(0, B2, i, j, k), 1) + V.at(0, B2, i, j, k + 1) + V.at(0, B2, i, j, k - 1)
+                                - V.at(2, B0, i, j, k + 1) - V.at(2, B0, i - 1, j, k + 1)
+                                - V.at(2, B0, i, j, k) - V.at(2, B0, i - 1, j, k), -3);
+        } else if (a == 1) {
+            if (q == B1) return 0.0;
+            if (q == B2 && fz)
+                return times_pow2(times_pow2(V.at(1, B2, i, j, k), 1) + V.at(1, B2, i, j, k + 1) + V.at(1, B2, i, j, k - 1)
+                                - V.at(2, B1, i, j, k + 1) - V.at(2, B1, i, j - 1, k + 1)
+                                - V.at(2, B1, i, j, k) - V.at(2, B1, i, j - 1, k), -3);
+            if (q == B0 && fx)
+                return times_pow2(times_pow2(V.at(1, B0, i, j, k), 1) + V.at(1, B0, i + 1, j, k) + V.at(1, B0, i - 1, j, k)
+                                - V.at(0, B1, i + 1, j, k) - V.at(0, B1, i + 1, j - 1, k)
+                                - V.at(0, B1, i, j, k) - V.at(0, B1, i, j - 1, k), -3);
+        } else {
+            if (q == B2) return 0.0;
+            if (q == B0 && fx)
+                return times_pow2(times_pow2(V.at(2, B0, i, j, k), 1) + V.at(2, B0, i + 1, j, k) + V.at(2, B0, i - 1, j, k)
+                                - V.at(0, B2, i + 1, j, k) - V.at(0, B2, i + 1, j, k - 1)
+                                - V.at(0, B2, i, j, k) - V.at(0, B2, i, j, k - 1), -3);
+            if (q == B1 && fy)
+                return times_pow2(times_pow2(V.at(2, B1, i, j, k), 1) + V.at(2, B1, i, j + 1, k) + V.at(2, B1, i, j - 1, k)
+                                - V.at(1, B2, i, j + 1, k) - V.at(1, B2, i, j + 1, k - 1)
+                                - V.at(1, B2, i, j, k) - V.at(1, B2, i, j, k - 1), -3);
+        }
+    }
+    return V.at(a, q, i, j, k);
+}
+
+// One RK stage's update of a zone (see the file's comment).  Bound by the
+// FP64 pipe, so the face area products of flat axes (zeros) are left out, and
+// the RK weights 1, 1/2 and 1/4 act on exponents; b1, b2: the weights of U0
+// and of the stage's result.
+template <int LAW>
+__global__ void __launch_bounds__(128) update_kernel(const double* __restrict__ Pin, double* __restrict__ Pout,
+                                                     double* __restrict__ U0, double* __restrict__ U,
+                                                     const __grid_constant__ FluxView V,
+                                                     const __grid_constant__ GridDesc G,
+                                                     const __grid_constant__ PhysParams pp,
+                                                     const __grid_constant__ fast64::Consts C, double fv, double b,
+                                                     int stage, const double* __restrict__ dtp,
+                                                     DevStatus* __restrict__ st, const double* __restrict__ S)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ;
+    if (st->code != 0 || st->halt || st->done) return;
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin >= (unsigned) G.n[0] * (unsigned) G.n[1]) return;
+    const int ii = (int) (lin % (unsigned) G.n[0]), jj = (int) (lin / (unsigned) G.n[0]), kk = blockIdx.y;
+    const int i = ii + G.g[0], j = jj + G.g[1], k = kk + G.g[2];
+    const long long pc = ((long long) k * G.N[1] + j) * G.N[0] + i;
+    const long long uc = ((long long) kk * G.n[1] + jj) * G.n[0] + ii;
+    const double dt = *dtp;
+    const bool fx = G.n[0] > 1, fy = G.n[1] > 1, fz = G.n[2] > 1;
+
+    double Pc[NQ], Uo[NQ], Up[NQ], Un[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) Pc[q] = Pin[q * G.sP + pc];
+
+    if (stage == 0) {
+        bool ok = C.ok && LAW != LAW_RMHD;
+        if constexpr (LAW != LAW_RMHD) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary(Pc[q]);
+            fast64::p2u<LAW>(C, Pc, Uo, ok);
+        }
+        if (!ok) {
+            const int e = law_p2u<LAW>(pp, Pc, Uo);
+            if (e != ST_OK) { record_status(st, e); return; }
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) { U0[q * G.sU + uc] = Uo[q]; Up[q] = Uo[q]; }
+    } else {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) { Uo[q] = U0[q * G.sU + uc]; Up[q] = U[q * G.sU + uc]; }
+    }
+
+    const int pow2 = b == 1.0 ? 0 : b == 0.5 ? -1 : b == 0.25 ? -2 : 1;   // b 's exponent, 1: not a power of two
+    bool fine = C.ok;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        // the sum over the faces in the reference's order; a flat axis adds
+        // and subtracts a zero, which only makes a -0 a +0
+        double sum = 0.0;
+        if (fx) sum = face_flux<NQ>(V, G, 0, q, i + 1, j, k) * G.dA[0] - face_flux<NQ>(V, G, 0, q, i, j, k) * G.dA[0];
+        if (fy) sum = sum + face_flux<NQ>(V, G, 1, q, i, j + 1, k) * G.dA[1] - face_flux<NQ>(V, G, 1, q, i, j, k) * G.dA[1];
+        else sum = fast64::add_zero(sum, false);
+        if (fz) sum = sum + face_flux<NQ>(V, G, 2, q, i, j, k + 1) * G.dA[2] - face_flux<NQ>(V, G, 2, q, i, j, k) * G.dA[2];
+        else sum = fast64::add_zero(sum, false);
+        double L = fv * sum;
+        if constexpr (LAW == LAW_MHD_COOL) {
+            // NewtonianMHD::addSourceTerms (ConservationLaws.cpp:489-501)
+            if (q == 4) L -= Pc[4] / (pp.gamma - 1.0) * pp.cooling_rate;
+            if (q == 8) L += Pc[4] / (pp.gamma - 1.0) * pp.cooling_rate;
+        }
+        if (S) L += S[q * G.sP + pc];  // the source terms function's array (SolutionSchemes.cpp:219-228)
+        const double X = Up[q] + dt * L;
+        if (pow2 == 0) {
+            // U0 0 + X: a zero plus X (NaN for an infinite U0)
+            Un[q] = fast64::expo(Uo[q]) == 0x7ffu ? Uo[q] * (1 - b) + X : fast64::add_zero(X, fast64::sign_bit(Uo[q]));
+        } else if (pow2 < 0) {
+            Un[q] = (pow2 == -1 ? times_pow2(Uo[q], -1) : Uo[q] * (1 - b)) + times_pow2(X, pow2);
+        } else {
+            Un[q] = Uo[q] * (1 - b) + X * b;
+        }
+        U[q * G.sU + uc] = Un[q];
+        fine = fine && fast64::ordinary(Un[q]);
+    }
+
+    double Pn[NQ];
+    if constexpr (LAW != LAW_RMHD) fast64::cons<LAW>(C, Un, Pn, fine);
+    else fine = false;
+    if (!fine) {
+        int code = ST_OK;
+        const int e = law_cons<LAW>(pp, Un, Pn, &code);
+        if (e == ST_INVERSION_FAILURE) {
+            atomicAdd(&st->failures, 1);
+            const unsigned long long z = (unsigned long long) uc;
+            const unsigned long long prev = atomicMin(&st->first_zone, z);
+            if (z < prev) atomicExch(&st->first_code, code);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) Pn[q] = Pc[q]; // a failed zone keeps its value
+        } else if (e != ST_OK) {
+            record_status(st, e);
+            return;
+        }
+    }
+
+    // the zone's cell, then (zones within a guard width of an edge) its guard
+    // images on every combination of axes
+    for (int c = 0; c <= G.g[2]; ++c) {
+        int oz, sz;
+        if (!guard_image(c, kk, G.n[2], G.g[2], G.bc, oz, sz)) continue;
+        for (int bb = 0; bb <= G.g[1]; ++bb) {
+            int oy, sy;
+            if (!guard_image(bb, jj, G.n[1], G.g[1], G.bc, oy, sy)) continue;
+            for (int a = 0; a <= G.g[0]; ++a) {
+                int ox, sx;
+                if (!guard_image(a, ii, G.n[0], G.g[0], G.bc, ox, sx)) continue;
+                const long long o = ((long long) oz * G.N[1] + oy) * G.N[0] + ox;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    double v = Pn[q];
+                    if ((q == 1 && sx) || (q == 2 && sy) || (q == 3 && sz)) v *= -1;
+                    Pout[q * G.sP + o] = v;
+                }
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FieldOperator::getCourantTimestep: min over interior zones of
+// lmin / max_direction(maxEigenvalueMagnitude).  Positive doubles order like
+// their bit patterns, so the minimum is an atomicMin on the bits; NaN and
+// +inf (bit patterns above DBL_MAX) never win, as in the reference's
+// "if (dt < courantTimestep)" starting from DBL_MAX.
+// lmin / lambda falls with lambda, also after rounding, so a block divides
+// once, by its largest eigenvalue.
+template <int LAW>
+__global__ void __launch_bounds__(128) courant_kernel(const double* __restrict__ P,
+                                                      const __grid_constant__ GridDesc G,
+                                                      const __grid_constant__ PhysParams pp,
+                                                      const __grid_constant__ fast64::Consts C,
+                                                      DevStatus* __restrict__ st)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ;
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long mine = 0;
+    if (lin < (unsigned) G.n[0] * (unsigned) G.n[1] && st->code == 0) {
+        const int ii = (int) (lin % (unsigned) G.n[0]), jj = (int) (lin / (unsigned) G.n[0]), kk = blockIdx.y;
+        const long long pc = ((long long) (kk + G.g[2]) * G.N[1] + (jj + G.g[1])) * G.N[0] + (ii + G.g[0]);
+        double Pc[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) Pc[q] = P[q * G.sP + pc];
+        double lmax = 0.0;
+        bool ok = C.ok && LAW != LAW_RMHD;
+        if constexpr (LAW != LAW_RMHD) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary(Pc[q]);
+            lmax = fast64::fastest<LAW>(C, Pc, ok);
+        }
+        if (!ok) {
+            double lam[3];
+            int e = ST_OK;
+            for (int a = 0; a < 3 && e == ST_OK; ++a) {
+                StateD<NQ> S;
+                e = law_prim<LAW>(pp, Pc, G.nrm[a], S);
+                lam[a] = max_eigen_magnitude<NQ>(S.A);
+            }
+            if (e != ST_OK) {
+                record_status(st, e);
+                lmax = 0.0;
+            } else {
+                lmax = lam[0];
+                if (lmax < lam[1]) lmax = lam[1];
+                if (lmax < lam[2]) lmax = lam[2];
+            }
+        }
+        mine = (unsigned long long) __double_as_longlong(lmax);
+    }
+    // warp then block maximum
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_down_sync(0xffffffffu, mine, off);
+        mine = o > mine ? o : mine;
+    }
+    __shared__ unsigned long long red[4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0) red[w] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int m = 1; m < (int) (blockDim.x >> 5); ++m) mine = red[m] > mine ? red[m] : mine;
+        const double dt = G.lmin / __longlong_as_double((long long) mine);
+        if (dt < 1.7976931348623157e308) atomicMin(&st->dt_bits, (unsigned long long) __double_as_longlong(dt));
+    }
+}
+
+// ---------------------------------------------------------------------------
+static PhysParams to_dev(const PhysParamsH& h)
+{
+    PhysParams p;
+    p.gamma = h.gamma;
+    p.plm_theta = h.plm_theta;
+    p.shenzha_A = h.shenzha_A;
+    p.pressure_floor = h.pressure_floor;
+    p.weno_is = h.weno_is;
+    p.cooling_rate = h.cooling_rate;
+    return p;
+}
+
+static fast64::Consts to_fast(const PhysParamsH& h, const GridDesc& G)
+{
+    fast64::Consts c;
+    c.ok = true;
+    c.gamma = h.gamma;
+    c.gm1 = h.gamma - 1.0;
+    c.theta = h.plm_theta;
+    c.shenzha_A = h.shenzha_A;
+    c.weno_is = h.weno_is;
+    c.ny0 = G.nrm[1][0];
+    c.gm1_div = ieee64::divisor(c.gm1, c.ok);
+    // ordinary constants, the normals that fast64.cuh assumes
+    const double small = 1e-3, large = 1e3;
+    c.ok = c.ok && c.gamma > small && c.gamma < large && c.gm1 > small && c.theta > small && c.theta < large &&
+           c.shenzha_A >= 0.0 && c.shenzha_A < 1e9 && c.ny0 > 1e-20 && c.ny0 < small;
+    for (int a = 0; a < 3; ++a)
+        for (int d = 0; d < 3; ++d)
+            if (!(a == 1 && d == 0)) c.ok = c.ok && G.nrm[a][d] == (a == d ? 1.0 : 0.0);
+    return c;
+}
+
+// Threads per block: few warps are spread over the SMs' schedulers, each of
+// which has its own half lane of FP64 per clock.
+static int block_size(long long threads) { return threads <= 152ll * 4 * 32 ? 32 : 128; }
+
+template <int LAW, int RECON, int RIEMANN>
+static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
+                        double* F, DevStatus* st, cudaStream_t s)
+{
+    // faces along the axis: the interior faces; across: interior rows, plus
+    // one guard row per side on fleshed axes when flux CT is on
+    FaceSpace X;
+    long long faces = 1;
+    for (int a = 0; a < 3; ++a) {
+        if (a == axis) { X.lo[a] = G.g[a]; X.nb[a] = G.n[a] + 1; }
+        else if (G.n[a] > 1) { const int e = G.ct ? 1 : 0; X.lo[a] = G.g[a] - e; X.nb[a] = G.n[a] + 2 * e; }
+        else { X.lo[a] = 0; X.nb[a] = 1; }
+        faces *= X.nb[a];
+    }
+    // runs as long as 16 warps per SM remain: a run of one forms every
+    // zone's reconstruction twice, one of eight 1/8 too many
+    const long long want = 152ll * 512;
+    X.nf = X.nb[axis];
+    X.run = HAS_FAST<LAW, RIEMANN> && RECON != RECON_PCM ? (int) (faces / want < 1 ? 1 : faces / want > 8 ? 8 : faces / want) : 1;
+    X.nb[axis] = (X.nf + X.run - 1) / X.run;
+    const long long slice = (long long) X.nb[0] * X.nb[1];
+    const int block = block_size(slice * X.nb[2]);
+    const dim3 grid((unsigned) ((slice + block - 1) / block), X.nb[2]);
+    X.axis = axis;
+    if constexpr (!HAS_FAST<LAW, RIEMANN>) {
+        flux_kernel<LAW, RECON, RIEMANN, -1><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st);
+    } else {
+        switch (axis) {
+            case 0: flux_kernel<LAW, RECON, RIEMANN, 0><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
+            case 1: flux_kernel<LAW, RECON, RIEMANN, 1><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
+            default: flux_kernel<LAW, RECON, RIEMANN, 2><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
+        }
+    }
+}
+
+template <int LAW, int RECON>
+static void flux_dispatch_r(int riemann, int axis, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C,
+                            const double* P, double* F, DevStatus* st, cudaStream_t s)
+{
+    if (riemann == RIEMANN_HLLC) flux_launch<LAW, RECON, RIEMANN_HLLC>(axis, G, pp, C, P, F, st, s);
+    else flux_launch<LAW, RECON, RIEMANN_HLLE>(axis, G, pp, C, P, F, st, s);
+}
+
+template <int LAW>
+void plain_flux_law(int recon, int riemann, int axis, const GridDesc& G, const PhysParamsH& ph, const double* P,
+                    double* F, DevStatus* st, cudaStream_t s)
+{
+    const PhysParams pp = to_dev(ph);
+    const fast64::Consts C = to_fast(ph, G);
+    switch (recon) {
+        case RECON_PCM: flux_dispatch_r<LAW, RECON_PCM>(riemann, axis, G, pp, C, P, F, st, s); break;
+        case RECON_PLM: flux_dispatch_r<LAW, RECON_PLM>(riemann, axis, G, pp, C, P, F, st, s); break;
+        default: flux_dispatch_r<LAW, RECON_WENO5>(riemann, axis, G, pp, C, P, F, st, s); break;
+    }
+}
+
+template <int LAW>
+void plain_update_law(const GridDesc& G, const PhysParamsH& ph, const double* Pin, double* Pout, double* U0, double* U,
+                      const double* Fx, const double* Fy, const double* Fz, double b, int stage, const double* dt,
+                      DevStatus* st, cudaStream_t s, const double* S)
+{
+    FluxView V;
+    V.F[0] = Fx; V.F[1] = Fy; V.F[2] = Fz;
+    V.sF = G.sF;
+    V.M0 = G.N[0] + 1;
+    V.M1 = G.N[1] + 1;
+    const double factor = -1.0;
+    const long long slice = (long long) G.n[0] * G.n[1];
+    const int block = block_size(slice * G.n[2]);
+    const dim3 grid((unsigned) ((slice + block - 1) / block), G.n[2]);
+    update_kernel<LAW><<<grid, block, 0, s>>>(Pin, Pout, U0, U, V, G, to_dev(ph), to_fast(ph, G), factor / G.dV, b,
+                                              stage, dt, st, S);
+}
+
+template <int LAW>
+void plain_courant_law(const GridDesc& G, const PhysParamsH& ph, const double* P, DevStatus* st, cudaStream_t s)
+{
+    const long long slice = (long long) G.n[0] * G.n[1];
+    const int block = block_size(slice * G.n[2]);
+    const dim3 grid((unsigned) ((slice + block - 1) / block), G.n[2]);
+    courant_kernel<LAW><<<grid, block, 0, s>>>(P, G, to_dev(ph), to_fast(ph, G), st);
+}
+
+// one translation unit per law instantiates the kernels (plain_*.cu)
+#define MARA_PLAIN_LAW(EXTERN, LAW)                                                                                  \
+    EXTERN template void plain_flux_law<LAW>(int, int, int, const GridDesc&, const PhysParamsH&, const double*,      \
+                                             double*, DevStatus*, cudaStream_t);                                    \
+    EXTERN template void plain_update_law<LAW>(const GridDesc&, const PhysParamsH&, const double*, double*, double*, \
+                                               double*, const double*, const double*, const double*, double, int,   \
+                                               const double*, DevStatus*, cudaStream_t, const double*);             \
+    EXTERN template void plain_courant_law<LAW>(const GridDesc&, const PhysParamsH&, const double*, DevStatus*,      \
+                                                cudaStream_t)
+
+} // namespace mara
