@@ -6,8 +6,11 @@
 // elsewhere).  The functions here return the bits of their counterparts in
 // physics_fp64.cuh (which name the reference's routines) from a third of the
 // FP64 operations:
-//  * divisions and square roots in integers (ieee64.cuh), those by one divisor
-//    sharing its reciprocal;
+//  * divisions, square roots and most products in integers (ieee64.cuh), the
+//    divisions by one divisor sharing its reciprocal: written mul(a, b) and
+//    div(a, b).  a * b stays on the FP64 pipe: the split between the two is
+//    flat (all products in integers against two thirds: within 1 % on KH
+//    1024^2 and MHD 64x56x48, 4 % for the latter on a 1024-zone tube);
 //  * each zone's slopes once, for the faces on both of its sides;
 //  * multiplications by powers of two on the exponent, comparisons on the bit
 //    patterns;
@@ -16,9 +19,8 @@
 //    The y normal keeps its x component cos(pi/2) = 6.1e-17;
 //  * eigenvalues only where they can be the largest or the smallest: rounding
 //    is monotone, so e.g. max(vn - c, vn, vn + c) is RN(vn + c).
-// They hold for ordinary operands: zero or of magnitude 2^-300 to 2^200
-// (ordinary()), positive densities and pressures, no division by zero.
-// Anything else clears `ok`, and the caller repeats the face or zone with the
+// They hold for ordinary operands (ordinary(), ordinary_pos()) and where no
+// divisor vanishes.  Anything else clears `ok`, and the caller repeats the face or zone with the
 // general functions, so NaNs, infinities and error codes stay theirs.
 #pragma once
 
@@ -43,11 +45,22 @@ F64_FN bool is_zero(double x) { return (bits(x) << 1) == 0; }
 F64_FN bool sign_bit(double x) { return (bits(x) >> 63) != 0; }
 F64_FN u32 expo(double x) { return (u32) (bits(x) >> 52) & 0x7ffu; }
 
-// zero, or of magnitude 2^-300 .. 2^201: products and quotients of a few of
-// these stay far inside the normal range, and so do their non-zero differences
-F64_FN bool ordinary(double x) { return expo(x) - 723u <= 500u || is_zero(x); }
+// Ordinary operands: a density or pressure of 2^-100 to 2^101, another field
+// zero or of magnitude 2^-330 to 2^101.  An edge value then is at least
+// 2^-153 and 2^-383 (or zero), and the products that the functions below form
+// without a check stay normal: the smallest is rho v v above 2^-920.
+F64_FN bool ordinary_pos(double x) { return (u32) (bits(x) >> 32) - (923u << 20) <= (200u << 20); }
+F64_FN bool ordinary(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (693u << 20) <= (430u << 20) || is_zero(x); }
+// field q of a primitive (or conserved: density and energy) state
+F64_FN bool ordinary_field(int q, double x) { return q == 0 || q == 4 ? ordinary_pos(x) : ordinary(x); }
+// a reconstructed density or pressure
+F64_FN bool edge_pos(double x) { return (u32) (bits(x) >> 32) - (869u << 20) <= (256u << 20); }
 
-// x 2^k for ordinary x (and what ordinary values were combined to)
+using ieee64::mul;
+using ieee64::div;
+using ieee64::sqrt_rn;
+
+// x 2^k for x zero or well inside the normal range
 F64_FN double scale(double x, int k)
 {
     return is_zero(x) ? x : from_bits(bits(x) + ((u64) (ieee64::i64) k << 52));
@@ -95,9 +108,8 @@ F64_FN double half_slope(double a, double rl, double d)
     return from_bits((same && m != 0 ? m - (1ull << 52) : 0ull) | neg);
 }
 
-// weno5 at both edges of a zone, from v[-2 .. 2] of magnitude below 2^61: the
-// smoothness indicators and the products that both edges use once
-F64_FN bool weno_ordinary(double x) { return expo(x) - 723u <= 360u || is_zero(x); }
+// weno5 at both edges of a zone, from ordinary v[-2 .. 2]: the smoothness
+// indicators and the products that both edges use once
 
 F64_FN double sq(double x) { return x * x; }
 
@@ -112,9 +124,9 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
     if (c.weno_is == WENO_BORGES08) {
         const double eps = 1e-14;
         const double tau5 = fabs(B0 - B2);
-        const double r0 = 1.0 + ieee64::div(tau5, B0 + eps, ok);
-        const double r1 = 1.0 + ieee64::div(tau5, B1 + eps, ok);
-        const double r2 = 1.0 + ieee64::div(tau5, B2 + eps, ok);
+        const double r0 = 1.0 + div(tau5, B0 + eps, ok);
+        const double r1 = 1.0 + div(tau5, B1 + eps, ok);
+        const double r2 = 1.0 + div(tau5, B2 + eps, ok);
         wr[0] = 0.3 * r0; wr[1] = 0.6 * r1; wr[2] = 0.1 * r2;
         wl[0] = 0.1 * r0; wl[1] = wr[1]; wl[2] = 0.3 * r2;
     } else {
@@ -123,7 +135,7 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
             ep = 1e-10;
             const double lo = bits(B0) < bits(B1) ? (bits(B0) < bits(B2) ? B0 : B2) : (bits(B1) < bits(B2) ? B1 : B2);
             const double hi = max_pos(max_pos(B0, B1), B2);
-            const double add = ieee64::div(lo, hi + ep, ok) * c.shenzha_A * lo;
+            const double add = div(lo, hi + ep, ok) * c.shenzha_A * lo;
             B0 = add + B0;
             B1 = add + B1;
             B2 = add + B2;
@@ -131,8 +143,8 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
         const Divisor e0 = ieee64::divisor(sq(ep + B0), ok);
         const Divisor e1 = ieee64::divisor(sq(ep + B1), ok);
         const Divisor e2 = ieee64::divisor(sq(ep + B2), ok);
-        wr[0] = ieee64::div(0.3, e0, ok); wr[1] = ieee64::div(0.6, e1, ok); wr[2] = ieee64::div(0.1, e2, ok);
-        wl[0] = ieee64::div(0.1, e0, ok); wl[1] = wr[1]; wl[2] = ieee64::div(0.3, e2, ok);
+        wr[0] = div(0.3, e0, ok); wr[1] = div(0.6, e1, ok); wr[2] = div(0.1, e2, ok);
+        wl[0] = div(0.1, e0, ok); wl[1] = wr[1]; wl[2] = div(0.3, e2, ok);
     }
     const double third = 1. / 3., sixth = 1. / 6., a56 = 5. / 6., a76 = 7. / 6., a116 = 11. / 6.;
     const double r0 = third * v[0] + a56 * v[1] - sixth * v[2];
@@ -141,8 +153,8 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
     const double l0 = a116 * v[0] - a76 * v[1] + third * v[2];
     const double l1 = third * v[-1] + a56 * v[0] - sixth * v[1];
     const double l2 = -sixth * v[-2] + a56 * v[-1] + third * v[0];
-    right = ieee64::div(wr[0] * r0 + wr[1] * r1 + wr[2] * r2, wr[0] + wr[1] + wr[2], ok);
-    left = ieee64::div(wl[0] * l0 + wl[1] * l1 + wl[2] * l2, wl[0] + wl[1] + wl[2], ok);
+    right = div(wr[0] * r0 + wr[1] * r1 + wr[2] * r2, wr[0] + wr[1] + wr[2], ok);
+    left = div(wl[0] * l0 + wl[1] * l1 + wl[2] * l2, wl[0] + wl[1] + wl[2], ok);
 }
 
 // ---------------------------------------------------------------------------
@@ -150,7 +162,7 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
 template <int AXIS>
 F64_FN double along(const Consts& c, double x, double y, double z)
 {
-    if constexpr (AXIS == 1) return add_zero(x * c.ny0 + y, sign_bit(z));
+    if constexpr (AXIS == 1) return add_zero(mul(x, c.ny0) + y, sign_bit(z));
     const double v = AXIS == 0 ? x : z;
     return is_zero(v) ? from_bits(bits(x) & bits(y) & bits(z) & SIGN) : v;
 }
@@ -160,7 +172,7 @@ template <int AXIS>
 F64_FN double add_normal(const Consts& c, int d, double x, double p)
 {
     if (d == AXIS) return x + p;
-    if (AXIS == 1 && d == 0) return x + p * c.ny0;
+    if (AXIS == 1 && d == 0) return x + mul(p, c.ny0);
     return add_zero(x, sign_bit(p));
 }
 
@@ -169,7 +181,7 @@ F64_FN double add_normal(const Consts& c, int d, double x, double p)
 template <int AXIS>
 F64_FN double times_along(double vn, double x, double x_times_axis)
 {
-    if constexpr (AXIS == 1) return vn * x;
+    if constexpr (AXIS == 1) return mul(vn, x);
     return is_zero(vn) ? from_bits((bits(vn) ^ bits(x)) & SIGN) : x_times_axis;
 }
 
@@ -180,52 +192,59 @@ template <int NQ> struct Side {
     double vn, ap, am;
 };
 
+F64_FN double dot(double a, double b, double c, double x, double y, double z)
+{
+    return a * x + b * y + c * z;
+}
+
 // hydro_prim
 template <int AXIS>
 F64_FN void hydro_side(const Consts& c, const double* P, Side<5>& S, bool& ok)
 {
-    const double cs = ieee64::sqrt_rn(ieee64::div(c.gamma * P[4], P[0], ok), ok);
-    const double vv = P[1] * P[1] + P[2] * P[2] + P[3] * P[3];
+    ok = ok && edge_pos(P[0]) && edge_pos(P[4]);
+    const double cs = sqrt_rn(div(mul(c.gamma, P[4]), P[0], ok), ok);
+    const double vv = dot(P[1], P[2], P[3], P[1], P[2], P[3]);
     const double vn = along<AXIS>(c, P[1], P[2], P[3]);
     S.vn = vn;
     S.U[0] = P[0];
-    S.U[1] = P[0] * P[1];
-    S.U[2] = P[0] * P[2];
-    S.U[3] = P[0] * P[3];
-    S.U[4] = half(P[0] * vv) + ieee64::div(P[4], c.gm1_div, ok);
+    S.U[1] = mul(P[0], P[1]);
+    S.U[2] = mul(P[0], P[2]);
+    S.U[3] = mul(P[0], P[3]);
+    S.U[4] = half(mul(P[0], vv)) + div(P[4], c.gm1_div, ok);
     S.F[0] = times_along<AXIS>(vn, S.U[0], S.U[1 + AXIS]);
-    S.F[1] = add_normal<AXIS>(c, 0, vn * S.U[1], P[4]);
-    S.F[2] = add_normal<AXIS>(c, 1, vn * S.U[2], P[4]);
-    S.F[3] = add_normal<AXIS>(c, 2, vn * S.U[3], P[4]);
-    S.F[4] = vn * S.U[4] + P[4] * vn;
+    S.F[1] = add_normal<AXIS>(c, 0, mul(vn, S.U[1]), P[4]);
+    S.F[2] = add_normal<AXIS>(c, 1, mul(vn, S.U[2]), P[4]);
+    S.F[3] = add_normal<AXIS>(c, 2, mul(vn, S.U[3]), P[4]);
+    S.F[4] = mul(vn, S.U[4]) + mul(P[4], vn);
     S.ap = clamp_pos(vn + cs);
     S.am = clamp_neg(vn - cs);
-    ok = ok && !is_zero(cs);
 }
 
 // mhd_prim; an auxiliary field (index 8) is carried without a flux
 template <int AXIS, int NQ>
 F64_FN void mhd_side(const Consts& c, const double* P, Side<NQ>& S, bool& ok)
 {
+    ok = ok && edge_pos(P[0]) && edge_pos(P[4]);
     const Divisor rho = ieee64::divisor(P[0], ok);
-    const double cs2 = ieee64::div(c.gamma * P[4], rho, ok);
-    const double vv = P[1] * P[1] + P[2] * P[2] + P[3] * P[3];
-    const double BB = P[5] * P[5] + P[6] * P[6] + P[7] * P[7];
-    const double Bv = P[5] * P[1] + P[6] * P[2] + P[7] * P[3];
+    const double cs2 = div(mul(c.gamma, P[4]), rho, ok);
+    const double vv = dot(P[1], P[2], P[3], P[1], P[2], P[3]);
+    const double BB = dot(P[5], P[6], P[7], P[5], P[6], P[7]);
+    const double Bv = dot(P[5], P[6], P[7], P[1], P[2], P[3]);
     const double vn = along<AXIS>(c, P[1], P[2], P[3]);
     const double Bn = along<AXIS>(c, P[5], P[6], P[7]);
     const double ps = P[4] + half(BB);
     S.vn = vn;
     S.U[0] = P[0];
 #pragma unroll
-    for (int d = 1; d < 4; ++d) S.U[d] = P[0] * P[d];
-    S.U[4] = half(P[0] * vv) + half(BB) + ieee64::div(P[4], c.gm1_div, ok);
+    for (int d = 1; d < 4; ++d) S.U[d] = mul(P[0], P[d]);
+    S.U[4] = half(mul(P[0], vv)) + half(BB) + div(P[4], c.gm1_div, ok);
 #pragma unroll
     for (int d = 5; d < NQ; ++d) S.U[d] = P[d];
     S.F[0] = times_along<AXIS>(vn, S.U[0], S.U[1 + AXIS]);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) S.F[1 + d] = add_normal<AXIS>(c, d, vn * S.U[1 + d] - Bn * P[5 + d], ps);
-    S.F[4] = vn * S.U[4] - Bn * Bv + ps * vn;
+    for (int d = 0; d < 3; ++d)
+        S.F[1 + d] = add_normal<AXIS>(c, d, mul(vn, S.U[1 + d]) - mul(Bn, P[5 + d]), ps);
+    S.F[4] = mul(vn, S.U[4]) - Bn * Bv + mul(ps, vn);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         if (AXIS != 1 && d == AXIS) {
@@ -234,19 +253,18 @@ F64_FN void mhd_side(const Consts& c, const double* P, Side<NQ>& S, bool& ok)
             const bool p = sign_bit(vn) != sign_bit(P[5 + d]), q = sign_bit(Bn) != sign_bit(P[1 + d]);
             S.F[5 + d] = from_bits(zero && p && !q ? SIGN : 0ull);
         } else {
-            S.F[5 + d] = vn * S.U[5 + d] - Bn * P[1 + d];
+            S.F[5 + d] = mul(vn, S.U[5 + d]) - mul(Bn, P[1 + d]);
         }
     }
     if constexpr (NQ > 8) S.F[8] = 0.0;
     // the fast speed; an Alfven speed that rounding puts above it wins
-    const double ca2 = ieee64::div(BB, rho, ok);
-    const double cn2 = ieee64::div(Bn * Bn, rho, ok);
+    const double ca2 = div(BB, rho, ok);
+    const double cn2 = div(mul(Bn, Bn), rho, ok);
     const double s = cs2 + ca2;
-    const double cF2 = half(s + ieee64::sqrt_rn(s * s - scale(cs2 * cn2, 2), ok));
-    const double cf = ieee64::sqrt_rn(max_pos(cF2, cn2), ok);
+    const double cF2 = half(s + sqrt_rn(mul(s, s) - scale(cs2, 2) * cn2, ok));
+    const double cf = sqrt_rn(max_pos(cF2, cn2), ok);
     S.ap = clamp_pos(vn + cf);
     S.am = clamp_neg(vn - cf);
-    ok = ok && !is_zero(cf) && !sign_bit(P[4]);
 }
 
 template <int LAW, int AXIS>
@@ -262,10 +280,10 @@ F64_FN void hlle(const Side<NQ>& L, const Side<NQ>& R, double* F, bool& ok)
 {
     const double ap = max_pos(L.ap, R.ap), am = min_neg(L.am, R.am);
     const Divisor den = ieee64::divisor(ap - am, ok);
-    const double apam = ap * am;
+    const double apam = mul(ap, am, ok);
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
-        F[q] = ieee64::div(ap * L.F[q] - am * R.F[q] + apam * (R.U[q] - L.U[q]), den, ok);
+        F[q] = div(ap * L.F[q] - am * R.F[q] + apam * (R.U[q] - L.U[q]), den, ok);
 }
 
 // the star state of the side the contact moves away from, chosen first
@@ -275,8 +293,8 @@ F64_FN void hllc(const Consts& c, const double* Pl, const double* Pr, const Side
 {
     const double ap = max_pos(L.ap, R.ap), am = min_neg(L.am, R.am);
     const double sl = am - L.vn, sr = ap - R.vn;
-    const double ml = Pl[0] * sl, mr = Pr[0] * sr;
-    const double lc = ieee64::div((Pr[4] - R.F[0] * sr) - (Pl[4] - L.F[0] * sl), ml - mr, ok);
+    const double ml = mul(Pl[0], sl, ok), mr = mul(Pr[0], sr, ok);
+    const double lc = div((Pr[4] - mul(R.F[0], sr, ok)) - (Pl[4] - mul(L.F[0], sl, ok)), ml - mr, ok);
     const bool left = !sign_bit(lc) || is_zero(lc);
     const double s = left ? am : ap, m = left ? ml : mr, vn = left ? L.vn : R.vn;
     double P[5], U[5], G[5];
@@ -286,40 +304,39 @@ F64_FN void hllc(const Consts& c, const double* Pl, const double* Pr, const Side
         U[q] = left ? L.U[q] : R.U[q];
         G[q] = left ? L.F[q] : R.F[q];
     }
-    const double f = ieee64::div(m, s - lc, ok);
+    const double f = div(m, s - lc, ok);
     const double w = lc - vn;
     double Us[5];
     Us[0] = f;
-    Us[4] = f * (ieee64::div(U[4], P[0], ok) + w * (lc + ieee64::div(P[4], m, ok)));
+    Us[4] = mul(f, div(U[4], P[0], ok) + mul(w, lc + div(P[4], m, ok), ok), ok);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) Us[1 + d] = f * add_normal<AXIS>(c, d, P[1 + d], w);
+    for (int d = 0; d < 3; ++d) Us[1 + d] = mul(f, add_normal<AXIS>(c, d, P[1 + d], w), ok);
     const bool supersonic = is_zero(am);
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
-        const double star = G[q] + s * (Us[q] - U[q]);
+        const double star = G[q] + mul(s, Us[q] - U[q], ok);
         F[q] = supersonic ? L.F[q] : star;
     }
 }
 
 // ---------------------------------------------------------------------------
-// hydro_cons; mhd_cons where it accepts the state as it is
+// hydro_cons; mhd_cons where it accepts the state as it is (U ordinary)
 template <int LAW>
 F64_FN void cons(const Consts& c, const double* U, double* P, bool& ok)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     const Divisor rho = ieee64::divisor(U[0], ok);
-    const double p2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
-    double e = U[4] - ieee64::div(half(p2), rho, ok);
+    double e = U[4] - div(half(dot(U[1], U[2], U[3], U[1], U[2], U[3])), rho, ok);
     if constexpr (LAW != LAW_HYDRO) {
-        e = e - half(U[5] * U[5] + U[6] * U[6] + U[7] * U[7]);
+        e = e - half(dot(U[5], U[6], U[7], U[5], U[6], U[7]));
 #pragma unroll
         for (int q = 5; q < NQ; ++q) P[q] = U[q];
-        ok = ok && !sign_bit(e) && !sign_bit(U[0]) && !sign_bit(U[4]);
+        ok = ok && !sign_bit(e);
     }
     P[0] = U[0];
-    P[4] = e * c.gm1;
+    P[4] = mul(e, c.gm1, ok);
 #pragma unroll
-    for (int q = 1; q < 4; ++q) P[q] = ieee64::div(U[q], rho, ok);
+    for (int q = 1; q < 4; ++q) P[q] = div(U[q], rho, ok);
 }
 
 // hydro_p2u, mhd_p2u
@@ -327,17 +344,16 @@ template <int LAW>
 F64_FN void p2u(const Consts& c, const double* P, double* U, bool& ok)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
-    const double vv = P[1] * P[1] + P[2] * P[2] + P[3] * P[3];
     U[0] = P[0];
 #pragma unroll
-    for (int d = 1; d < 4; ++d) U[d] = P[0] * P[d];
-    double e = half(P[0] * vv);
+    for (int d = 1; d < 4; ++d) U[d] = mul(P[0], P[d]);
+    double e = half(mul(P[0], dot(P[1], P[2], P[3], P[1], P[2], P[3])));
     if constexpr (LAW != LAW_HYDRO) {
-        e = e + half(P[5] * P[5] + P[6] * P[6] + P[7] * P[7]);
+        e = e + half(dot(P[5], P[6], P[7], P[5], P[6], P[7]));
 #pragma unroll
         for (int q = 5; q < NQ; ++q) U[q] = P[q];
     }
-    U[4] = e + ieee64::div(P[4], c.gm1_div, ok);
+    U[4] = e + div(P[4], c.gm1_div, ok);
 }
 
 // The largest max_eigen_magnitude over the three face normals: on each,
@@ -345,27 +361,41 @@ F64_FN void p2u(const Consts& c, const double* P, double* U, bool& ok)
 template <int LAW>
 F64_FN double fastest(const Consts& c, const double* P, bool& ok)
 {
-    const double v[3] = {P[1], P[1] * c.ny0 + P[2], P[3]};
+    const double v[3] = {P[1], mul(P[1], c.ny0) + P[2], P[3]};
     const Divisor rho = ieee64::divisor(P[0], ok);
-    const double cs2 = ieee64::div(c.gamma * P[4], rho, ok);
+    const double cs2 = div(mul(c.gamma, P[4]), rho, ok);
     if constexpr (LAW == LAW_HYDRO) {
         u64 vmax = mag(v[0]) > mag(v[1]) ? mag(v[0]) : mag(v[1]);
         vmax = vmax > mag(v[2]) ? vmax : mag(v[2]);
-        return from_bits(vmax) + ieee64::sqrt_rn(cs2, ok);
+        return from_bits(vmax) + sqrt_rn(cs2, ok);
     } else {
-        const double BB = P[5] * P[5] + P[6] * P[6] + P[7] * P[7];
-        const double B[3] = {P[5], P[5] * c.ny0 + P[6], P[7]};
-        const double s = cs2 + ieee64::div(BB, rho, ok);
-        const double s2 = s * s;
+        const double BB = dot(P[5], P[6], P[7], P[5], P[6], P[7]);
+        const double B[3] = {P[5], mul(P[5], c.ny0) + P[6], P[7]};
+        const double s = cs2 + div(BB, rho, ok);
+        const double s2 = mul(s, s);
         double m = 0.0;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const double cn2 = ieee64::div(B[a] * B[a], rho, ok);
-            const double cF2 = half(s + ieee64::sqrt_rn(s2 - scale(cs2 * cn2, 2), ok));
-            m = max_pos(m, from_bits(mag(v[a])) + ieee64::sqrt_rn(max_pos(cF2, cn2), ok));
+            const double cn2 = div(mul(B[a], B[a], ok), rho, ok);
+            const double cF2 = half(s + sqrt_rn(s2 - scale(cs2, 2) * cn2, ok));
+            m = max_pos(m, from_bits(mag(v[a])) + sqrt_rn(max_pos(cF2, cn2), ok));
         }
         return m;
     }
+}
+
+// a b for any operands: on the FP64 pipe only where the integer product does
+// not hold (the asm keeps the compiler from issuing both)
+F64_FN double mul_any(double a, double b)
+{
+    bool ok = true;
+    double r = mul(a, b, ok);
+#if defined(__CUDA_ARCH__)
+    if (!ok) asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+#else
+    if (!ok) r = a * b;
+#endif
+    return r;
 }
 
 } // namespace fast64

@@ -98,8 +98,13 @@ struct FaceSpace {
     int axis;
 };
 
+// resident blocks per SM: registers (168 or 128 a thread) against warps in
+// flight; the hydro kernel loses 1 to 11 % at 4 to 6 blocks (spills), the MHD
+// kernel gains 1 % at 4
+template <int LAW> constexpr int FLUX_BLOCKS = LAW == LAW_HYDRO ? 3 : 4;
+
 template <int LAW, int RECON, int RIEMANN, int AXIS>
-__global__ void __launch_bounds__(128) flux_kernel(const double* __restrict__ P, double* __restrict__ F,
+__global__ void __launch_bounds__(128, AXIS < 0 ? 1 : FLUX_BLOCKS<LAW>) flux_kernel(const double* __restrict__ P, double* __restrict__ F,
                                                    const __grid_constant__ GridDesc G,
                                                    const __grid_constant__ PhysParams pp,
                                                    const __grid_constant__ fast64::Consts C,
@@ -146,7 +151,7 @@ __global__ void __launch_bounds__(128) flux_kernel(const double* __restrict__ P,
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
                 const double v = p[q * G.sP + z * stride];
-                o = o && (RECON == RECON_WENO5 ? fast64::weno_ordinary(v) : fast64::ordinary(v));
+                o = o && fast64::ordinary_field(q, v);
             }
             fine = 2 * fine + o;
         }
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(128) flux_kernel(const double* __restrict__ P,
                 const double* v = p + q * G.sP;
                 if constexpr (RECON == RECON_PCM) {
                     PR[q] = next[q] = v[0];
-                    o = o && fast64::ordinary(v[0]);
+                    o = o && fast64::ordinary_field(q, v[0]);
                 } else if constexpr (RECON == RECON_PLM) {
                     const double c = v[0], r = v[stride];
                     const double b = C.theta * (r - c);
@@ -182,19 +187,32 @@ __global__ void __launch_bounds__(128) flux_kernel(const double* __restrict__ P,
                     d[q] = b;
                     PR[q] = c - h;
                     next[q] = c + h;
-                    o = o && fast64::ordinary(r);
+                    o = o && fast64::ordinary_field(q, r);
                 } else {
                     const double w[5] = {v[-2 * stride], v[-stride], v[0], v[stride], v[2 * stride]};
                     fast64::weno5_edges(C, &w[2], PR[q], next[q], ok_left);
-                    o = o && fast64::weno_ordinary(w[4]);
+                    o = o && fast64::ordinary_field(q, w[4]);
                 }
             }
             fine = 2 * fine + o;
             ok = ok && ok_left && (fine & ((1u << 2 * S) - 1u)) == (1u << 2 * S) - 1u;
             fast64::Side<NQ> L, R;
             double Fh[NQ];
-            fast64::side<LAW, AXIS>(C, PL, L, ok);
-            fast64::side<LAW, AXIS>(C, PR, R, ok);
+            // the two sides in a loop: its code once (the kernels run out of
+            // the instruction cache; KH 1024^2 5.42 -> 5.27 ms, MHD 64x56x48
+            // 3.78 -> 3.58)
+            double Ps[NQ];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) Ps[q] = PL[q];
+#pragma unroll 1
+            for (int s = 0; s < 2; ++s) {
+                fast64::side<LAW, AXIS>(C, Ps, R, ok);
+                if (s == 0) {
+                    L = R;
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) Ps[q] = PR[q];
+                }
+            }
             if constexpr (RIEMANN == RIEMANN_HLLC) fast64::hllc<AXIS>(C, PL, PR, L, R, Fh, ok);
             else fast64::hlle<NQ>(L, R, Fh, ok);
             if (ok) {
@@ -279,8 +297,10 @@ __device__ __forceinline__ double face_flux(const FluxView& V, const GridDesc& G
 // FP64 pipe, so the face area products of flat axes (zeros) are left out, and
 // the RK weights 1, 1/2 and 1/4 act on exponents; b1, b2: the weights of U0
 // and of the stage's result.
+// Resident blocks: hydro 1 to 5 a SM 5.60 ms, 8 5.39 (KH 1024^2, four steps);
+// MHD 1 3.94, 4 3.66, 5 3.57, 8 3.67 (64x56x48).
 template <int LAW>
-__global__ void __launch_bounds__(128) update_kernel(const double* __restrict__ Pin, double* __restrict__ Pout,
+__global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 1 : 5) update_kernel(const double* __restrict__ Pin, double* __restrict__ Pout,
                                                      double* __restrict__ U0, double* __restrict__ U,
                                                      const __grid_constant__ FluxView V,
                                                      const __grid_constant__ GridDesc G,
@@ -308,7 +328,7 @@ __global__ void __launch_bounds__(128) update_kernel(const double* __restrict__ 
         bool ok = C.ok && LAW != LAW_RMHD;
         if constexpr (LAW != LAW_RMHD) {
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary(Pc[q]);
+            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
             fast64::p2u<LAW>(C, Pc, Uo, ok);
         }
         if (!ok) {
@@ -329,19 +349,19 @@ __global__ void __launch_bounds__(128) update_kernel(const double* __restrict__ 
         // the sum over the faces in the reference's order; a flat axis adds
         // and subtracts a zero, which only makes a -0 a +0
         double sum = 0.0;
-        if (fx) sum = face_flux<NQ>(V, G, 0, q, i + 1, j, k) * G.dA[0] - face_flux<NQ>(V, G, 0, q, i, j, k) * G.dA[0];
-        if (fy) sum = sum + face_flux<NQ>(V, G, 1, q, i, j + 1, k) * G.dA[1] - face_flux<NQ>(V, G, 1, q, i, j, k) * G.dA[1];
+        if (fx) sum = fast64::mul_any(face_flux<NQ>(V, G, 0, q, i + 1, j, k), G.dA[0]) - fast64::mul_any(face_flux<NQ>(V, G, 0, q, i, j, k), G.dA[0]);
+        if (fy) sum = sum + fast64::mul_any(face_flux<NQ>(V, G, 1, q, i, j + 1, k), G.dA[1]) - fast64::mul_any(face_flux<NQ>(V, G, 1, q, i, j, k), G.dA[1]);
         else sum = fast64::add_zero(sum, false);
-        if (fz) sum = sum + face_flux<NQ>(V, G, 2, q, i, j, k + 1) * G.dA[2] - face_flux<NQ>(V, G, 2, q, i, j, k) * G.dA[2];
+        if (fz) sum = sum + fast64::mul_any(face_flux<NQ>(V, G, 2, q, i, j, k + 1), G.dA[2]) - fast64::mul_any(face_flux<NQ>(V, G, 2, q, i, j, k), G.dA[2]);
         else sum = fast64::add_zero(sum, false);
-        double L = fv * sum;
+        double L = fast64::mul_any(fv, sum);
         if constexpr (LAW == LAW_MHD_COOL) {
             // NewtonianMHD::addSourceTerms (ConservationLaws.cpp:489-501)
             if (q == 4) L -= Pc[4] / (pp.gamma - 1.0) * pp.cooling_rate;
             if (q == 8) L += Pc[4] / (pp.gamma - 1.0) * pp.cooling_rate;
         }
         if (S) L += S[q * G.sP + pc];  // the source terms function's array (SolutionSchemes.cpp:219-228)
-        const double X = Up[q] + dt * L;
+        const double X = Up[q] + fast64::mul_any(dt, L);
         if (pow2 == 0) {
             // U0 0 + X: a zero plus X (NaN for an infinite U0)
             Un[q] = fast64::expo(Uo[q]) == 0x7ffu ? Uo[q] * (1 - b) + X : fast64::add_zero(X, fast64::sign_bit(Uo[q]));
@@ -351,7 +371,7 @@ __global__ void __launch_bounds__(128) update_kernel(const double* __restrict__ 
             Un[q] = Uo[q] * (1 - b) + X * b;
         }
         U[q * G.sU + uc] = Un[q];
-        fine = fine && fast64::ordinary(Un[q]);
+        fine = fine && fast64::ordinary_field(q, Un[q]);
     }
 
     double Pn[NQ];
@@ -424,7 +444,7 @@ __global__ void __launch_bounds__(128) courant_kernel(const double* __restrict__
         bool ok = C.ok && LAW != LAW_RMHD;
         if constexpr (LAW != LAW_RMHD) {
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary(Pc[q]);
+            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
             lmax = fast64::fastest<LAW>(C, Pc, ok);
         }
         if (!ok) {
@@ -515,11 +535,15 @@ static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const
         else { X.lo[a] = 0; X.nb[a] = 1; }
         faces *= X.nb[a];
     }
-    // runs as long as 16 warps per SM remain: a run of one forms every
-    // zone's reconstruction twice, one of eight 1/8 too many
-    const long long want = 152ll * 512;
+    // a run of one forms every zone's reconstruction twice, one of eight 1/8
+    // too many: runs as long as four waves of resident threads remain (KH
+    // 1024^2, four steps: 5.42 ms at 4 faces a run, 5.61 at 8 and 2, 6.28 at 1)
     X.nf = X.nb[axis];
-    X.run = HAS_FAST<LAW, RIEMANN> && RECON != RECON_PCM ? (int) (faces / want < 1 ? 1 : faces / want > 8 ? 8 : faces / want) : 1;
+    X.run = 1;
+    if (HAS_FAST<LAW, RIEMANN> && RECON != RECON_PCM) {
+        const long long want = 152ll * 1536;
+        X.run = (int) (faces < 2 * want ? 1 : faces > 8 * want ? 8 : faces / want);
+    }
     X.nb[axis] = (X.nf + X.run - 1) / X.run;
     const long long slice = (long long) X.nb[0] * X.nb[1];
     const int block = block_size(slice * X.nb[2]);

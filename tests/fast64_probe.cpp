@@ -58,6 +58,7 @@ static double any()
     }
 }
 
+#ifndef PROBE_IEEE_ONLY
 // A zone's primitives.  kind 0: smooth, 1: zeros and equal values, 2: strong
 // jumps, 3: wide magnitudes, 4: anything; hydro pressure and density positive
 // for kinds 0 to 3
@@ -69,7 +70,7 @@ static void zone(int kind, int nq, const double* base, double* P)
         if (kind == 0) v = base[q] * (1 + 0.1 * (uni() - 0.5));
         else if (kind == 1) v = pos ? (rnd() & 1 ? 1.0 : base[q]) : rnd() % 4 == 0 ? base[q] : rnd() % 3 == 0 ? -0.0 : 0.0;
         else if (kind == 2) v = pos ? exp(8 * (uni() - 0.5)) : 6 * (uni() - 0.5);
-        else if (kind == 3) v = pos ? fabs(wide(30)) : wide(rnd() % 8 ? 20 : 290);
+        else if (kind == 3) v = pos ? fabs(wide(30)) : wide(rnd() % 8 ? 20 : 320);
         else v = any();
         P[q] = v;
     }
@@ -91,7 +92,7 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
             double v[2 * S];
             for (int s = 0; s < 2 * S; ++s) {
                 v[s] = Z[s][q];
-                ok = ok && (RECON == RECON_WENO5 ? fast64::weno_ordinary(v[s]) : fast64::ordinary(v[s]));
+                ok = ok && fast64::ordinary_field(q, v[s]);
             }
             if constexpr (RECON == RECON_PCM) { PL[q] = QL[q] = v[0]; PR[q] = QR[q] = v[1]; }
             else if constexpr (RECON == RECON_PLM) {
@@ -183,7 +184,7 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
         zone(kind, NQ, base, P);
         bool ord = C.ok;
-        for (int q = 0; q < NQ; ++q) ord = ord && fast64::ordinary(P[q]);
+        for (int q = 0; q < NQ; ++q) ord = ord && fast64::ordinary_field(q, P[q]);
         double U[NQ], W[NQ];
         bool ok = ord;
         law_p2u<LAW>(pp, P, U);
@@ -195,7 +196,7 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
         for (int t = 0; t < 2; ++t) {
             double D[NQ], A[NQ], B[NQ];
             bool o2 = C.ok;
-            for (int q = 0; q < NQ; ++q) { D[q] = t ? U[q] : P[q]; o2 = o2 && fast64::ordinary(D[q]); A[q] = 0; }
+            for (int q = 0; q < NQ; ++q) { D[q] = t ? U[q] : P[q]; o2 = o2 && fast64::ordinary_field(q, D[q]); A[q] = 0; }
             int code = 0;
             const int e = law_cons<LAW>(pp, D, A, &code);
             fast64::cons<LAW>(C, D, B, o2);
@@ -230,6 +231,8 @@ extern "C" long probe_zones(long n, u64 seed, int law, double gamma, int kind, l
     return zones<LAW_MHD_COOL>(n, pp, C, nrm, kind, accepted);
 }
 
+#endif  // PROBE_IEEE_ONLY
+
 extern "C" long probe_ieee(long n, u64 seed, long* accepted)
 {
     state = seed;
@@ -244,6 +247,9 @@ extern "C" long probe_ieee(long n, u64 seed, long* accepted)
         if (ok) { ++*accepted; bad += !same(q, x / d); }
         double a = fabs(x);
         if (m % 8 == 4) { a = d * d; a = rnd() & 1 ? nextafter(a, 2 * a) : rnd() & 1 ? nextafter(a, 0) : a; }
+        ok = true;
+        const double p = ieee64::mul(x, d, ok);
+        if (ok) { ++*accepted; bad += !same(p, x * d); }
         ok = true;
         const double r = ieee64::sqrt_rn(a, ok);
         if (ok) { ++*accepted; bad += !same(r, sqrt(a)); }

@@ -1,0 +1,74 @@
+"""The plain path's forms with fewer FP64 operations (mara2_gb300/csrc/
+fast64.cuh, ieee64.cuh), built for the host, bit for bit the general ones
+(physics_fp64.cuh) and the host's own division, square root and product:
+every law, reconstruction, solver, axis and smoothness indicator they cover,
+on seeded operands - smooth states, exact zeros of either sign and equal
+states, strong jumps, wide magnitudes, and any bit patterns (infinities, NaNs,
+subnormals), which the forms must refuse or get right.  The hardware's seeds
+of the division and square root enter within a few units in the last place,
+so those are tested with seeds shifted both ways."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+HYDRO, MHD, MHD_COOL = 0, 1, 3
+SMOOTH, ZEROS, JUMPS, WIDE, ANY = range(5)
+
+
+def _build(path, ulps, *flags):
+    cxx = shutil.which("g++")
+    if cxx is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("needs g++ and the CUDA headers")
+    so = os.path.join(str(path), f"libfast64_{ulps}.so")
+    subprocess.run([cxx, "-O2", "-ffp-contract=off", "-std=c++17", "-fPIC", "-shared", f"-DIEEE64_SEED_ULPS={ulps}", *flags,
+                    "-I" + os.path.join(CUDA, "include"), os.path.join(ROOT, "tests", "fast64_probe.cpp"), "-o", so],
+                   check=True)
+    lib = C.CDLL(so)
+    for f in ("probe_ieee",) if flags else ("probe_faces", "probe_zones", "probe_ieee"):
+        getattr(lib, f).restype = C.c_long
+    return lib
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("fast64"), 0)
+
+
+@pytest.mark.parametrize("ulps", [-2, 0, 2])
+def test_integer_division_root_and_product_round_correctly(tmp_path, ulps):
+    acc = C.c_long()
+    n = 400000
+    assert _build(tmp_path, ulps, "-DPROBE_IEEE_ONLY").probe_ieee(C.c_long(n), C.c_ulonglong(5), C.byref(acc)) == 0
+    assert acc.value > 2.8 * n
+
+
+CASES = [(HYDRO, r, s) for r in range(3) for s in range(2)] + [(law, r, 0) for law in (MHD, MHD_COOL) for r in range(3)]
+
+
+@pytest.mark.parametrize("law,recon,riemann", CASES)
+def test_face_flux_has_the_general_forms_bits(lib, law, recon, riemann):
+    n = 4000
+    acc = C.c_long()
+    for axis, gamma, theta in ((0, 5.0 / 3, 1.5), (1, 1.4, 1.0), (2, 4.0 / 3, 2.0)):
+        for weno in (range(3) if recon == 2 else (2,)):
+            for kind in range(5):
+                bad = lib.probe_faces(C.c_long(n), C.c_ulonglong(100 * kind + axis), law, recon, riemann, axis, weno,
+                                      C.c_double(gamma), C.c_double(theta), kind, C.byref(acc))
+                assert bad == 0, (axis, weno, kind)
+                if kind in (SMOOTH, ZEROS):
+                    assert acc.value == n
+
+
+@pytest.mark.parametrize("law", [HYDRO, MHD, MHD_COOL])
+def test_zone_conversions_and_wave_speeds_have_the_general_forms_bits(lib, law):
+    n = 20000
+    acc = C.c_long()
+    for kind in range(5):
+        assert lib.probe_zones(C.c_long(n), C.c_ulonglong(kind), law, C.c_double(5.0 / 3), kind, C.byref(acc)) == 0
+        if kind in (SMOOTH, ZEROS, JUMPS):
+            assert acc.value == n
