@@ -77,6 +77,12 @@ F64_FN double add_zero(double x, bool z_negative)
 // non-positive ones (a zero counts as +0)
 F64_FN double max_pos(double a, double b) { return bits(a) > bits(b) ? a : b; }
 F64_FN double min_neg(double a, double b) { return bits(a) > bits(b) ? a : b; }
+// a < b for numbers, -0 below +0
+F64_FN bool less(double a, double b)
+{
+    const ieee64::i64 x = (ieee64::i64) bits(a), y = (ieee64::i64) bits(b), m = 0x7fffffffffffffffll;
+    return (x ^ ((x >> 63) & m)) < (y ^ ((y >> 63) & m));
+}
 // max(x, +0) and min(x, +0) for x without -0
 F64_FN double clamp_pos(double x) { return sign_bit(x) ? 0.0 : x; }
 F64_FN double clamp_neg(double x) { return sign_bit(x) ? x : 0.0; }
@@ -86,7 +92,8 @@ struct Consts {
     double gamma, gm1, theta, ny0;   // ny0: x component of the y normal
     double shenzha_A;
     int weno_is;
-    Divisor gm1_div;
+    double gamf;                     // (gamma - 1) / gamma
+    Divisor gm1_div, d3, d6, d9, d27;
     bool ok;                         // the constants themselves are ordinary
 };
 
@@ -111,14 +118,15 @@ F64_FN double half_slope(double a, double rl, double d)
 // weno5 at both edges of a zone, from ordinary v[-2 .. 2]: the smoothness
 // indicators and the products that both edges use once
 
-F64_FN double sq(double x) { return x * x; }
+F64_FN double sq(double x) { return mul(x, x); }
 
 F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& right, bool& ok)
 {
-    const double q = 1. / 4., t = 13. / 12.;
-    double B0 = t * sq(v[0] - scale(v[1], 1) + v[2]) + q * sq(3 * v[0] - scale(v[1], 2) + v[2]);
-    double B1 = t * sq(v[-1] - scale(v[0], 1) + v[1]) + q * sq(v[-1] - v[1]);
-    double B2 = t * sq(v[-2] - scale(v[-1], 1) + v[0]) + q * sq(v[-2] - scale(v[-1], 2) + 3 * v[0]);
+    const double t = 13. / 12.;
+    const double v3 = 3 * v[0];
+    double B0 = t * sq(v[0] - scale(v[1], 1) + v[2]) + scale(sq(v3 - scale(v[1], 2) + v[2]), -2);
+    double B1 = t * sq(v[-1] - scale(v[0], 1) + v[1]) + scale(sq(v[-1] - v[1]), -2);
+    double B2 = t * sq(v[-2] - scale(v[-1], 1) + v[0]) + scale(sq(v[-2] - scale(v[-1], 2) + v3), -2);
     // w = d / e for the three stencils
     double wl[3], wr[3];
     if (c.weno_is == WENO_BORGES08) {
@@ -147,14 +155,14 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
         wl[0] = div(0.1, e0, ok); wl[1] = wr[1]; wl[2] = div(0.3, e2, ok);
     }
     const double third = 1. / 3., sixth = 1. / 6., a56 = 5. / 6., a76 = 7. / 6., a116 = 11. / 6.;
-    const double r0 = third * v[0] + a56 * v[1] - sixth * v[2];
-    const double r1 = -sixth * v[-1] + a56 * v[0] + third * v[1];
-    const double r2 = third * v[-2] - a76 * v[-1] + a116 * v[0];
-    const double l0 = a116 * v[0] - a76 * v[1] + third * v[2];
-    const double l1 = third * v[-1] + a56 * v[0] - sixth * v[1];
-    const double l2 = -sixth * v[-2] + a56 * v[-1] + third * v[0];
-    right = div(wr[0] * r0 + wr[1] * r1 + wr[2] * r2, wr[0] + wr[1] + wr[2], ok);
-    left = div(wl[0] * l0 + wl[1] * l1 + wl[2] * l2, wl[0] + wl[1] + wl[2], ok);
+    const double c0 = mul(a56, v[0]), t0 = mul(third, v[0]), e0 = mul(a116, v[0]);
+    const double tp = mul(third, v[1]), tm = mul(third, v[-1]), sp = mul(sixth, v[1]), sm = mul(sixth, v[-1]);
+    const double tp2 = mul(third, v[2]), tm2 = mul(third, v[-2]), sp2 = mul(sixth, v[2]), sm2 = mul(sixth, v[-2]);
+    const double cp = mul(a56, v[1]), cm = mul(a56, v[-1]), gp = mul(a76, v[1]), gm = mul(a76, v[-1]);
+    const double r0 = t0 + cp - sp2, r1 = -sm + c0 + tp, r2 = tm2 - gm + e0;
+    const double l0 = e0 - gp + tp2, l1 = tm + c0 - sp, l2 = -sm2 + cm + t0;
+    right = div(mul(wr[0], r0) + mul(wr[1], r1) + mul(wr[2], r2), wr[0] + wr[1] + wr[2], ok);
+    left = div(mul(wl[0], l0) + mul(wl[1], l1) + mul(wl[2], l2), wl[0] + wl[1] + wl[2], ok);
 }
 
 // ---------------------------------------------------------------------------
@@ -275,15 +283,11 @@ F64_FN void side(const Consts& c, const double* P, Side<LawInfo<LAW>::NQ>& S, bo
 }
 
 // ---------------------------------------------------------------------------
-template <int NQ>
-F64_FN void hlle(const Side<NQ>& L, const Side<NQ>& R, double* F, bool& ok)
+// hlle of one field, from the sides' clamped wave speeds
+F64_FN double hlle(double apl, double apr, double aml, double amr, double fl, double fr, double ul, double ur, bool& ok)
 {
-    const double ap = max_pos(L.ap, R.ap), am = min_neg(L.am, R.am);
-    const Divisor den = ieee64::divisor(ap - am, ok);
-    const double apam = mul(ap, am, ok);
-#pragma unroll
-    for (int q = 0; q < NQ; ++q)
-        F[q] = div(ap * L.F[q] - am * R.F[q] + apam * (R.U[q] - L.U[q]), den, ok);
+    const double ap = max_pos(apl, apr), am = min_neg(aml, amr);
+    return div(ap * fl - am * fr + ap * am * (ur - ul), ap - am, ok);
 }
 
 // the star state of the side the contact moves away from, chosen first

@@ -28,6 +28,7 @@
 #include "../../include/mara_gpu.h"
 #include "internal.h"
 #include "fast64.cuh"
+#include "fast64_rmhd.cuh"
 #include "physics_fp64.cuh"
 
 namespace mara {
@@ -82,15 +83,14 @@ __device__ __noinline__ int face_general(const double* P, long long sP, long lon
     return ST_OK;
 }
 
-// laws and solvers that fast64.cuh covers
-template <int LAW, int RIEMANN>
-constexpr bool HAS_FAST = LAW != LAW_RMHD && (RIEMANN == RIEMANN_HLLE || LAW == LAW_HYDRO);
+// The HLLC faces of one axis, each thread a run of consecutive faces along
+// it: a zone's reconstruction serves the faces on both of its sides.  Bound by
+// the FP64 pipe (fast64.cuh; KH 1024^2 421 -> about 185 us an axis, of which
+// the additions alone take 170); a face whose operands are not ordinary goes
+// through face_general, as do all faces of the magnetic laws, for which the
+// solver is not meant (AXIS < 0, the axis at run time).
+template <int LAW> constexpr bool HLLC_FAST = LAW == LAW_HYDRO;
 
-// The faces of one axis, each thread a run of consecutive faces along it: a
-// zone's reconstruction serves the faces on both of its sides.  Bound by the
-// FP64 pipe (fast64.cuh); a face whose operands are not ordinary goes through
-// face_general, as do all faces of the laws without a fast form (AXIS < 0,
-// the axis at run time).
 struct FaceSpace {
     int lo[3];   // first face (right cell) and row of each axis
     int nb[3];   // threads per axis: runs along the faces' axis, rows across it
@@ -98,13 +98,9 @@ struct FaceSpace {
     int axis;
 };
 
-// resident blocks per SM: registers (168 or 128 a thread) against warps in
-// flight; the hydro kernel loses 1 to 11 % at 4 to 6 blocks (spills), the MHD
-// kernel gains 1 % at 4
-template <int LAW> constexpr int FLUX_BLOCKS = LAW == LAW_HYDRO ? 3 : 4;
-
+// Three blocks per SM (168 registers): 4, 5 and 6 lose 1, 6 and 11 % to spills.
 template <int LAW, int RECON, int RIEMANN, int AXIS>
-__global__ void __launch_bounds__(128, AXIS < 0 ? 1 : FLUX_BLOCKS<LAW>) flux_kernel(const double* __restrict__ P, double* __restrict__ F,
+__global__ void __launch_bounds__(128, AXIS < 0 ? 1 : 3) flux_kernel(const double* __restrict__ P, double* __restrict__ F,
                                                    const __grid_constant__ GridDesc G,
                                                    const __grid_constant__ PhysParams pp,
                                                    const __grid_constant__ fast64::Consts C,
@@ -213,8 +209,7 @@ __global__ void __launch_bounds__(128, AXIS < 0 ? 1 : FLUX_BLOCKS<LAW>) flux_ker
                     for (int q = 0; q < NQ; ++q) Ps[q] = PR[q];
                 }
             }
-            if constexpr (RIEMANN == RIEMANN_HLLC) fast64::hllc<AXIS>(C, PL, PR, L, R, Fh, ok);
-            else fast64::hlle<NQ>(L, R, Fh, ok);
+            fast64::hllc<AXIS>(C, PL, PR, L, R, Fh, ok);
             if (ok) {
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) f[q * G.sF] = Fh[q];
@@ -226,6 +221,135 @@ __global__ void __launch_bounds__(128, AXIS < 0 ? 1 : FLUX_BLOCKS<LAW>) flux_ker
 #pragma unroll
             for (int q = 0; q < NQ; ++q) PL[q] = next[q];
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same for HLLE, a block's threads sharing a tile of faces in three
+// phases through shared memory: the edge values of every (zone, field), the
+// state of every (face, side), the HLLE flux of every (face, field).  Each
+// phase is a short loop over independent items, so its code stays in the
+// instruction cache and small grids still fill the schedulers.  Bound by the
+// FP64 pipe (66 to 72 % busy).  Against a thread per run of faces: MHD
+// 64x56x48 115 to 138 -> 91 to 102 us an axis, a 1024-zone tube's run 2.95 ->
+// 2.77 ms.  Blocks of 32, 64, 128 and 256 threads: 3.26, 3.27, 3.32, 3.43 ms
+// (MHD 64x56x48, two steps and their transfers).
+struct TileSpace {
+    int lo[3];      // first face (right cell) and rows of each axis
+    int nf;         // faces along the axis
+    int ncol;       // rows of the axis that runs across the tile
+    int len, width; // faces along and across a tile, at most TILE_FACES in all
+    int na, nc;     // tiles along and across
+};
+
+constexpr int TILE_THREADS = 64, TILE_FACES = TILE_THREADS / 2, TILE_ZONES = TILE_FACES + 4;
+
+template <int RECON>
+__device__ __forceinline__ void zone_edges(const fast64::Consts& C, const double* p, long long s, int q, double& left,
+                                           double& right, bool& ok)
+{
+    if constexpr (RECON == RECON_PCM) {
+        left = right = p[0];
+        ok = ok && fast64::ordinary_field(q, p[0]);
+    } else if constexpr (RECON == RECON_PLM) {
+        const double l = p[-s], c = p[0], r = p[s];
+        const double h = fast64::half_slope(C.theta * (c - l), r - l, C.theta * (r - c));
+        left = c - h;
+        right = c + h;
+        ok = ok && fast64::ordinary_field(q, l) && fast64::ordinary_field(q, c) && fast64::ordinary_field(q, r);
+    } else {
+        const double w[5] = {p[-2 * s], p[-s], p[0], p[s], p[2 * s]};
+#pragma unroll
+        for (int m = 0; m < 5; ++m) ok = ok && fast64::ordinary_field(q, w[m]);
+        fast64::weno5_edges(C, &w[2], left, right, ok);
+    }
+}
+
+template <int LAW, int AXIS>
+__device__ __forceinline__ void face_side(const fast64::Consts& C, const double* P, fast64::Side<LawInfo<LAW>::NQ>& S,
+                                          bool& ok)
+{
+    if constexpr (LAW == LAW_RMHD) fast64::rmhd_side<AXIS>(C, P, S, ok);
+    else fast64::side<LAW, AXIS>(C, P, S, ok);
+}
+
+template <int LAW, int RECON, int AXIS>
+__global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS) flux_tile_kernel(const double* __restrict__ P, double* __restrict__ F,
+                                                           const __grid_constant__ GridDesc G,
+                                                           const __grid_constant__ PhysParams pp,
+                                                           const __grid_constant__ fast64::Consts C,
+                                                           const __grid_constant__ TileSpace X,
+                                                           DevStatus* __restrict__ st)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ;
+    __shared__ double edge[2][NQ][TILE_ZONES];           // left and right edge of each zone
+    __shared__ double sU[2][NQ][TILE_FACES], sF[2][NQ][TILE_FACES], sA[2][2][TILE_FACES];
+    __shared__ unsigned char odd_zone[TILE_ZONES], odd_face[TILE_FACES];   // operands out of the ordinary
+    const int tid = threadIdx.x;
+    for (int z = tid; z < TILE_ZONES; z += TILE_THREADS) odd_zone[z] = 0;
+    if (tid < TILE_FACES) odd_face[tid] = 0;
+    const int code = st->code, failures = st->failures;
+    if (__syncthreads_or(code != 0 || st->done || failures != 0)) {
+        if (code == 0 && failures != 0) st->halt = 1;    // failures are final once the stage ended
+        return;
+    }
+    const int b = blockIdx.x;
+    const int a0 = (b % X.na) * X.len, c0 = (b / X.na) % X.nc * X.width, o = b / X.na / X.nc;
+    const int len = min(X.len, X.nf - a0), width = min(X.width, X.ncol - c0);
+    const int faces = len * width, zones = faces + width;
+    const int i = X.lo[0] + (AXIS == 0 ? a0 : c0);
+    const int j = X.lo[1] + (AXIS == 1 ? a0 : AXIS == 0 ? c0 : o);
+    const int k = X.lo[2] + (AXIS == 2 ? a0 : o);
+    const long long s0 = 1, s1 = G.N[0], s2 = (long long) G.N[0] * G.N[1];
+    const long long stride = AXIS == 0 ? s0 : AXIS == 1 ? s1 : s2, cstride = AXIS == 0 ? s1 : s0;
+    const double* p = P + ((long long) k * G.N[1] + j) * G.N[0] + i;   // cell on the right of the tile's first face
+    for (int it = tid; it < NQ * zones; it += TILE_THREADS) {
+        const int q = it / zones, z = it - q * zones, s = z / width, w = z - s * width;
+        bool ok = true;
+        double l, r;
+        zone_edges<RECON>(C, p + q * G.sP + (s - 1) * stride + w * cstride, stride, q, l, r, ok);
+        edge[0][q][z] = l;
+        edge[1][q][z] = r;
+        if (!ok) odd_zone[z] = 1;
+    }
+    __syncthreads();
+    if (tid < 2 * faces) {
+        const int s = tid >= faces ? 1 : 0, f = tid - s * faces, z = f + s * width;
+        double Ps[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) Ps[q] = edge[1 - s][q][z];
+        fast64::Side<NQ> S;
+        bool ok = C.ok && !odd_zone[z];
+        face_side<LAW, AXIS>(C, Ps, S, ok);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            sU[s][q][f] = S.U[q];
+            sF[s][q][f] = S.F[q];
+        }
+        sA[s][0][f] = S.ap;
+        sA[s][1][f] = S.am;
+        if (!ok) odd_face[f] = 1;
+    }
+    __syncthreads();
+    const long long f0 = 1, f1 = G.N[0] + 1, f2 = (long long) (G.N[0] + 1) * (G.N[1] + 1);
+    const long long fstride = AXIS == 0 ? f0 : AXIS == 1 ? f1 : f2, fcstride = AXIS == 0 ? f1 : f0;
+    double* out = F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
+    for (int it = tid; it < NQ * faces; it += TILE_THREADS) {
+        const int q = it / faces, f = it - q * faces, s = f / width, w = f - s * width;
+        bool ok = !odd_face[f];
+        const double h = fast64::hlle(sA[0][0][f], sA[1][0][f], sA[0][1][f], sA[1][1][f], sF[0][q][f], sF[1][q][f],
+                                      sU[0][q][f], sU[1][q][f], ok);
+        double* to = out + s * fstride + w * fcstride;
+        if (ok) to[q * G.sF] = h;
+        else odd_face[f] = 1;   // every field of the face by the general functions, below
+    }
+    __syncthreads();
+    if (tid < faces && odd_face[tid]) {
+        const int s = tid / width, w = tid - s * width;
+        const int e = face_general<LAW, RECON, RIEMANN_HLLE>(p + s * stride + w * cstride, G.sP, stride,
+                                                             G.nrm[AXIS][0], G.nrm[AXIS][1], G.nrm[AXIS][2], &pp,
+                                                             out + s * fstride + w * fcstride, G.sF);
+        if (e != ST_OK) record_status(st, e);
     }
 }
 
@@ -325,12 +449,11 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
     for (int q = 0; q < NQ; ++q) Pc[q] = Pin[q * G.sP + pc];
 
     if (stage == 0) {
-        bool ok = C.ok && LAW != LAW_RMHD;
-        if constexpr (LAW != LAW_RMHD) {
+        bool ok = C.ok;
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
-            fast64::p2u<LAW>(C, Pc, Uo, ok);
-        }
+        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
+        if constexpr (LAW == LAW_RMHD) fast64::rmhd_p2u(C, Pc, Uo, ok);
+        else fast64::p2u<LAW>(C, Pc, Uo, ok);
         if (!ok) {
             const int e = law_p2u<LAW>(pp, Pc, Uo);
             if (e != ST_OK) { record_status(st, e); return; }
@@ -375,8 +498,8 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
     }
 
     double Pn[NQ];
-    if constexpr (LAW != LAW_RMHD) fast64::cons<LAW>(C, Un, Pn, fine);
-    else fine = false;
+    if constexpr (LAW == LAW_RMHD) fast64::rmhd_cons(C, Un, Pn, fine);
+    else fast64::cons<LAW>(C, Un, Pn, fine);
     if (!fine) {
         int code = ST_OK;
         const int e = law_cons<LAW>(pp, Un, Pn, &code);
@@ -432,36 +555,37 @@ __global__ void __launch_bounds__(128) courant_kernel(const double* __restrict__
                                                       DevStatus* __restrict__ st)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
-    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    // the relativistic law's three normals cost a quartic each: a thread each
+    constexpr int AXES = LAW == LAW_RMHD ? 3 : 1;
+    const unsigned slice = (unsigned) G.n[0] * (unsigned) G.n[1];
+    const unsigned item = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long mine = 0;
-    if (lin < (unsigned) G.n[0] * (unsigned) G.n[1] && st->code == 0) {
+    if (item < AXES * slice && st->code == 0) {
+        const int axis = (int) (item / slice);
+        const unsigned lin = item - axis * slice;
         const int ii = (int) (lin % (unsigned) G.n[0]), jj = (int) (lin / (unsigned) G.n[0]), kk = blockIdx.y;
         const long long pc = ((long long) (kk + G.g[2]) * G.N[1] + (jj + G.g[1])) * G.N[0] + (ii + G.g[0]);
         double Pc[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) Pc[q] = P[q * G.sP + pc];
         double lmax = 0.0;
-        bool ok = C.ok && LAW != LAW_RMHD;
-        if constexpr (LAW != LAW_RMHD) {
+        bool ok = C.ok;
 #pragma unroll
-            for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
-            lmax = fast64::fastest<LAW>(C, Pc, ok);
-        }
+        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
+        if constexpr (LAW == LAW_RMHD) lmax = fast64::rmhd_fastest(C, Pc, axis, ok);
+        else lmax = fast64::fastest<LAW>(C, Pc, ok);
         if (!ok) {
-            double lam[3];
             int e = ST_OK;
-            for (int a = 0; a < 3 && e == ST_OK; ++a) {
+            lmax = 0.0;
+            for (int a = AXES == 3 ? axis : 0; a <= (AXES == 3 ? axis : 2) && e == ST_OK; ++a) {
                 StateD<NQ> S;
                 e = law_prim<LAW>(pp, Pc, G.nrm[a], S);
-                lam[a] = max_eigen_magnitude<NQ>(S.A);
+                const double lam = max_eigen_magnitude<NQ>(S.A);
+                if (e == ST_OK && lmax < lam) lmax = lam;
             }
             if (e != ST_OK) {
                 record_status(st, e);
                 lmax = 0.0;
-            } else {
-                lmax = lam[0];
-                if (lmax < lam[1]) lmax = lam[1];
-                if (lmax < lam[2]) lmax = lam[2];
             }
         }
         mine = (unsigned long long) __double_as_longlong(lmax);
@@ -506,7 +630,12 @@ static fast64::Consts to_fast(const PhysParamsH& h, const GridDesc& G)
     c.shenzha_A = h.shenzha_A;
     c.weno_is = h.weno_is;
     c.ny0 = G.nrm[1][0];
+    c.gamf = (h.gamma - 1.0) / h.gamma;
     c.gm1_div = ieee64::divisor(c.gm1, c.ok);
+    c.d3 = ieee64::divisor(3.0, c.ok);
+    c.d6 = ieee64::divisor(6.0, c.ok);
+    c.d9 = ieee64::divisor(9.0, c.ok);
+    c.d27 = ieee64::divisor(27.0, c.ok);
     // ordinary constants, the normals that fast64.cuh assumes
     const double small = 1e-3, large = 1e3;
     c.ok = c.ok && c.gamma > small && c.gamma < large && c.gm1 > small && c.theta > small && c.theta < large &&
@@ -527,6 +656,31 @@ static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const
 {
     // faces along the axis: the interior faces; across: interior rows, plus
     // one guard row per side on fleshed axes when flux CT is on
+    if constexpr (RIEMANN == RIEMANN_HLLE) {
+        TileSpace T;
+        int nb[3];
+        for (int a = 0; a < 3; ++a) {
+            const int e = G.n[a] > 1 && a != axis && G.ct ? 1 : 0;
+            T.lo[a] = G.g[a] - e;
+            nb[a] = G.n[a] + 2 * e + (a == axis ? 1 : 0);
+        }
+        // across the tile: rows of y for faces along x, four zones of x (a
+        // 32-byte sector) otherwise; along it, equal lengths of at most 64 or 16
+        const int cross = axis == 0 ? 1 : 0, outer = axis == 2 ? 1 : 2;
+        const int most = axis == 0 ? TILE_FACES : TILE_FACES / 4;
+        T.nf = nb[axis];
+        T.ncol = nb[cross];
+        T.width = axis == 0 ? 1 : 4;
+        T.na = (T.nf + most - 1) / most;
+        T.len = (T.nf + T.na - 1) / T.na;
+        T.nc = (T.ncol + T.width - 1) / T.width;
+        const dim3 grid((unsigned) ((long long) T.na * T.nc * nb[outer]));
+        switch (axis) {
+            case 0: flux_tile_kernel<LAW, RECON, 0><<<grid, TILE_THREADS, 0, s>>>(P, F, G, pp, C, T, st); break;
+            case 1: flux_tile_kernel<LAW, RECON, 1><<<grid, TILE_THREADS, 0, s>>>(P, F, G, pp, C, T, st); break;
+            default: flux_tile_kernel<LAW, RECON, 2><<<grid, TILE_THREADS, 0, s>>>(P, F, G, pp, C, T, st); break;
+        }
+    } else {
     FaceSpace X;
     long long faces = 1;
     for (int a = 0; a < 3; ++a) {
@@ -540,7 +694,7 @@ static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const
     // 1024^2, four steps: 5.42 ms at 4 faces a run, 5.61 at 8 and 2, 6.28 at 1)
     X.nf = X.nb[axis];
     X.run = 1;
-    if (HAS_FAST<LAW, RIEMANN> && RECON != RECON_PCM) {
+    if (HLLC_FAST<LAW> && RECON != RECON_PCM) {
         const long long want = 152ll * 1536;
         X.run = (int) (faces < 2 * want ? 1 : faces > 8 * want ? 8 : faces / want);
     }
@@ -549,7 +703,7 @@ static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const
     const int block = block_size(slice * X.nb[2]);
     const dim3 grid((unsigned) ((slice + block - 1) / block), X.nb[2]);
     X.axis = axis;
-    if constexpr (!HAS_FAST<LAW, RIEMANN>) {
+    if constexpr (!HLLC_FAST<LAW>) {
         flux_kernel<LAW, RECON, RIEMANN, -1><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st);
     } else {
         switch (axis) {
@@ -557,6 +711,7 @@ static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const
             case 1: flux_kernel<LAW, RECON, RIEMANN, 1><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
             default: flux_kernel<LAW, RECON, RIEMANN, 2><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
         }
+    }
     }
 }
 
@@ -602,7 +757,7 @@ void plain_update_law(const GridDesc& G, const PhysParamsH& ph, const double* Pi
 template <int LAW>
 void plain_courant_law(const GridDesc& G, const PhysParamsH& ph, const double* P, DevStatus* st, cudaStream_t s)
 {
-    const long long slice = (long long) G.n[0] * G.n[1];
+    const long long slice = (long long) G.n[0] * G.n[1] * (LAW == LAW_RMHD ? 3 : 1);
     const int block = block_size(slice * G.n[2]);
     const dim3 grid((unsigned) ((slice + block - 1) / block), G.n[2]);
     courant_kernel<LAW><<<grid, block, 0, s>>>(P, G, to_dev(ph), to_fast(ph, G), st);

@@ -11,9 +11,15 @@
 static inline long long __double_as_longlong(double x) { long long b; memcpy(&b, &x, 8); return b; }
 static inline double __longlong_as_double(long long b) { double x; memcpy(&x, &b, 8); return x; }
 
-#include "../mara2_gb300/csrc/fast64.cuh"
+#ifdef PROBE_IEEE_ONLY
+#include "../mara2_gb300/csrc/ieee64.cuh"
+#else
+#include "../mara2_gb300/csrc/fast64_rmhd.cuh"
+#endif
 
+#ifndef PROBE_IEEE_ONLY
 using namespace mara;
+#endif
 typedef unsigned long long u64;
 
 static u64 state;
@@ -62,7 +68,7 @@ static double any()
 // A zone's primitives.  kind 0: smooth, 1: zeros and equal values, 2: strong
 // jumps, 3: wide magnitudes, 4: anything; hydro pressure and density positive
 // for kinds 0 to 3
-static void zone(int kind, int nq, const double* base, double* P)
+static void zone(int law, int kind, int nq, const double* base, double* P)
 {
     for (int q = 0; q < nq; ++q) {
         const bool pos = q == 0 || q == 4;
@@ -72,6 +78,7 @@ static void zone(int kind, int nq, const double* base, double* P)
         else if (kind == 2) v = pos ? exp(8 * (uni() - 0.5)) : 6 * (uni() - 0.5);
         else if (kind == 3) v = pos ? fabs(wide(30)) : wide(rnd() % 8 ? 20 : 320);
         else v = any();
+        if (law == LAW_RMHD && kind < 4 && !pos && q < 4) v *= kind == 2 ? 0.16 : 0.5;   // mostly below light speed
         P[q] = v;
     }
 }
@@ -84,7 +91,7 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
     for (long m = 0; m < n; ++m) {
         double Z[2 * S][NQ], base[NQ];
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
-        for (int s = 0; s < 2 * S; ++s) zone(kind, NQ, base, Z[s]);
+        for (int s = 0; s < 2 * S; ++s) zone(LAW, kind, NQ, base, Z[s]);
         if (kind == 1 && rnd() % 3 == 0) for (int s = 1; s < 2 * S; ++s) memcpy(Z[s], Z[0], sizeof(Z[0]));
         double PL[NQ], PR[NQ], QL[NQ], QR[NQ];
         bool ok = C.ok;
@@ -113,14 +120,20 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
         StateD<NQ> L, R;
         const int e = law_prim<LAW>(pp, QL, nrm[AXIS], L) | law_prim<LAW>(pp, QR, nrm[AXIS], R);
         fast64::Side<NQ> l, r;
-        fast64::side<LAW, AXIS>(C, PL, l, ok);
-        fast64::side<LAW, AXIS>(C, PR, r, ok);
+        if constexpr (LAW == LAW_RMHD) {
+            fast64::rmhd_side<AXIS>(C, PL, l, ok);
+            fast64::rmhd_side<AXIS>(C, PR, r, ok);
+        } else {
+            fast64::side<LAW, AXIS>(C, PL, l, ok);
+            fast64::side<LAW, AXIS>(C, PR, r, ok);
+        }
         if constexpr (RIEMANN == RIEMANN_HLLC) {
             hllc<NQ>(L, R, nrm[AXIS], H);
             fast64::hllc<AXIS>(C, PL, PR, l, r, F, ok);
         } else {
             hlle<NQ>(L, R, H);
-            fast64::hlle<NQ>(l, r, F, ok);
+            for (int q = 0; q < NQ; ++q)
+                F[q] = fast64::hlle(l.ap, r.ap, l.am, r.am, l.F[q], r.F[q], l.U[q], r.U[q], ok);
         }
         if (!ok) continue;
         ++*accepted;
@@ -148,7 +161,12 @@ static void constants(PhysParams& pp, fast64::Consts& C, double (*nrm)[3], int w
     C.shenzha_A = 50.0;
     C.weno_is = weno;
     C.ny0 = n[1][0];
+    C.gamf = (gamma - 1.0) / gamma;
     C.gm1_div = ieee64::divisor(C.gm1, C.ok);
+    C.d3 = ieee64::divisor(3.0, C.ok);
+    C.d6 = ieee64::divisor(6.0, C.ok);
+    C.d9 = ieee64::divisor(9.0, C.ok);
+    C.d27 = ieee64::divisor(27.0, C.ok);
 }
 
 extern "C" long probe_faces(long n, u64 seed, int law, int recon, int riemann, int axis, int weno, double gamma,
@@ -171,6 +189,7 @@ extern "C" long probe_faces(long n, u64 seed, int law, int recon, int riemann, i
     if (law == LAW_HYDRO && riemann == RIEMANN_HLLC) { RECONS(LAW_HYDRO, RIEMANN_HLLC); }
     if (law == LAW_HYDRO) { RECONS(LAW_HYDRO, RIEMANN_HLLE); }
     if (law == LAW_MHD) { RECONS(LAW_MHD, RIEMANN_HLLE); }
+    if (law == LAW_RMHD) { RECONS(LAW_RMHD, RIEMANN_HLLE); }
     RECONS(LAW_MHD_COOL, RIEMANN_HLLE);
 }
 
@@ -182,14 +201,19 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
     for (long m = 0; m < n; ++m) {
         double base[NQ], P[NQ];
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
-        zone(kind, NQ, base, P);
+        zone(LAW, kind, NQ, base, P);
         bool ord = C.ok;
         for (int q = 0; q < NQ; ++q) ord = ord && fast64::ordinary_field(q, P[q]);
         double U[NQ], W[NQ];
         bool ok = ord;
-        law_p2u<LAW>(pp, P, U);
-        fast64::p2u<LAW>(C, P, W, ok);
         bool wrong = false;
+        const int ep = law_p2u<LAW>(pp, P, U);
+        if constexpr (LAW == LAW_RMHD) {
+            fast64::rmhd_p2u(C, P, W, ok);
+            wrong = ok && ep != ST_OK;
+        } else {
+            fast64::p2u<LAW>(C, P, W, ok);
+        }
         if (ok) for (int q = 0; q < NQ; ++q) wrong = wrong || !same(U[q], W[q]);
         *accepted += ok;
         // the same numbers as conserved densities, and the zone's own
@@ -199,7 +223,8 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
             for (int q = 0; q < NQ; ++q) { D[q] = t ? U[q] : P[q]; o2 = o2 && fast64::ordinary_field(q, D[q]); A[q] = 0; }
             int code = 0;
             const int e = law_cons<LAW>(pp, D, A, &code);
-            fast64::cons<LAW>(C, D, B, o2);
+            if constexpr (LAW == LAW_RMHD) fast64::rmhd_cons(C, D, B, o2);
+            else fast64::cons<LAW>(C, D, B, o2);
             if (o2) { wrong = wrong || e != ST_OK; for (int q = 0; q < NQ; ++q) wrong = wrong || !same(A[q], B[q]); }
         }
         double lmax = 0;
@@ -211,7 +236,12 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
             if (a == 0 || lmax < x) lmax = x;
         }
         ok = ord;
-        const double f = fast64::fastest<LAW>(C, P, ok);
+        double f;
+        if constexpr (LAW == LAW_RMHD) {
+            f = 0;
+            for (int a = 0; a < 3; ++a) { const double x = fast64::rmhd_fastest(C, P, a, ok); if (f < x) f = x; }
+        }
+        else f = fast64::fastest<LAW>(C, P, ok);
         if (ok) wrong = wrong || !same(f, lmax);
         bad += wrong;
     }
@@ -227,6 +257,7 @@ extern "C" long probe_zones(long n, u64 seed, int law, double gamma, int kind, l
     double nrm[3][3];
     constants(pp, C, nrm, WENO_SHENZHA10, gamma, 1.5);
     if (law == LAW_HYDRO) return zones<LAW_HYDRO>(n, pp, C, nrm, kind, accepted);
+    if (law == LAW_RMHD) return zones<LAW_RMHD>(n, pp, C, nrm, kind, accepted);
     if (law == LAW_MHD) return zones<LAW_MHD>(n, pp, C, nrm, kind, accepted);
     return zones<LAW_MHD_COOL>(n, pp, C, nrm, kind, accepted);
 }
@@ -256,3 +287,32 @@ extern "C" long probe_ieee(long n, u64 seed, long* accepted)
     }
     return bad;
 }
+
+#ifndef PROBE_IEEE_ONLY
+// ziv64.cuh against crmath.cuh: arc cosines, sines and cosines of their
+// thirds, cube roots
+extern "C" long probe_ziv(long n, u64 seed, long* accepted)
+{
+    state = seed;
+    *accepted = 0;
+    long bad = 0;
+    for (long m = 0; m < n; ++m) {
+        const double u = uni();
+        const double z = m % 4 == 0 ? 2 * u - 1 : m % 4 == 1 ? -1 + exp(-36 * u) : m % 4 == 2 ? 1 - exp(-10 * u)
+                                                             : (m % 8 == 3 ? -1.0 : (2 * u - 1) * exp(-20 * uni()));
+        bool ok = true;
+        const double a = ziv64::arccos(z, ok);
+        if (ok) { ++*accepted; bad += !same(a, crm::acos_cr(z)); }
+        const double t = m & 1 ? crm::acos_cr(z) / 3.0 : uni() * 1.05;
+        double c, s;
+        ok = true;
+        ziv64::sincos_third(t, c, s, ok);
+        if (ok) { ++*accepted; bad += !same(c, crm::cos_cr(t)) || !same(s, crm::sin_cr(t)); }
+        const double x = exp((uni() - 0.5) * (m & 1 ? 10 : 400));
+        ok = true;
+        const double y = ziv64::pow_third(x, ok);
+        if (ok) { ++*accepted; bad += !same(y, crm::pow_third(x)); }
+    }
+    return bad;
+}
+#endif

@@ -1,6 +1,6 @@
 """The plain path's forms with fewer FP64 operations (mara2_gb300/csrc/
-fast64.cuh, ieee64.cuh), built for the host, bit for bit the general ones
-(physics_fp64.cuh) and the host's own division, square root and product:
+fast64.cuh, fast64_rmhd.cuh, ieee64.cuh, ziv64.cuh), built for the host, bit for bit the general ones
+(physics_fp64.cuh, crmath.cuh) and the host's own division, square root and product:
 every law, reconstruction, solver, axis and smoothness indicator they cover,
 on seeded operands - smooth states, exact zeros of either sign and equal
 states, strong jumps, wide magnitudes, and any bit patterns (infinities, NaNs,
@@ -16,7 +16,7 @@ import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-HYDRO, MHD, MHD_COOL = 0, 1, 3
+HYDRO, MHD, RMHD, MHD_COOL = 0, 1, 2, 3
 SMOOTH, ZEROS, JUMPS, WIDE, ANY = range(5)
 
 
@@ -29,7 +29,7 @@ def _build(path, ulps, *flags):
                     "-I" + os.path.join(CUDA, "include"), os.path.join(ROOT, "tests", "fast64_probe.cpp"), "-o", so],
                    check=True)
     lib = C.CDLL(so)
-    for f in ("probe_ieee",) if flags else ("probe_faces", "probe_zones", "probe_ieee"):
+    for f in ("probe_ieee",) if flags else ("probe_faces", "probe_zones", "probe_ieee", "probe_ziv"):
         getattr(lib, f).restype = C.c_long
     return lib
 
@@ -47,7 +47,7 @@ def test_integer_division_root_and_product_round_correctly(tmp_path, ulps):
     assert acc.value > 2.8 * n
 
 
-CASES = [(HYDRO, r, s) for r in range(3) for s in range(2)] + [(law, r, 0) for law in (MHD, MHD_COOL) for r in range(3)]
+CASES = [(HYDRO, r, s) for r in range(3) for s in range(2)] + [(law, r, 0) for law in (MHD, RMHD, MHD_COOL) for r in range(3)]
 
 
 @pytest.mark.parametrize("law,recon,riemann", CASES)
@@ -64,7 +64,7 @@ def test_face_flux_has_the_general_forms_bits(lib, law, recon, riemann):
                     assert acc.value == n
 
 
-@pytest.mark.parametrize("law", [HYDRO, MHD, MHD_COOL])
+@pytest.mark.parametrize("law", [HYDRO, MHD, RMHD, MHD_COOL])
 def test_zone_conversions_and_wave_speeds_have_the_general_forms_bits(lib, law):
     n = 20000
     acc = C.c_long()
@@ -72,3 +72,10 @@ def test_zone_conversions_and_wave_speeds_have_the_general_forms_bits(lib, law):
         assert lib.probe_zones(C.c_long(n), C.c_ulonglong(kind), law, C.c_double(5.0 / 3), kind, C.byref(acc)) == 0
         if kind in (SMOOTH, ZEROS, JUMPS):
             assert acc.value == n
+
+
+def test_two_phase_functions_round_as_the_accurate_ones(lib):
+    n = 200000
+    acc = C.c_long()
+    assert lib.probe_ziv(C.c_long(n), C.c_ulonglong(3), C.byref(acc)) == 0
+    assert acc.value > 2.9 * n
