@@ -97,6 +97,30 @@ struct Consts {
     bool ok;                         // the constants themselves are ordinary
 };
 
+// The constants of a configuration, with the normals CartesianMeshGeometry
+// gives (ny0: its yhat's x component).
+static inline Consts make_consts(double gamma, double theta, double shenzha_A, int weno_is, double ny0)
+{
+    Consts c;
+    c.ok = true;
+    c.gamma = gamma;
+    c.gm1 = gamma - 1.0;
+    c.gamf = (gamma - 1.0) / gamma;
+    c.theta = theta;
+    c.shenzha_A = shenzha_A;
+    c.weno_is = weno_is;
+    c.ny0 = ny0;
+    c.gm1_div = ieee64::divisor(c.gm1, c.ok);
+    c.d3 = ieee64::divisor(3.0, c.ok);
+    c.d6 = ieee64::divisor(6.0, c.ok);
+    c.d9 = ieee64::divisor(9.0, c.ok);
+    c.d27 = ieee64::divisor(27.0, c.ok);
+    const double small = 1e-3, large = 1e3;
+    c.ok = c.ok && gamma > small && gamma < large && c.gm1 > small && theta > small && theta < large &&
+           shenzha_A >= 0.0 && shenzha_A < 1e9 && ny0 > 1e-20 && ny0 < small;
+    return c;
+}
+
 // ---------------------------------------------------------------------------
 // The generalised minmod's half slope, 0.5 minmod(theta, l, c, r), from its
 // one-sided differences a = theta (c - l), d = theta (r - c) and r - l.  The

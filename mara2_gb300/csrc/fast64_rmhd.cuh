@@ -280,9 +280,9 @@ F64_FN double rmhd_fastest(const Consts& c, const double* P, int a, bool& ok)
     return max_pos(ap, from_bits(mag(am)));
 }
 
-// rm_anton2dzw from rmhd_cons's start, with its reconstruction and checks;
-// ok cleared where it does not succeed
-F64_FN void rmhd_newton(const Consts& c, const double* U, double* P, bool& ok)
+// rm_anton2dzw with its reconstruction and checks, from rmhd_cons's start or
+// the given one (Z0 > 0); ok cleared where it does not succeed
+F64_FN void rmhd_newton(const Consts& c, const double* U, double* P, bool& ok, double Z0 = 0.0, double W0 = 0.0)
 {
     const double D = U[0], Tau = U[4];
     const double S2 = U[1] * U[1] + U[2] * U[2] + U[3] * U[3];
@@ -290,9 +290,11 @@ F64_FN void rmhd_newton(const Consts& c, const double* U, double* P, bool& ok)
     const double BS = U[5] * U[1] + U[6] * U[2] + U[7] * U[3];
     const double BS2 = BS * BS;
     const double g = c.gamf;
-    double Z = sqrt_rn(S2 + D * D, ok);
-    const Divisor vD = ieee64::divisor(D, ok);
-    double W = div(Z, vD, ok);
+    double Z = Z0, W = W0;
+    if (Z0 == 0.0) {
+        Z = sqrt_rn(S2 + D * D, ok);
+        W = div(Z, D, ok);
+    }
     double error = 1.0;
     int it = 0;
     while (ok && error > 1e-12) {

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "diagnostics.cuh"
+#include "fast64_rmhd.cuh"
 #include "hydro_cluster.cuh"
 #include "hydro_tile.cuh"
 #include "mixed.h"
@@ -638,8 +639,11 @@ constexpr int CONV_BLOCK = 256;
 
 template <int LAW, bool ACC64>
 __global__ void __launch_bounds__(CONV_BLOCK) load_kernel(const double* __restrict__ aos, long long c0, long long c1,
-                                                          float* Uh, float* Ul, float* Pf, GridF G, PhysParams pp,
-                                                          DevStatus* st, unsigned long long* cfl)
+                                                          float* Uh, float* Ul, float* Pf,
+                                                          const __grid_constant__ GridF G,
+                                                          const __grid_constant__ PhysParams pp,
+                                                          const __grid_constant__ fast64::Consts C, DevStatus* st,
+                                                          unsigned long long* cfl)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     __shared__ double slab[CONV_BLOCK * NQ];
@@ -665,6 +669,16 @@ __global__ void __launch_bounds__(CONV_BLOCK) load_kernel(const double* __restri
             double U[NQ];
             if constexpr (LAW == LAW_HYDRO) {
                 hydro_p2u_d(P, G.inv_gm1_d, U);
+            } else if constexpr (LAW == LAW_RMHD) {
+                // (RMHD 512^2 with general functions: 811 us, FP64-bound)
+                bool ok = C.ok;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, P[q]);
+                fast64::rmhd_p2u(C, P, U, ok);
+                if (!ok) {
+                    const int e = law_p2u<LAW>(pp, P, U);
+                    if (e != ST_OK) atomicCAS(&st->code, 0, e);
+                }
             } else {
                 const int e = law_p2u<LAW>(pp, P, U);
                 if (e != ST_OK) atomicCAS(&st->code, 0, e);
@@ -695,9 +709,12 @@ __global__ void __launch_bounds__(CONV_BLOCK) load_kernel(const double* __restri
 
 // FP64 primitives of cell c (AoS order) from the FP32-pair state; a guard
 // zone is the boundary image of an interior zone
+// (Pf: the general form's FP32 primitives, from which the relativistic
+// recovery starts, or null)
 template <int LAW, bool L2ONLY = false, bool ACC64 = false>
 __device__ __forceinline__ void store_cell(const float* Uh, const float* Ul, long long c, const GridF& G,
-                                           const PhysParams& pp, double* out)
+                                           const PhysParams& pp, double* out, const float* Pf = nullptr,
+                                           const fast64::Consts* C = nullptr)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     const int k = (int) (c % G.N[2]);
@@ -716,6 +733,23 @@ __device__ __forceinline__ void store_cell(const float* Uh, const float* Ul, lon
     }
     if constexpr (LAW == LAW_HYDRO) {
         hydro_u2p_d(U, G.gm1_d, P);
+    } else if constexpr (LAW == LAW_RMHD) {
+        // ConsToPrimRMHD's iteration from the zone's FP32 primitives, two
+        // iterations instead of about eight, to the same 1e-12 step; else
+        // from its own start
+        bool ok = C->ok;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, U[q]);
+        const long long pc = ((long long) (kk + G.g[2]) * G.N[1] + (jj + G.g[1])) * G.N[0] + (ii + G.g[0]);
+        const float rho = Pf[pc], v1 = Pf[G.sP + pc], v2 = Pf[2 * G.sP + pc], v3 = Pf[3 * G.sP + pc], pre = Pf[4 * G.sP + pc];
+        const float V2 = v1 * v1 + v2 * v2 + v3 * v3;
+        const float W2 = 1.0f / (1.0f - V2), Z = (rho + pre * G.rm_hcoef) * W2;
+        ok = ok && V2 < 1.0f && rho > 0.0f && pre > 0.0f && Z > 0.0f && Z < 1e30f;
+        fast64::rmhd_newton(*C, U, P, ok, (double) Z, (double) sqrtf(W2));
+        if (!ok) {
+            int code = 0;
+            law_cons<LAW>(pp, U, P, &code);
+        }
     } else {
         int code = 0;
         law_cons<LAW>(pp, U, P, &code);
@@ -731,13 +765,17 @@ __device__ __forceinline__ void store_cell(const float* Uh, const float* Ul, lon
 // block's slab written as one contiguous run
 template <int LAW, bool ACC64>
 __global__ void __launch_bounds__(CONV_BLOCK) store_kernel(const float* Uh, const float* Ul, double* __restrict__ aos,
-                                                           long long c0, long long c1, GridF G, PhysParams pp)
+                                                           long long c0, long long c1,
+                                                           const __grid_constant__ GridF G,
+                                                           const __grid_constant__ PhysParams pp,
+                                                           const float* __restrict__ Pf,
+                                                           const __grid_constant__ fast64::Consts C)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     __shared__ double slab[CONV_BLOCK * NQ];
     const long long b0 = c0 + blockIdx.x * (long long) CONV_BLOCK;
     const int nc = (int) min((long long) CONV_BLOCK, c1 - b0);
-    if (threadIdx.x < nc) store_cell<LAW, false, ACC64>(Uh, Ul, b0 + threadIdx.x, G, pp, &slab[threadIdx.x * NQ]);
+    if (threadIdx.x < nc) store_cell<LAW, false, ACC64>(Uh, Ul, b0 + threadIdx.x, G, pp, &slab[threadIdx.x * NQ], Pf, &C);
     __syncthreads();
     for (int e = threadIdx.x; e < nc * NQ; e += CONV_BLOCK) aos[b0 * NQ + e] = slab[e];
 }
@@ -807,6 +845,7 @@ struct MixedState {
     GridDesc G;
     GridF GF;
     PhysParams pp;
+    fast64::Consts fc;
     bool fused = false;
     bool acc64 = false;      // MARA_PRECISION_MIXED_FP64: Uh hold FP64 accumulators
     float* Uh[3] = {nullptr, nullptr, nullptr};
@@ -869,6 +908,7 @@ int mixed_create(const MaraGpuConfig* c, const GridDesc& G, MixedState** out, cu
     }
     m->pp.gamma = c->gamma; m->pp.plm_theta = c->plm_theta; m->pp.shenzha_A = c->shenzha_A;
     m->pp.pressure_floor = c->pressure_floor; m->pp.weno_is = c->weno_is;
+    m->fc = fast64::make_consts(c->gamma, c->plm_theta, c->shenzha_A, c->weno_is, G.nrm[1][0]);
 
     m->fused = c->law == MARA_LAW_HYDRO && G.n[2] == 1 && c->recon != MARA_RECON_WENO5 && G.n[0] > 1;
     m->acc64 = c->precision == MARA_PRECISION_MIXED_FP64;
@@ -988,15 +1028,15 @@ static void load_range(MixedState* m, const double* aos, long long c0, long long
     switch (m->cfg.law) {
         case MARA_LAW_HYDRO:
             // the fused form reduces the first Courant step here
-            load_kernel<LAW_HYDRO, ACC64><<<nb, 256, 0, s>>>(aos, c0, c1, m->Uh[r], m->Ul[r], m->Pf, m->GF, m->pp, st,
+            load_kernel<LAW_HYDRO, ACC64><<<nb, 256, 0, s>>>(aos, c0, c1, m->Uh[r], m->Ul[r], m->Pf, m->GF, m->pp, m->fc, st,
                                                              m->fused ? m->dcfl : nullptr);
             break;
         case MARA_LAW_MHD:
-            load_kernel<LAW_MHD, ACC64><<<nb, 256, 0, s>>>(aos, c0, c1, m->Uh[r], m->Ul[r], m->Pf, m->GF, m->pp, st,
+            load_kernel<LAW_MHD, ACC64><<<nb, 256, 0, s>>>(aos, c0, c1, m->Uh[r], m->Ul[r], m->Pf, m->GF, m->pp, m->fc, st,
                                                            nullptr);
             break;
         default:
-            load_kernel<LAW_RMHD, ACC64><<<nb, 256, 0, s>>>(aos, c0, c1, m->Uh[r], m->Ul[r], m->Pf, m->GF, m->pp, st,
+            load_kernel<LAW_RMHD, ACC64><<<nb, 256, 0, s>>>(aos, c0, c1, m->Uh[r], m->Ul[r], m->Pf, m->GF, m->pp, m->fc, st,
                                                             nullptr);
             break;
     }
@@ -1023,13 +1063,13 @@ static void store_range(MixedState* m, double* aos, long long c0, long long c1, 
     const int r = host_rot(m);
     switch (m->cfg.law) {
         case MARA_LAW_HYDRO:
-            store_kernel<LAW_HYDRO, ACC64><<<nb, 256, 0, s>>>(m->Uh[r], m->Ul[r], aos, c0, c1, m->GF, m->pp);
+            store_kernel<LAW_HYDRO, ACC64><<<nb, 256, 0, s>>>(m->Uh[r], m->Ul[r], aos, c0, c1, m->GF, m->pp, m->Pf, m->fc);
             break;
         case MARA_LAW_MHD:
-            store_kernel<LAW_MHD, ACC64><<<nb, 256, 0, s>>>(m->Uh[r], m->Ul[r], aos, c0, c1, m->GF, m->pp);
+            store_kernel<LAW_MHD, ACC64><<<nb, 256, 0, s>>>(m->Uh[r], m->Ul[r], aos, c0, c1, m->GF, m->pp, m->Pf, m->fc);
             break;
         default:
-            store_kernel<LAW_RMHD, ACC64><<<nb, 256, 0, s>>>(m->Uh[r], m->Ul[r], aos, c0, c1, m->GF, m->pp);
+            store_kernel<LAW_RMHD, ACC64><<<nb, 256, 0, s>>>(m->Uh[r], m->Ul[r], aos, c0, c1, m->GF, m->pp, m->Pf, m->fc);
             break;
     }
 }

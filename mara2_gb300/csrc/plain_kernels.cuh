@@ -622,24 +622,7 @@ static PhysParams to_dev(const PhysParamsH& h)
 
 static fast64::Consts to_fast(const PhysParamsH& h, const GridDesc& G)
 {
-    fast64::Consts c;
-    c.ok = true;
-    c.gamma = h.gamma;
-    c.gm1 = h.gamma - 1.0;
-    c.theta = h.plm_theta;
-    c.shenzha_A = h.shenzha_A;
-    c.weno_is = h.weno_is;
-    c.ny0 = G.nrm[1][0];
-    c.gamf = (h.gamma - 1.0) / h.gamma;
-    c.gm1_div = ieee64::divisor(c.gm1, c.ok);
-    c.d3 = ieee64::divisor(3.0, c.ok);
-    c.d6 = ieee64::divisor(6.0, c.ok);
-    c.d9 = ieee64::divisor(9.0, c.ok);
-    c.d27 = ieee64::divisor(27.0, c.ok);
-    // ordinary constants, the normals that fast64.cuh assumes
-    const double small = 1e-3, large = 1e3;
-    c.ok = c.ok && c.gamma > small && c.gamma < large && c.gm1 > small && c.theta > small && c.theta < large &&
-           c.shenzha_A >= 0.0 && c.shenzha_A < 1e9 && c.ny0 > 1e-20 && c.ny0 < small;
+    fast64::Consts c = fast64::make_consts(h.gamma, h.plm_theta, h.shenzha_A, h.weno_is, G.nrm[1][0]);
     for (int a = 0; a < 3; ++a)
         for (int d = 0; d < 3; ++d)
             if (!(a == 1 && d == 0)) c.ok = c.ok && G.nrm[a][d] == (a == d ? 1.0 : 0.0);

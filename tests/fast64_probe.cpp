@@ -154,19 +154,7 @@ static void constants(PhysParams& pp, fast64::Consts& C, double (*nrm)[3], int w
     pp.weno_is = weno;
     const double n[3][3] = {{1, 0, 0}, {cos(M_PI / 2), 1, 0}, {0, 0, 1}};
     memcpy(nrm, n, sizeof(n));
-    C.ok = true;
-    C.gamma = gamma;
-    C.gm1 = gamma - 1.0;
-    C.theta = theta;
-    C.shenzha_A = 50.0;
-    C.weno_is = weno;
-    C.ny0 = n[1][0];
-    C.gamf = (gamma - 1.0) / gamma;
-    C.gm1_div = ieee64::divisor(C.gm1, C.ok);
-    C.d3 = ieee64::divisor(3.0, C.ok);
-    C.d6 = ieee64::divisor(6.0, C.ok);
-    C.d9 = ieee64::divisor(9.0, C.ok);
-    C.d27 = ieee64::divisor(27.0, C.ok);
+    C = fast64::make_consts(gamma, theta, 50.0, weno, n[1][0]);
 }
 
 extern "C" long probe_faces(long n, u64 seed, int law, int recon, int riemann, int axis, int weno, double gamma,
