@@ -29,6 +29,7 @@ UNITS = {
     "plain_mhd.cu": ["--fmad=false"],
     "plain_mhd_cool.cu": ["--fmad=false"],
     "plain_rmhd.cu": ["--fmad=false"],
+    "plain_cluster.cu": ["--fmad=false"],
     "plain_fp64.cu": ["--fmad=false"],
     "mixed.cu": ["--fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],
     "batch.cu": ["--fmad=true", "-prec-div=false", "-prec-sqrt=false", "-ftz=true"],

@@ -56,7 +56,7 @@ struct PhysParamsH {
     double cooling_rate;
 };
 
-// ---- plain FP64 path (plain_fp64.cu) -----------------------------------------
+// ---- plain FP64 path (plain_*.cu) --------------------------------------------
 void plain_flux(int law, int recon, int riemann, int axis, const GridDesc& G, const PhysParamsH& pp,
                 const double* P, double* F, DevStatus* st, cudaStream_t s);
 void plain_update(int law, const GridDesc& G, const PhysParamsH& pp, const double* Pin, double* Pout,
@@ -65,6 +65,14 @@ void plain_update(int law, const GridDesc& G, const PhysParamsH& pp, const doubl
                   const double* S = nullptr);
 void plain_courant(int law, const GridDesc& G, const PhysParamsH& pp, const double* P, DevStatus* st,
                    cudaStream_t s);
+
+// nsteps driver-loop steps of a small 1-D hydro grid in one launch on a
+// cluster of ctas CTAs (plain_cluster_ctas; 0: not for this grid).  The state
+// is read from Pcur; it ends in Pother if an odd number of RK stages ran.
+int plain_cluster_ctas(int law, int recon, int riemann, const GridDesc& G);
+int plain_cluster_steps(int ctas, int recon, int riemann, const GridDesc& G, const PhysParamsH& pp, double* Pcur,
+                        double* Pother, double cfl, double t_final, int order, int nsteps, DevStatus* st,
+                        cudaStream_t s);
 
 // ---- diagnostics (diagnostics.cu) ----------------------------------------------
 void launch_monopole_max(const void* P, bool fp32, const GridDesc& G, double h, unsigned long long* out,

@@ -315,6 +315,7 @@ struct MaraGpuHandle {
     double* U0 = nullptr;
     double* U = nullptr;
     double* F[3] = {nullptr, nullptr, nullptr};
+    int cluster = 0;                     // CTAs of the 1-D plain path's cluster loop (0: none)
     double* stage_aos = nullptr;         // device AoS staging for transposes
     DevStatus* st = nullptr;
     DevStatus* st_host = nullptr;        // pinned mirror
@@ -619,6 +620,7 @@ int mara_gpu_create(const MaraGpuConfig* config, MaraGpuHandle** out)
         if (!rc) rc = alloc(h, (void**) &h->U, ubytes);
         for (int a = 0; a < 3 && !rc; ++a)
             if (G.n[a] > 1) rc = alloc(h, (void**) &h->F[a], fbytes);
+        if (!rc) h->cluster = plain_cluster_ctas(kernel_law(config), config->recon, config->riemann, G);
     } else if (!rc) {
         rc = mixed_create(config, G, &h->mixed, h->stream, &h->bytes);
     }
@@ -935,14 +937,33 @@ static int launches_per_run_step(MaraGpuHandle* h)
     return n + h->cfg.rk_order;
 }
 
+// whether the driver loop of this handle runs in launches of many steps
+static bool loop_on_cluster(MaraGpuHandle* h)
+{
+    if (h->timing) return false;
+    return h->mixed ? mixed_cluster_capable(h->mixed) : h->cluster != 0 && !h->src_fn;
+}
+
 static int enqueue_run(MaraGpuHandle* h, int max_steps, double cfl, double t_final)
 {
-    if (h->mixed && !h->timing && mixed_cluster_capable(h->mixed)) {
+    if (h->mixed && loop_on_cluster(h)) {
         // a small 1-D grid: chunks of steps, each one launch on a cluster
         for (int left = max_steps; left > 0; left -= CLUSTER_STEPS) {
             const int k = left < CLUSTER_STEPS ? left : CLUSTER_STEPS;
             const int rc = mixed_enqueue_cluster_steps(h->mixed, k, cfl, t_final, h->st, h->stream);
             if (rc) return rc;
+            h->steps += k;
+            h->launches++;
+        }
+        return cuda_status(cudaGetLastError());
+    }
+    if (loop_on_cluster(h)) {
+        for (int left = max_steps; left > 0; left -= CLUSTER_STEPS) {
+            const int k = left < CLUSTER_STEPS ? left : CLUSTER_STEPS;
+            const int rc = plain_cluster_steps(h->cluster, h->cfg.recon, h->cfg.riemann, h->G, h->pp, h->P[h->cur],
+                                               h->P[1 - h->cur], cfl, t_final, h->cfg.rk_order, k, h->st, h->stream);
+            if (rc) return rc;
+            h->cur = (h->cur + k * h->cfg.rk_order) & 1;
             h->steps += k;
             h->launches++;
         }
@@ -986,9 +1007,10 @@ int mara_gpu_run(MaraGpuHandle* h, int max_steps, double cfl, double t_final, do
     CK(cudaSetDevice(h->cfg.device));
     k_run_begin<<<1, 1, 0, h->stream>>>(h->st, *t);
     h->launches++;
-    // with an end time, look at the device's done flag every 64 steps so the
-    // host stops enqueuing once the run has reached t_final
-    const int chunk = t_final >= 0.0 ? 64 : max_steps;
+    // with an end time, look at the device's done flag every 64 steps (every
+    // launch of a cluster loop) so the host stops enqueuing once the run has
+    // reached t_final
+    const int chunk = t_final < 0.0 ? max_steps : loop_on_cluster(h) ? CLUSTER_STEPS : 64;
     int rc = MARA_OK;
     for (int left = max_steps; left > 0 && rc == MARA_OK; left -= chunk) {
         rc = enqueue_run(h, left < chunk ? left : chunk, cfl, t_final);

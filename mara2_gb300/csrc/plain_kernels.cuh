@@ -417,10 +417,20 @@ __device__ __forceinline__ double face_flux(const FluxView& V, const GridDesc& G
     return V.at(a, q, i, j, k);
 }
 
+// U0 (1 - b) + (U + dt L) b
+__device__ __forceinline__ double rk_combine_plain(double Uo, double Up, double L, double dt, double b)
+{
+    const double X = Up + fast64::mul_any(dt, L);
+    if (b == 1.0)   // U0 0 + X: a zero plus X (NaN for an infinite U0)
+        return fast64::expo(Uo) == 0x7ffu ? Uo * (1 - b) + X : fast64::add_zero(X, fast64::sign_bit(Uo));
+    if (b == 0.5) return times_pow2(Uo, -1) + times_pow2(X, -1);
+    if (b == 0.25) return Uo * (1 - b) + times_pow2(X, -2);
+    return Uo * (1 - b) + X * b;
+}
+
 // One RK stage's update of a zone (see the file's comment).  Bound by the
 // FP64 pipe, so the face area products of flat axes (zeros) are left out, and
-// the RK weights 1, 1/2 and 1/4 act on exponents; b1, b2: the weights of U0
-// and of the stage's result.
+// the RK weights 1, 1/2 and 1/4 act on exponents.
 // Resident blocks: hydro 1 to 5 a SM 5.60 ms, 8 5.39 (KH 1024^2, four steps);
 // MHD 1 3.94, 4 3.66, 5 3.57, 8 3.67 (64x56x48).
 template <int LAW>
@@ -465,7 +475,6 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
         for (int q = 0; q < NQ; ++q) { Uo[q] = U0[q * G.sU + uc]; Up[q] = U[q * G.sU + uc]; }
     }
 
-    const int pow2 = b == 1.0 ? 0 : b == 0.5 ? -1 : b == 0.25 ? -2 : 1;   // b 's exponent, 1: not a power of two
     bool fine = C.ok;
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
@@ -484,15 +493,7 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
             if (q == 8) L += Pc[4] / (pp.gamma - 1.0) * pp.cooling_rate;
         }
         if (S) L += S[q * G.sP + pc];  // the source terms function's array (SolutionSchemes.cpp:219-228)
-        const double X = Up[q] + fast64::mul_any(dt, L);
-        if (pow2 == 0) {
-            // U0 0 + X: a zero plus X (NaN for an infinite U0)
-            Un[q] = fast64::expo(Uo[q]) == 0x7ffu ? Uo[q] * (1 - b) + X : fast64::add_zero(X, fast64::sign_bit(Uo[q]));
-        } else if (pow2 < 0) {
-            Un[q] = (pow2 == -1 ? times_pow2(Uo[q], -1) : Uo[q] * (1 - b)) + times_pow2(X, pow2);
-        } else {
-            Un[q] = Uo[q] * (1 - b) + X * b;
-        }
+        Un[q] = rk_combine_plain(Uo[q], Up[q], L, dt, b);
         U[q * G.sU + uc] = Un[q];
         fine = fine && fast64::ordinary_field(q, Un[q]);
     }
