@@ -311,7 +311,7 @@ F64_FN void side(const Consts& c, const double* P, Side<LawInfo<LAW>::NQ>& S, bo
 F64_FN double hlle(double apl, double apr, double aml, double amr, double fl, double fr, double ul, double ur, bool& ok)
 {
     const double ap = max_pos(apl, apr), am = min_neg(aml, amr);
-    return div(ap * fl - am * fr + ap * am * (ur - ul), ap - am, ok);
+    return div(mul(ap, fl, ok) - mul(am, fr, ok) + ap * am * (ur - ul), ap - am, ok);
 }
 
 // the star state of the side the contact moves away from, chosen first

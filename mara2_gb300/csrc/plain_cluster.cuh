@@ -10,8 +10,8 @@
 // threads share the edge values by (zone, field), the states by (face, side),
 // the fluxes by (face, field), the RK combine by (zone, field) and the
 // recovery by zone, so that every scheduler's half lane of FP64 has work.
-// The Courant step of the new state is reduced across the cluster, so dt never
-// leaves it.  Arithmetic, dt sequence, clock and buffers are those of the step
+// The Courant step is reduced across the cluster between a step's first states
+// and its first update, so dt never leaves it.  Arithmetic, dt sequence, clock and buffers are those of the step
 // kernels (plain_kernels.cuh), bit for bit; hydro has no error codes.
 #pragma once
 
@@ -99,19 +99,6 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
         const int q = it / (mine + 2 * S), z = it - q * (mine + 2 * S) - S;
         Pbuf[q * W + S + z] = Pa[q * G.sP + G.g[0] + z0 + z];
     }
-    __syncthreads();
-    {
-        u64 v = 0;
-        for (int z = tid; z < mine; z += nt) {
-            double P[NQ];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) P[q] = Pbuf[q * W + S + z];
-            const u64 l = fastest(P);
-            v = l > v ? l : v;
-        }
-        reduce(v, 1);
-    }
-
     double t = st->t, dt = st->dt;
     u64 bits = 0;
     bool done = false, fresh = true;
@@ -122,23 +109,6 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
             double* Ps = Pbuf + par * NQ * W;
             double* Pn = Pbuf + (par ^ 1) * NQ * W;
             cluster.sync();
-            if (rk == 0) {
-                u64 l = 0;
-                for (int k = 0; k < nc; ++k) {
-                    const u64 o = cluster.map_shared_rank(red, k)[(step + 1) & 1];
-                    l = o > l ? o : l;
-                }
-                const double courant = G.lmin / __longlong_as_double((long long) l);
-                bits = (u64) __double_as_longlong(courant < DBL_MAX ? courant : DBL_MAX);
-                const double c = cfl * __longlong_as_double((long long) bits);
-                if (t_final >= 0.0) {
-                    if (!(t < t_final)) { done = true; break; }
-                    const double rest = t_final - t;
-                    dt = c < rest ? c : rest;
-                } else {
-                    dt = c;
-                }
-            }
             if (!fresh && tid < 2 * S) {
                 const int local = tid < S ? tid - S : mine + (tid - S);
                 int flip = 0;
@@ -171,22 +141,54 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
                 if (!ok) odd_zone[z] = 1;
             }
             __syncthreads();
-            for (int it = tid; it < 2 * (mine + 1); it += nt) {
-                const int s = it > mine ? 1 : 0, f = it - s * (mine + 1);
-                double P[NQ];
+            // the states of both sides of every face; at a step's start, on
+            // warps of their own, the zones' conserved densities and largest
+            // eigenvalues
+            const int sides = 2 * (mine + 1), warped = (sides + 31) / 32 * 32, zoned = (mine + 31) / 32 * 32;
+            u64 v = 0;
+            for (int it = tid; it < warped + (rk == 0 ? 2 * zoned : 0); it += nt) {
+                if (it < sides) {
+                    const int s = it > mine ? 1 : 0, f = it - s * (mine + 1);
+                    double P[NQ];
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) P[q] = E[((1 - s) * NQ + q) * (m + 2) + f + s];
-                fast64::Side<NQ> T;
-                bool ok = C.ok && !odd_zone[f + s];
-                fast64::hydro_side<0>(C, P, T, ok);
+                    for (int q = 0; q < NQ; ++q) P[q] = E[((1 - s) * NQ + q) * (m + 2) + f + s];
+                    fast64::Side<NQ> T;
+                    bool ok = C.ok && !odd_zone[f + s];
+                    fast64::hydro_side<0>(C, P, T, ok);
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    sU[(s * NQ + q) * (m + 1) + f] = T.U[q];
-                    sF[(s * NQ + q) * (m + 1) + f] = T.F[q];
+                    for (int q = 0; q < NQ; ++q) {
+                        sU[(s * NQ + q) * (m + 1) + f] = T.U[q];
+                        sF[(s * NQ + q) * (m + 1) + f] = T.F[q];
+                    }
+                    sA[(2 * s) * (m + 1) + f] = T.ap;
+                    sA[(2 * s + 1) * (m + 1) + f] = T.am;
+                    if (!ok) odd_face[f] = 1;
+                } else if (it >= warped) {
+                    const bool speeds = it >= warped + zoned;
+                    const int z = it - warped - (speeds ? zoned : 0);
+                    if (z >= mine) continue;
+                    double P[NQ];
+                    bool ok = C.ok;
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) {
+                        P[q] = Ps[q * W + S + z];
+                        ok = ok && fast64::ordinary_field(q, P[q]);
+                    }
+                    if (speeds) {
+                        const u64 l = fastest(P);
+                        v = l > v ? l : v;
+                    } else {
+                        double D[NQ];
+                        fast64::p2u<LAW_HYDRO>(C, P, D, ok);
+                        if (!ok) law_p2u<LAW_HYDRO>(pp, P, D);
+#pragma unroll
+                        for (int q = 0; q < NQ; ++q) U0[q * m + z] = U[q * m + z] = D[q];
+                    }
                 }
-                sA[(2 * s) * (m + 1) + f] = T.ap;
-                sA[(2 * s + 1) * (m + 1) + f] = T.am;
-                if (!ok) odd_face[f] = 1;
+            }
+            if (rk == 0) {
+                reduce(v, step & 1);
+                cluster.barrier_arrive();   // its wait: where dt is needed
             }
             __syncthreads();
             if constexpr (RIEMANN == RIEMANN_HLLE) {
@@ -231,18 +233,21 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
                                                             Fx + f, m + 1);
             }
             if (rk == 0) {
-                for (int z = tid; z < mine; z += nt) {
-                    double P[NQ], D[NQ];
-                    bool ok = C.ok;
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) {
-                        P[q] = Ps[q * W + S + z];
-                        ok = ok && fast64::ordinary_field(q, P[q]);
-                    }
-                    fast64::p2u<LAW_HYDRO>(C, P, D, ok);
-                    if (!ok) law_p2u<LAW_HYDRO>(pp, P, D);
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) U0[q * m + z] = U[q * m + z] = D[q];
+                cluster.barrier_wait();
+                u64 l = 0;
+                for (int k = 0; k < nc; ++k) {
+                    const u64 o = cluster.map_shared_rank(red, k)[step & 1];
+                    l = o > l ? o : l;
+                }
+                const double courant = G.lmin / __longlong_as_double((long long) l);
+                bits = (u64) __double_as_longlong(courant < DBL_MAX ? courant : DBL_MAX);
+                const double c = cfl * __longlong_as_double((long long) bits);
+                if (t_final >= 0.0) {
+                    if (!(t < t_final)) { done = true; break; }
+                    const double rest = t_final - t;
+                    dt = c < rest ? c : rest;
+                } else {
+                    dt = c;
                 }
             }
             __syncthreads();
@@ -253,7 +258,6 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
                 U[q * m + z] = rk_combine_plain(U0[q * m + z], U[q * m + z], fast64::mul_any(fv, sum), dt, b);
             }
             __syncthreads();
-            u64 v = 0;
             for (int z = tid; z < mine; z += nt) {
                 double D[NQ], P[NQ];
                 bool ok = C.ok;
@@ -269,12 +273,7 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
                 }
 #pragma unroll
                 for (int q = 0; q < NQ; ++q) Pn[q * W + S + z] = P[q];
-                if (rk == order - 1) {
-                    const u64 l = fastest(P);
-                    v = l > v ? l : v;
-                }
             }
-            if (rk == order - 1) reduce(v, step & 1);
         }
         if (done) break;
         t += dt;

@@ -253,7 +253,7 @@ __device__ __forceinline__ void zone_edges(const fast64::Consts& C, const double
         ok = ok && fast64::ordinary_field(q, p[0]);
     } else if constexpr (RECON == RECON_PLM) {
         const double l = p[-s], c = p[0], r = p[s];
-        const double h = fast64::half_slope(C.theta * (c - l), r - l, C.theta * (r - c));
+        const double h = fast64::half_slope(fast64::mul(C.theta, c - l), r - l, fast64::mul(C.theta, r - c));
         left = c - h;
         right = c + h;
         ok = ok && fast64::ordinary_field(q, l) && fast64::ordinary_field(q, c) && fast64::ordinary_field(q, r);
