@@ -930,9 +930,8 @@ static int build_run_graph(MaraGpuHandle* h, int which, double cfl, double t_fin
 
 static int launches_per_run_step(MaraGpuHandle* h)
 {
-    if (h->mixed && mixed_fused(h->mixed)) return mixed_launches_per_step(h->mixed);
+    if (h->mixed) return mixed_launches_per_step(h->mixed);
     int n = 2 /* courant init + courant */ + 2 /* dt, time */;
-    if (h->mixed) return n + mixed_launches_per_step(h->mixed);
     for (int a = 0; a < 3; ++a) if (h->G.n[a] > 1) n += h->cfg.rk_order;
     return n + h->cfg.rk_order;
 }

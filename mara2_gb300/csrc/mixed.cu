@@ -102,7 +102,11 @@ __global__ void __launch_bounds__(128) flux_f_kernel(const float* __restrict__ P
     else hlle_f<NQ>(L, R, Fh);
     const long long f = ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) F[q * G.sF + f] = Fh[q];
+    for (int q = 0; q < NQ; ++q) {
+        // under flux CT nothing reads the flux of the normal magnetic field
+        if (AXIS >= 0 && NQ == 8 && q == 5 + AXIS && G.ct) continue;
+        F[q * G.sF + f] = Fh[q];
+    }
 }
 
 struct FluxViewF {
@@ -493,7 +497,12 @@ __device__ __forceinline__ float zone_dt_f(const GridF& G, const float* P, DevSt
 // stage input and output may be one array, RK1).  Eight blocks per SM: the
 // kernel is bound by memory latency, and 32 resident warps with a few spilled
 // registers beat 20 warps without (MHD 256^3: 2.34e9 -> 2.64e9 zone-updates/s).
-template <int LAW, bool ACC64>
+//
+// LINEAR: the zones of a z-slice as one index space, where rows would leave
+// blocks partly empty (112 zones: an eighth; 130: almost half).  Rows cost
+// less registers, so they stay where they fill their blocks (RMHD 512^2, 16
+// steps: rows 4.25 ms, linear 4.34; hydro 112x90x75: 3.97 -> 3.55 linear).
+template <int LAW, bool ACC64, bool LINEAR>
 __global__ void __launch_bounds__(128, 8) update_f_kernel(float* __restrict__ Pf, const float* U0h, const float* U0l,
                                                        const float* Uph, const float* Upl, float* Unh, float* Unl,
                                                        FluxViewF V, GridF G,
@@ -504,9 +513,11 @@ __global__ void __launch_bounds__(128, 8) update_f_kernel(float* __restrict__ Pf
     constexpr int NQ = LawInfo<LAW>::NQ;
     pdl_chain();
     if (*done || st->code || st->halt) return;
-    const int ii = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = ii < G.n[0];
-    const int jj = blockIdx.y, kk = blockIdx.z;
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool active = lin < (LINEAR ? (unsigned) G.n[0] * (unsigned) G.n[1] : (unsigned) G.n[0]);
+    const int ii = LINEAR ? (int) (lin % (unsigned) G.n[0]) : (int) lin;
+    const int jj = LINEAR ? (int) (lin / (unsigned) G.n[0]) : (int) blockIdx.y;
+    const int kk = LINEAR ? blockIdx.y : blockIdx.z;
     const int i = ii + G.g[0], j = jj + G.g[1], k = kk + G.g[2];
     const long long uc = ((long long) kk * G.n[1] + jj) * G.n[0] + ii;
     const long long pc = ((long long) k * G.N[1] + j) * G.N[0] + i;
@@ -524,13 +535,10 @@ __global__ void __launch_bounds__(128, 8) update_f_kernel(float* __restrict__ Pf
         float Pold[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            if constexpr (ACC64) {
-                U0[q] = reinterpret_cast<const double*>(U0h)[q * G.sU + uc];
-                Up[q] = reinterpret_cast<const double*>(Uph)[q * G.sU + uc];
-            } else {
-                U0[q] = {U0h[q * G.sU + uc], U0l[q * G.sU + uc]};
-                Up[q] = {Uph[q * G.sU + uc], Upl[q * G.sU + uc]};
-            }
+            if constexpr (ACC64) Up[q] = reinterpret_cast<const double*>(Uph)[q * G.sU + uc];
+            else Up[q] = {Uph[q * G.sU + uc], Upl[q * G.sU + uc]};
+            if constexpr (ACC64) U0[q] = reinterpret_cast<const double*>(U0h)[q * G.sU + uc];
+            else U0[q] = {U0h[q * G.sU + uc], U0l[q * G.sU + uc]};
             if constexpr (LAW == LAW_RMHD) Pold[q] = Pf[q * G.sP + pc];
         }
 #pragma unroll
@@ -607,10 +615,11 @@ __global__ void __launch_bounds__(256) courant_f_kernel(const float* __restrict_
                                                         unsigned long long* __restrict__ dst, DevStatus* st)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
-    const int ii = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
     float zdt = 3.0e38f;
-    if (ii < G.n[0]) {
-        const long long pc = ((long long) (blockIdx.z + G.g[2]) * G.N[1] + (blockIdx.y + G.g[1])) * G.N[0] + (ii + G.g[0]);
+    if (lin < (unsigned) G.n[0] * (unsigned) G.n[1]) {
+        const int ii = (int) (lin % (unsigned) G.n[0]), jj = (int) (lin / (unsigned) G.n[0]);
+        const long long pc = ((long long) (blockIdx.y + G.g[2]) * G.N[1] + (jj + G.g[1])) * G.N[0] + (ii + G.g[0]);
         float P[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) P[q] = Pf[q * G.sP + pc];
@@ -804,6 +813,36 @@ __global__ void k_cfl_commit(unsigned long long* bits, const unsigned long long*
 {
     pdl_chain();
     if (!st->done && !st->code && !st->halt) *bits = *next;
+}
+
+// Start and end of one driver-loop step of the general form, in one thread
+// each: the Courant step becomes the handle's, dt, the reduction slot of the
+// last stage; then, if the step ran, its Courant step and the clock
+// (k_cfl_publish, k_dt_from_courant, k_cfl_reset; k_cfl_commit,
+// k_advance_time: six launches otherwise)
+__global__ void k_general_begin(const unsigned long long* bits, unsigned long long* next, DevStatus* st, double cfl,
+                                double t_final)
+{
+    pdl_chain();
+    *next = (unsigned long long) __double_as_longlong(DBL_MAX);
+    st->dt_bits = *bits;
+    if (st->done) return;
+    double dt = cfl * __longlong_as_double((long long) *bits);
+    if (t_final >= 0.0) {
+        if (!(st->t < t_final)) { st->done = 1; return; }
+        const double dt2 = t_final - st->t;
+        dt = dt < dt2 ? dt : dt2;
+    }
+    st->dt = dt;
+}
+__global__ void k_general_end(unsigned long long* bits, const unsigned long long* next, DevStatus* st)
+{
+    pdl_chain();
+    if (st->done || st->code) return;
+    if (!st->halt) *bits = *next;
+    st->t += st->dt;
+    st->steps += 1;
+    st->taken += 1;
 }
 
 // Start of one driver-loop step of the fused path, in one thread: the Courant
@@ -1006,7 +1045,7 @@ static int host_rot(const MixedState* m) { return m->rot; }
 
 static void courant_general(MixedState* m, DevStatus* st, cudaStream_t s)
 {
-    dim3 grid((m->G.n[0] + 255) / 256, m->G.n[1], m->G.n[2]);
+    dim3 grid((unsigned) (((long long) m->G.n[0] * m->G.n[1] + 255) / 256), m->G.n[2]);
     switch (m->cfg.law) {
         case MARA_LAW_HYDRO: courant_f_kernel<LAW_HYDRO><<<grid, 256, 0, s>>>(m->Pf, m->GF, m->dcfl, st); break;
         case MARA_LAW_MHD: courant_f_kernel<LAW_MHD><<<grid, 256, 0, s>>>(m->Pf, m->GF, m->dcfl, st); break;
@@ -1205,7 +1244,9 @@ static void flux_f(MixedState* m, int axis, const int* done, DevStatus* st, cuda
 static const float B_TAB[3][3] = {{1.f, 0.f, 0.f}, {1.f, 0.5f, 0.f}, {1.f, 0.25f, 2.f / 3.f}};
 
 
-static void general_step(MixedState* m, const double* dt, DevStatus* st, cudaStream_t s)
+// the stages; the last reduces the new state's Courant step into dcfl_next,
+// which the caller has reset and commits
+static void general_stages(MixedState* m, const double* dt, DevStatus* st, cudaStream_t s)
 {
     const int order = m->cfg.rk_order;
     const int* done = &st->done;
@@ -1216,6 +1257,10 @@ static void general_step(MixedState* m, const double* dt, DevStatus* st, cudaStr
     V.M0 = m->G.N[0] + 1;
     V.M1 = m->G.N[1] + 1;
     const int sb = 0, tb = 1;
+    const int n0 = m->G.n[0], blocks = (n0 + 127) / 128;
+    const bool linear = 16 * 128 * blocks > 17 * n0 && m->G.n[1] > 1;   // rows leave over 1/17 of their threads idle
+    const dim3 grid = linear ? dim3((unsigned) (((long long) n0 * m->G.n[1] + 127) / 128), m->G.n[2])
+                             : dim3(blocks, m->G.n[1], m->G.n[2]);
     for (int rk = 0; rk < order; ++rk) {
         for (int a = 0; a < 3; ++a) {
             if (m->G.n[a] <= 1) continue;
@@ -1238,28 +1283,37 @@ static void general_step(MixedState* m, const double* dt, DevStatus* st, cudaStr
         const int src = rk == 0 ? sb : tb;
         const int dst = rk == order - 1 ? sb : tb;
         const bool last = rk == order - 1;
-        // the last stage also reduces the new state's Courant step
-        if (last) chain_launch(k_cfl_reset, dim3(1), dim3(1), s, m->dcfl_next);
         unsigned long long* cfl = last ? m->dcfl_next : nullptr;
-        dim3 grid((m->G.n[0] + 127) / 128, m->G.n[1], m->G.n[2]);
         timed(m, s, [&] {
 #define MARA_UPDATE_ARGS m->Pf, m->Uh[sb], m->Ul[sb], m->Uh[src], m->Ul[src], m->Uh[dst], m->Ul[dst], V, m->GF, dt, b, 1.f - b, done, st, cfl
+#define MARA_UPDATE(LAW, ACC)                                                                                         \
+    do {                                                                                                              \
+        if (linear) chain_launch(update_f_kernel<LAW, ACC, true>, grid, dim3(128), s, MARA_UPDATE_ARGS);              \
+        else chain_launch(update_f_kernel<LAW, ACC, false>, grid, dim3(128), s, MARA_UPDATE_ARGS);                    \
+    } while (0)
             if (m->acc64) {
                 switch (m->cfg.law) {
-                    case MARA_LAW_HYDRO: chain_launch(update_f_kernel<LAW_HYDRO, true>, grid, dim3(128), s, MARA_UPDATE_ARGS); break;
-                    case MARA_LAW_MHD: chain_launch(update_f_kernel<LAW_MHD, true>, grid, dim3(128), s, MARA_UPDATE_ARGS); break;
-                    default: chain_launch(update_f_kernel<LAW_RMHD, true>, grid, dim3(128), s, MARA_UPDATE_ARGS); break;
+                    case MARA_LAW_HYDRO: MARA_UPDATE(LAW_HYDRO, true); break;
+                    case MARA_LAW_MHD: MARA_UPDATE(LAW_MHD, true); break;
+                    default: MARA_UPDATE(LAW_RMHD, true); break;
                 }
             } else {
                 switch (m->cfg.law) {
-                    case MARA_LAW_HYDRO: chain_launch(update_f_kernel<LAW_HYDRO, false>, grid, dim3(128), s, MARA_UPDATE_ARGS); break;
-                    case MARA_LAW_MHD: chain_launch(update_f_kernel<LAW_MHD, false>, grid, dim3(128), s, MARA_UPDATE_ARGS); break;
-                    default: chain_launch(update_f_kernel<LAW_RMHD, false>, grid, dim3(128), s, MARA_UPDATE_ARGS); break;
+                    case MARA_LAW_HYDRO: MARA_UPDATE(LAW_HYDRO, false); break;
+                    case MARA_LAW_MHD: MARA_UPDATE(LAW_MHD, false); break;
+                    default: MARA_UPDATE(LAW_RMHD, false); break;
                 }
             }
+#undef MARA_UPDATE
 #undef MARA_UPDATE_ARGS
         });
     }
+}
+
+static void general_step(MixedState* m, const double* dt, DevStatus* st, cudaStream_t s)
+{
+    chain_launch(k_cfl_reset, dim3(1), dim3(1), s, m->dcfl_next);
+    general_stages(m, dt, st, s);
     chain_launch(k_cfl_commit, dim3(1), dim3(1), s, m->dcfl, (const unsigned long long*) m->dcfl_next,
                  (const DevStatus*) st);
 }
@@ -1332,7 +1386,13 @@ void mixed_enqueue_step(MixedState* m, const double* dt, DevStatus* st, cudaStre
 
 bool mixed_enqueue_run_step(MixedState* m, double cfl, double t_final, DevStatus* st, cudaStream_t s)
 {
-    if (!m->fused) return false;
+    if (!m->fused) {
+        chain_launch(k_general_begin, dim3(1), dim3(1), s, (const unsigned long long*) m->dcfl, m->dcfl_next, st, cfl,
+                     t_final);
+        general_stages(m, &st->dt, st, s);
+        chain_launch(k_general_end, dim3(1), dim3(1), s, m->dcfl, (const unsigned long long*) m->dcfl_next, st);
+        return true;
+    }
     k_fused_run_begin<<<1, 1, 0, s>>>(m->dcfl, st, cfl, t_final);
     fused_step(m, &st->dt, st, s);
     if (m->cfg.rk_order == 1) m->rot ^= 1;
