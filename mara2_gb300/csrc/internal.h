@@ -57,8 +57,10 @@ struct PhysParamsH {
 };
 
 // ---- plain FP64 path (plain_*.cu) --------------------------------------------
-void plain_flux(int law, int recon, int riemann, int axis, const GridDesc& G, const PhysParamsH& pp,
-                const double* P, double* F, DevStatus* st, cudaStream_t s);
+// the face fluxes of every fleshed axis (F[a]), and its number of launches
+int plain_flux_launches(int law, int recon, int riemann, const GridDesc& G);
+void plain_flux(int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& pp, const double* P,
+                double* const* F, DevStatus* st, cudaStream_t s);
 void plain_update(int law, const GridDesc& G, const PhysParamsH& pp, const double* Pin, double* Pout,
                   double* U0, double* U, const double* Fx, const double* Fy, const double* Fz,
                   double b, int stage, const double* dt, DevStatus* st, cudaStream_t s,

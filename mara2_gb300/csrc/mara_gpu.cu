@@ -465,13 +465,12 @@ static void enqueue_plain_step(MaraGpuHandle* h)
     const MaraGpuConfig& c = h->cfg;
     const double* b = c.rk_order == 1 ? b1 : c.rk_order == 2 ? b2 : b3;
     for (int rk = 0; rk < c.rk_order; ++rk) {
-        for (int a = 0; a < 3; ++a) {
-            if (h->G.n[a] <= 1) continue;
+        {
             TimedPair tp;
             timed_begin(h, 0, tp);
-            plain_flux(kernel_law(&c), c.recon, c.riemann, a, h->G, h->pp, h->P[h->cur], h->F[a], h->st, h->stream);
+            plain_flux(kernel_law(&c), c.recon, c.riemann, h->G, h->pp, h->P[h->cur], h->F, h->st, h->stream);
             timed_end(h, tp);
-            h->launches++;
+            h->launches += plain_flux_launches(kernel_law(&h->cfg), h->cfg.recon, h->cfg.riemann, h->G);
         }
         const double* S = nullptr;
         if (h->src_fn) {
@@ -932,8 +931,7 @@ static int launches_per_run_step(MaraGpuHandle* h)
 {
     if (h->mixed) return mixed_launches_per_step(h->mixed);
     int n = 2 /* courant init + courant */ + 2 /* dt, time */;
-    for (int a = 0; a < 3; ++a) if (h->G.n[a] > 1) n += h->cfg.rk_order;
-    return n + h->cfg.rk_order;
+    return n + h->cfg.rk_order * (plain_flux_launches(kernel_law(&h->cfg), h->cfg.recon, h->cfg.riemann, h->G) + 1);
 }
 
 // whether the driver loop of this handle runs in launches of many steps

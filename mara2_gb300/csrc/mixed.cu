@@ -207,6 +207,15 @@ __device__ __forceinline__ int rm_reconstruct_rcp(const C2pRmhd& s, double Z, do
     return ST_OK;
 }
 
+// 1 / x, rounded to nearest, on the integer pipes where that holds
+__device__ __forceinline__ double rcp_rn(double x)
+{
+    bool ok = true;
+    double r = ieee64::div(1.0, x, ok);
+    if (!ok) r = 1.0 / x;
+    return r;
+}
+
 __device__ __forceinline__ int rm_anton2dzw_rcp(const C2pRmhd& s, double* P)
 {
     const int bad = rm_check_cons(s.Cons);
@@ -214,8 +223,8 @@ __device__ __forceinline__ int rm_anton2dzw_rcp(const C2pRmhd& s, double* P)
     int it = 0;
     double error = 1.0, W = s.W_start, Z = s.Z_start;
     const double D = s.D, Tau = s.Tau, S2 = s.S2, B2 = s.B2, BS2 = s.BS2, gamf = s.gamf;
-    const double iD = 1.0 / D;
-    double iW = 1.0 / W, iZ = 1.0 / Z;
+    const double iD = rcp_rn(D);
+    double iW = rcp_rn(W), iZ = rcp_rn(Z);
     while (error > 1e-12) {
         const double Z2 = Z * Z, Z3 = Z * Z2, W2 = W * W;
         const double iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
@@ -227,7 +236,7 @@ __device__ __forceinline__ int rm_anton2dzw_rcp(const C2pRmhd& s, double* P)
         const double df1dW = B2 * iW3 + (2 * Z - D * W) * iW3 * gamf;
         const double f0 = -S2 + BZ * BZ * (W2 - 1) * iW2 - (2 * Z + B2) * BS2 * iZ2;
         const double f1 = -Tau + Z + B2 - Pre - 0.5 * B2 * iW2 - 0.5 * BS2 * iZ2 - D;
-        const double idet = 1.0 / (df0dZ * df1dW - df0dW * df1dZ);
+        const double idet = rcp_rn(df0dZ * df1dW - df0dW * df1dZ);
         const double dZ = -(df1dW * f0 - df0dW * f1) * idet;
         const double dW = -(df0dZ * f1 - df1dZ * f0) * idet;
         double Z_new = Z + dZ;
@@ -238,8 +247,8 @@ __device__ __forceinline__ int rm_anton2dzw_rcp(const C2pRmhd& s, double* P)
         W_new = (W_new < 1e12) ? W_new : 1e12;
         Z = Z_new;
         W = W_new;
-        iZ = 1.0 / Z;
-        iW = 1.0 / W;
+        iZ = rcp_rn(Z);
+        iW = rcp_rn(W);
         error = fabs(dZ * iZ) + fabs(dW * iW);
         ++it;
         if (it == 250) return ST_C2P_MAXITER;

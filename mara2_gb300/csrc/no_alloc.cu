@@ -93,8 +93,7 @@ static int noalloc_advance(const MaraGpuConfig* config, const GridDesc& G, size_
     const double* b = config->rk_order == 1 ? b1 : config->rk_order == 2 ? b2 : b3;
     int c = 0;
     for (int rk = 0; rk < config->rk_order; ++rk) {
-        for (int a = 0; a < 3; ++a)
-            if (G.n[a] > 1) plain_flux(law, config->recon, config->riemann, a, G, pp, P[c], F[a], st, s);
+        plain_flux(law, config->recon, config->riemann, G, pp, P[c], F, st, s);
         plain_update(law, G, pp, P[c], P[1 - c], U0, U, F[0], F[1], F[2], b[rk], rk, &st->dt, st, s);
         c = 1 - c;
     }

@@ -9,14 +9,22 @@ MARA_PLAIN_LAW(extern, LAW_MHD);
 MARA_PLAIN_LAW(extern, LAW_MHD_COOL);
 MARA_PLAIN_LAW(extern, LAW_RMHD);
 
-void plain_flux(int law, int recon, int riemann, int axis, const GridDesc& G, const PhysParamsH& ph,
-                const double* P, double* F, DevStatus* st, cudaStream_t s)
+int plain_flux_launches(int law, int recon, int riemann, const GridDesc& G)
+{
+    int axes = 0;
+    for (int a = 0; a < 3; ++a) axes += G.n[a] > 1;
+    const bool runs = law == LAW_HYDRO && recon == RECON_PLM && (long long) G.n[0] * G.n[1] * G.n[2] >= HLLC_RUN_ZONES;
+    return riemann == RIEMANN_HLLC && (law != LAW_HYDRO || runs) ? axes : 1;
+}
+
+void plain_flux(int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& ph, const double* P,
+                double* const* F, DevStatus* st, cudaStream_t s)
 {
     switch (law) {
-        case LAW_HYDRO: plain_flux_law<LAW_HYDRO>(recon, riemann, axis, G, ph, P, F, st, s); break;
-        case LAW_MHD: plain_flux_law<LAW_MHD>(recon, riemann, axis, G, ph, P, F, st, s); break;
-        case LAW_MHD_COOL: plain_flux_law<LAW_MHD_COOL>(recon, riemann, axis, G, ph, P, F, st, s); break;
-        default: plain_flux_law<LAW_RMHD>(recon, riemann, axis, G, ph, P, F, st, s); break;
+        case LAW_HYDRO: plain_flux_law<LAW_HYDRO>(recon, riemann, G, ph, P, F, st, s); break;
+        case LAW_MHD: plain_flux_law<LAW_MHD>(recon, riemann, G, ph, P, F, st, s); break;
+        case LAW_MHD_COOL: plain_flux_law<LAW_MHD_COOL>(recon, riemann, G, ph, P, F, st, s); break;
+        default: plain_flux_law<LAW_RMHD>(recon, riemann, G, ph, P, F, st, s); break;
     }
 }
 

@@ -83,152 +83,41 @@ __device__ __noinline__ int face_general(const double* P, long long sP, long lon
     return ST_OK;
 }
 
-// The HLLC faces of one axis, each thread a run of consecutive faces along
-// it: a zone's reconstruction serves the faces on both of its sides.  Bound by
-// the FP64 pipe (fast64.cuh; KH 1024^2 421 -> about 185 us an axis, of which
-// the additions alone take 170); a face whose operands are not ordinary goes
-// through face_general, as do all faces of the magnetic laws, for which the
-// solver is not meant (AXIS < 0, the axis at run time).
-template <int LAW> constexpr bool HLLC_FAST = LAW == LAW_HYDRO;
-
+// The faces of one axis with the general functions: HLLC with a magnetic law,
+// which the solver is not meant for (it leaves the magnetic fluxes zero).
 struct FaceSpace {
     int lo[3];   // first face (right cell) and row of each axis
-    int nb[3];   // threads per axis: runs along the faces' axis, rows across it
-    int nf, run; // faces along the axis, faces per run
+    int nb[3];   // faces and rows per axis
     int axis;
 };
 
-// Three blocks per SM (168 registers): 4, 5 and 6 lose 1, 6 and 11 % to spills.
-template <int LAW, int RECON, int RIEMANN, int AXIS>
-__global__ void __launch_bounds__(128, AXIS < 0 ? 1 : 3) flux_kernel(const double* __restrict__ P, double* __restrict__ F,
-                                                   const __grid_constant__ GridDesc G,
-                                                   const __grid_constant__ PhysParams pp,
-                                                   const __grid_constant__ fast64::Consts C,
-                                                   const __grid_constant__ FaceSpace X, DevStatus* __restrict__ st)
+template <int LAW, int RECON, int RIEMANN>
+__global__ void __launch_bounds__(128) flux_general_kernel(const double* __restrict__ P, double* __restrict__ F,
+                                                           const __grid_constant__ GridDesc G,
+                                                           const __grid_constant__ PhysParams pp,
+                                                           const __grid_constant__ FaceSpace X,
+                                                           DevStatus* __restrict__ st)
 {
-    constexpr int NQ = LawInfo<LAW>::NQ;
-    constexpr int S = ReconInfo<RECON>::S;
     if (st->code != 0 || st->done) return;
     if (st->failures != 0) { st->halt = 1; return; }  // failures are final once the stage ended
-    // the threads of one z-slice as one index space (rows of n + 1 or n + 2
-    // faces would leave a nearly empty block per row)
     const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
     if (lin >= (unsigned) X.nb[0] * (unsigned) X.nb[1]) return;
-    const int axis = AXIS < 0 ? X.axis : AXIS;
-    int x[3] = {(int) (lin % (unsigned) X.nb[0]), (int) (lin / (unsigned) X.nb[0]), (int) blockIdx.y};
-    const int row = axis == 0 ? x[0] : axis == 1 ? x[1] : x[2];
-    const int first = row * X.run;
-    const int count = min(X.run, X.nf - first);
-    if (axis == 0) x[0] = first;
-    else if (axis == 1) x[1] = first;
-    else x[2] = first;
-    const int i = X.lo[0] + x[0], j = X.lo[1] + x[1], k = X.lo[2] + x[2];
-    const long long stride = axis == 0 ? 1 : axis == 1 ? (long long) G.N[0] : (long long) G.N[0] * G.N[1];
-    const long long fstride = axis == 0 ? 1 : axis == 1 ? (long long) (G.N[0] + 1) : (long long) (G.N[0] + 1) * (G.N[1] + 1);
-    const double* p = P + ((long long) k * G.N[1] + j) * G.N[0] + i;  // cell on the right of the face
-    double* f = F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
-
-    if constexpr (AXIS < 0) {
-        for (int m = 0; m < count; ++m, p += stride, f += fstride) {
-            const int e = face_general<LAW, RECON, RIEMANN>(p, G.sP, stride, G.nrm[axis][0], G.nrm[axis][1],
-                                                            G.nrm[axis][2], &pp, f, G.sF);
-            if (e != ST_OK) { record_status(st, e); return; }
-        }
-    } else {
-        // PL: the right edge of the zone on the face's left; d (PLM): the
-        // scaled difference across the face; fine: one bit per zone of the
-        // stencil, set where its values are ordinary
-        double PL[NQ], d[RECON == RECON_PLM ? NQ : 1];
-        unsigned fine = 0;
-        bool ok_left = true;
-#pragma unroll
-        for (int z = -S; z < S - 1; ++z) {
-            bool o = true;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const double v = p[q * G.sP + z * stride];
-                o = o && fast64::ordinary_field(q, v);
-            }
-            fine = 2 * fine + o;
-        }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const double* v = p + q * G.sP;
-            if constexpr (RECON == RECON_PCM) {
-                PL[q] = v[-stride];
-            } else if constexpr (RECON == RECON_PLM) {
-                const double a = C.theta * (v[-stride] - v[-2 * stride]);
-                d[q] = C.theta * (v[0] - v[-stride]);
-                PL[q] = v[-stride] + fast64::half_slope(a, v[0] - v[-2 * stride], d[q]);
-            } else {
-                const double w[5] = {v[-3 * stride], v[-2 * stride], v[-stride], v[0], v[stride]};
-                double left;
-                fast64::weno5_edges(C, &w[2], left, PL[q], ok_left);
-            }
-        }
-        for (int m = 0; m < count; ++m, p += stride, f += fstride) {
-            double PR[NQ], next[NQ];
-            bool ok = ok_left && C.ok, o = true;
-            ok_left = true;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                const double* v = p + q * G.sP;
-                if constexpr (RECON == RECON_PCM) {
-                    PR[q] = next[q] = v[0];
-                    o = o && fast64::ordinary_field(q, v[0]);
-                } else if constexpr (RECON == RECON_PLM) {
-                    const double c = v[0], r = v[stride];
-                    const double b = C.theta * (r - c);
-                    const double h = fast64::half_slope(d[q], r - v[-stride], b);
-                    d[q] = b;
-                    PR[q] = c - h;
-                    next[q] = c + h;
-                    o = o && fast64::ordinary_field(q, r);
-                } else {
-                    const double w[5] = {v[-2 * stride], v[-stride], v[0], v[stride], v[2 * stride]};
-                    fast64::weno5_edges(C, &w[2], PR[q], next[q], ok_left);
-                    o = o && fast64::ordinary_field(q, w[4]);
-                }
-            }
-            fine = 2 * fine + o;
-            ok = ok && ok_left && (fine & ((1u << 2 * S) - 1u)) == (1u << 2 * S) - 1u;
-            fast64::Side<NQ> L, R;
-            double Fh[NQ];
-            // the two sides in a loop: its code once (the kernels run out of
-            // the instruction cache; KH 1024^2 5.42 -> 5.27 ms, MHD 64x56x48
-            // 3.78 -> 3.58)
-            double Ps[NQ];
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) Ps[q] = PL[q];
-#pragma unroll 1
-            for (int s = 0; s < 2; ++s) {
-                fast64::side<LAW, AXIS>(C, Ps, R, ok);
-                if (s == 0) {
-                    L = R;
-#pragma unroll
-                    for (int q = 0; q < NQ; ++q) Ps[q] = PR[q];
-                }
-            }
-            fast64::hllc<AXIS>(C, PL, PR, L, R, Fh, ok);
-            if (ok) {
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) f[q * G.sF] = Fh[q];
-            } else {
-                const int e = face_general<LAW, RECON, RIEMANN>(p, G.sP, stride, G.nrm[AXIS][0], G.nrm[AXIS][1],
-                                                                G.nrm[AXIS][2], &pp, f, G.sF);
-                if (e != ST_OK) { record_status(st, e); return; }
-            }
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) PL[q] = next[q];
-        }
-    }
+    const int i = X.lo[0] + (int) (lin % (unsigned) X.nb[0]), j = X.lo[1] + (int) (lin / (unsigned) X.nb[0]);
+    const int k = X.lo[2] + (int) blockIdx.y;
+    const long long stride = X.axis == 0 ? 1 : X.axis == 1 ? (long long) G.N[0] : (long long) G.N[0] * G.N[1];
+    const double* n = G.nrm[X.axis];
+    const int e = face_general<LAW, RECON, RIEMANN>(P + ((long long) k * G.N[1] + j) * G.N[0] + i, G.sP, stride, n[0],
+                                                    n[1], n[2], &pp,
+                                                    F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i, G.sF);
+    if (e != ST_OK) record_status(st, e);
 }
 
 // ---------------------------------------------------------------------------
-// The same for HLLE, a block's threads sharing a tile of faces in three
+// The faces of one axis, a block's threads sharing a tile of them in three
 // phases through shared memory: the edge values of every (zone, field), the
-// state of every (face, side), the HLLE flux of every (face, field).  Each
-// phase is a short loop over independent items, so its code stays in the
+// state of every (face, side), the HLLE flux of every (face, field) or the
+// HLLC flux of every face.  A face whose operands are not ordinary
+// (fast64.cuh) goes through face_general.  Each phase is a short loop over independent items, so its code stays in the
 // instruction cache and small grids still fill the schedulers.  Bound by the
 // FP64 pipe (66 to 72 % busy).  Against a thread per run of faces: MHD
 // 64x56x48 115 to 138 -> 91 to 102 us an axis, a 1024-zone tube's run 2.95 ->
@@ -273,27 +162,21 @@ __device__ __forceinline__ void face_side(const fast64::Consts& C, const double*
     else fast64::side<LAW, AXIS>(C, P, S, ok);
 }
 
-template <int LAW, int RECON, int AXIS>
-__global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS) flux_tile_kernel(const double* __restrict__ P, double* __restrict__ F,
-                                                           const __grid_constant__ GridDesc G,
-                                                           const __grid_constant__ PhysParams pp,
-                                                           const __grid_constant__ fast64::Consts C,
-                                                           const __grid_constant__ TileSpace X,
-                                                           DevStatus* __restrict__ st)
+// a block's shared memory
+template <int NQ> struct TileShared {
+    double edge[2][NQ][TILE_ZONES];           // left and right edge of each zone
+    double U[2][NQ][TILE_FACES], F[2][NQ][TILE_FACES], A[2][2][TILE_FACES];   // states by side; ap, am
+    unsigned char odd_zone[TILE_ZONES], odd_face[TILE_FACES];                 // operands out of the ordinary
+};
+
+// tile b of the faces along AXIS
+template <int LAW, int RECON, int RIEMANN, int AXIS>
+__device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, const double* __restrict__ P,
+                                          double* __restrict__ F, const GridDesc& G, const PhysParams& pp,
+                                          const fast64::Consts& C, const TileSpace& X, int b, DevStatus* st)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
-    __shared__ double edge[2][NQ][TILE_ZONES];           // left and right edge of each zone
-    __shared__ double sU[2][NQ][TILE_FACES], sF[2][NQ][TILE_FACES], sA[2][2][TILE_FACES];
-    __shared__ unsigned char odd_zone[TILE_ZONES], odd_face[TILE_FACES];   // operands out of the ordinary
     const int tid = threadIdx.x;
-    for (int z = tid; z < TILE_ZONES; z += TILE_THREADS) odd_zone[z] = 0;
-    if (tid < TILE_FACES) odd_face[tid] = 0;
-    const int code = st->code, failures = st->failures;
-    if (__syncthreads_or(code != 0 || st->done || failures != 0)) {
-        if (code == 0 && failures != 0) st->halt = 1;    // failures are final once the stage ended
-        return;
-    }
-    const int b = blockIdx.x;
     const int a0 = (b % X.na) * X.len, c0 = (b / X.na) % X.nc * X.width, o = b / X.na / X.nc;
     const int len = min(X.len, X.nf - a0), width = min(X.width, X.ncol - c0);
     const int faces = len * width, zones = faces + width;
@@ -308,48 +191,212 @@ __global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS) flux_tile_ke
         bool ok = true;
         double l, r;
         zone_edges<RECON>(C, p + q * G.sP + (s - 1) * stride + w * cstride, stride, q, l, r, ok);
-        edge[0][q][z] = l;
-        edge[1][q][z] = r;
-        if (!ok) odd_zone[z] = 1;
+        sm.edge[0][q][z] = l;
+        sm.edge[1][q][z] = r;
+        if (!ok) sm.odd_zone[z] = 1;
     }
     __syncthreads();
     if (tid < 2 * faces) {
         const int s = tid >= faces ? 1 : 0, f = tid - s * faces, z = f + s * width;
         double Ps[NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) Ps[q] = edge[1 - s][q][z];
+        for (int q = 0; q < NQ; ++q) Ps[q] = sm.edge[1 - s][q][z];
         fast64::Side<NQ> S;
-        bool ok = C.ok && !odd_zone[z];
+        bool ok = C.ok && !sm.odd_zone[z];
         face_side<LAW, AXIS>(C, Ps, S, ok);
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
-            sU[s][q][f] = S.U[q];
-            sF[s][q][f] = S.F[q];
+            sm.U[s][q][f] = S.U[q];
+            sm.F[s][q][f] = S.F[q];
         }
-        sA[s][0][f] = S.ap;
-        sA[s][1][f] = S.am;
-        if (!ok) odd_face[f] = 1;
+        sm.A[s][0][f] = S.ap;
+        sm.A[s][1][f] = S.am;
+        if (!ok) sm.odd_face[f] = 1;
     }
     __syncthreads();
     const long long f0 = 1, f1 = G.N[0] + 1, f2 = (long long) (G.N[0] + 1) * (G.N[1] + 1);
     const long long fstride = AXIS == 0 ? f0 : AXIS == 1 ? f1 : f2, fcstride = AXIS == 0 ? f1 : f0;
     double* out = F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
-    for (int it = tid; it < NQ * faces; it += TILE_THREADS) {
-        const int q = it / faces, f = it - q * faces, s = f / width, w = f - s * width;
-        bool ok = !odd_face[f];
-        const double h = fast64::hlle(sA[0][0][f], sA[1][0][f], sA[0][1][f], sA[1][1][f], sF[0][q][f], sF[1][q][f],
-                                      sU[0][q][f], sU[1][q][f], ok);
+    if constexpr (RIEMANN == RIEMANN_HLLE) {
+        for (int it = tid; it < NQ * faces; it += TILE_THREADS) {
+            const int q = it / faces, f = it - q * faces, s = f / width, w = f - s * width;
+            bool ok = !sm.odd_face[f];
+            const double h = fast64::hlle(sm.A[0][0][f], sm.A[1][0][f], sm.A[0][1][f], sm.A[1][1][f], sm.F[0][q][f],
+                                          sm.F[1][q][f], sm.U[0][q][f], sm.U[1][q][f], ok);
+            double* to = out + s * fstride + w * fcstride;
+            if (ok) to[q * G.sF] = h;
+            else sm.odd_face[f] = 1;   // every field of the face by the general functions, below
+        }
+    } else if (tid < faces) {
+        // HLLC's star state couples the fields: a thread per face
+        const int f = tid, s = f / width, w = f - s * width;
+        double Pl[NQ], Pr[NQ], h[NQ];
+        fast64::Side<NQ> L, R;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            Pl[q] = sm.edge[1][q][f];
+            Pr[q] = sm.edge[0][q][f + width];
+            L.U[q] = sm.U[0][q][f];
+            R.U[q] = sm.U[1][q][f];
+            L.F[q] = sm.F[0][q][f];
+            R.F[q] = sm.F[1][q][f];
+        }
+        L.ap = sm.A[0][0][f];
+        L.am = sm.A[0][1][f];
+        R.ap = sm.A[1][0][f];
+        R.am = sm.A[1][1][f];
+        L.vn = fast64::along<AXIS>(C, Pl[1], Pl[2], Pl[3]);
+        R.vn = fast64::along<AXIS>(C, Pr[1], Pr[2], Pr[3]);
+        bool ok = !sm.odd_face[f];
+        fast64::hllc<AXIS>(C, Pl, Pr, L, R, h, ok);
         double* to = out + s * fstride + w * fcstride;
-        if (ok) to[q * G.sF] = h;
-        else odd_face[f] = 1;   // every field of the face by the general functions, below
+        if (ok) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) to[q * G.sF] = h[q];
+        } else {
+            sm.odd_face[f] = 1;
+        }
     }
     __syncthreads();
-    if (tid < faces && odd_face[tid]) {
+    if (tid < faces && sm.odd_face[tid]) {
         const int s = tid / width, w = tid - s * width;
-        const int e = face_general<LAW, RECON, RIEMANN_HLLE>(p + s * stride + w * cstride, G.sP, stride,
+        const int e = face_general<LAW, RECON, RIEMANN>(p + s * stride + w * cstride, G.sP, stride,
                                                              G.nrm[AXIS][0], G.nrm[AXIS][1], G.nrm[AXIS][2], &pp,
                                                              out + s * fstride + w * fcstride, G.sF);
         if (e != ST_OK) record_status(st, e);
+    }
+}
+
+// All axes in one launch: the tiles of axis a are blocks first[a] to
+// first[a + 1] - 1, so that small grids run their axes side by side.
+struct TileSpaces {
+    TileSpace axis[3];
+    int first[4];
+    double* F[3];
+};
+
+template <int LAW, int RECON, int RIEMANN>
+__global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS)
+    flux_tile_kernel(const double* __restrict__ P, const __grid_constant__ TileSpaces X,
+                     const __grid_constant__ GridDesc G, const __grid_constant__ PhysParams pp,
+                     const __grid_constant__ fast64::Consts C, DevStatus* __restrict__ st)
+{
+    __shared__ TileShared<LawInfo<LAW>::NQ> sm;
+    const int tid = threadIdx.x;
+    for (int z = tid; z < TILE_ZONES; z += TILE_THREADS) sm.odd_zone[z] = 0;
+    if (tid < TILE_FACES) sm.odd_face[tid] = 0;
+    const int code = st->code, failures = st->failures;
+    if (__syncthreads_or(code != 0 || st->done || failures != 0)) {
+        if (code == 0 && failures != 0) st->halt = 1;    // failures are final once the stage ended
+        return;
+    }
+    const int b = blockIdx.x;
+    if (b < X.first[1]) flux_tile<LAW, RECON, RIEMANN, 0>(sm, P, X.F[0], G, pp, C, X.axis[0], b, st);
+    else if (b < X.first[2]) flux_tile<LAW, RECON, RIEMANN, 1>(sm, P, X.F[1], G, pp, C, X.axis[1], b - X.first[1], st);
+    else flux_tile<LAW, RECON, RIEMANN, 2>(sm, P, X.F[2], G, pp, C, X.axis[2], b - X.first[2], st);
+}
+
+// ---------------------------------------------------------------------------
+// The PLM HLLC faces of one axis of a large hydro grid, each thread a run of
+// consecutive faces along it: a zone's slopes serve the faces on both of its
+// sides without a trip through shared memory.  Bound by the FP64 pipe (KH
+// 1024^2 658 to 714 -> about 185 us an axis, of which the additions alone
+// take 170).
+struct RunSpace {
+    int lo[3];   // first face (right cell) and row of each axis
+    int nb[3];   // threads per axis: runs along the faces' axis, rows across it
+    int nf, run; // faces along the axis, faces per run
+};
+
+// Three blocks per SM (168 registers): 4, 5 and 6 lose 1, 6 and 11 % to spills.
+template <int AXIS>
+__global__ void __launch_bounds__(128, 3) flux_run_kernel(const double* __restrict__ P, double* __restrict__ F,
+                                                          const __grid_constant__ GridDesc G,
+                                                          const __grid_constant__ PhysParams pp,
+                                                          const __grid_constant__ fast64::Consts C,
+                                                          const __grid_constant__ RunSpace X,
+                                                          DevStatus* __restrict__ st)
+{
+    constexpr int NQ = LawInfo<LAW_HYDRO>::NQ;
+    if (st->code != 0 || st->done) return;
+    if (st->failures != 0) { st->halt = 1; return; }  // failures are final once the stage ended
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin >= (unsigned) X.nb[0] * (unsigned) X.nb[1]) return;
+    int x[3] = {(int) (lin % (unsigned) X.nb[0]), (int) (lin / (unsigned) X.nb[0]), (int) blockIdx.y};
+    const int first = (AXIS == 0 ? x[0] : AXIS == 1 ? x[1] : x[2]) * X.run;
+    const int count = min(X.run, X.nf - first);
+    if (AXIS == 0) x[0] = first;
+    else if (AXIS == 1) x[1] = first;
+    else x[2] = first;
+    const int i = X.lo[0] + x[0], j = X.lo[1] + x[1], k = X.lo[2] + x[2];
+    const long long stride = AXIS == 0 ? 1 : AXIS == 1 ? (long long) G.N[0] : (long long) G.N[0] * G.N[1];
+    const long long fstride = AXIS == 0   ? 1
+                              : AXIS == 1 ? (long long) (G.N[0] + 1)
+                                          : (long long) (G.N[0] + 1) * (G.N[1] + 1);
+    const double* p = P + ((long long) k * G.N[1] + j) * G.N[0] + i;  // cell on the right of the face
+    double* f = F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
+
+    // PL: the right edge of the zone on the face's left; d: the scaled
+    // difference across the face; fine: one bit per zone of the stencil, set
+    // where its values are ordinary
+    double PL[NQ], d[NQ];
+    unsigned fine = 0;
+#pragma unroll
+    for (int z = -2; z < 1; ++z) {
+        bool o = true;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) o = o && fast64::ordinary_field(q, p[q * G.sP + z * stride]);
+        fine = 2 * fine + o;
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const double* v = p + q * G.sP;
+        const double a = C.theta * (v[-stride] - v[-2 * stride]);
+        d[q] = C.theta * (v[0] - v[-stride]);
+        PL[q] = v[-stride] + fast64::half_slope(a, v[0] - v[-2 * stride], d[q]);
+    }
+    for (int m = 0; m < count; ++m, p += stride, f += fstride) {
+        double PR[NQ], next[NQ];
+        bool o = true;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double* v = p + q * G.sP;
+            const double c = v[0], r = v[stride];
+            const double b = C.theta * (r - c);
+            const double h = fast64::half_slope(d[q], r - v[-stride], b);
+            d[q] = b;
+            PR[q] = c - h;
+            next[q] = c + h;
+            o = o && fast64::ordinary_field(q, r);
+        }
+        fine = 2 * fine + o;
+        bool ok = C.ok && (fine & 15u) == 15u;
+        // the two sides in a loop: its code once (the kernel runs out of the
+        // instruction cache; KH 1024^2, four steps, 5.42 -> 5.27 ms)
+        fast64::Side<NQ> L, R;
+        double Ps[NQ], h[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) Ps[q] = PL[q];
+#pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+            fast64::hydro_side<AXIS>(C, Ps, R, ok);
+            if (s == 0) {
+                L = R;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) Ps[q] = PR[q];
+            }
+        }
+        fast64::hllc<AXIS>(C, PL, PR, L, R, h, ok);
+        if (ok) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) f[q * G.sF] = h[q];
+        } else {
+            const int e = face_general<LAW_HYDRO, RECON_PLM, RIEMANN_HLLC>(p, G.sP, stride, G.nrm[AXIS][0],
+                                                                           G.nrm[AXIS][1], G.nrm[AXIS][2], &pp, f, G.sF);
+            if (e != ST_OK) { record_status(st, e); return; }
+        }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) PL[q] = next[q];
     }
 }
 
@@ -634,89 +681,113 @@ static fast64::Consts to_fast(const PhysParamsH& h, const GridDesc& G)
 // which has its own half lane of FP64 per clock.
 static int block_size(long long threads) { return threads <= 152ll * 4 * 32 ? 32 : 128; }
 
-template <int LAW, int RECON, int RIEMANN>
-static void flux_launch(int axis, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
-                        double* F, DevStatus* st, cudaStream_t s)
+// faces along the axis: the interior faces; across: interior rows, plus one
+// guard row per side on fleshed axes when flux CT is on
+static void face_rows(const GridDesc& G, int axis, int* lo, int* nb)
 {
-    // faces along the axis: the interior faces; across: interior rows, plus
-    // one guard row per side on fleshed axes when flux CT is on
-    if constexpr (RIEMANN == RIEMANN_HLLE) {
-        TileSpace T;
-        int nb[3];
-        for (int a = 0; a < 3; ++a) {
-            const int e = G.n[a] > 1 && a != axis && G.ct ? 1 : 0;
-            T.lo[a] = G.g[a] - e;
-            nb[a] = G.n[a] + 2 * e + (a == axis ? 1 : 0);
-        }
-        // across the tile: rows of y for faces along x, four zones of x (a
-        // 32-byte sector) otherwise; along it, equal lengths of at most 64 or 16
-        const int cross = axis == 0 ? 1 : 0, outer = axis == 2 ? 1 : 2;
-        const int most = axis == 0 ? TILE_FACES : TILE_FACES / 4;
-        T.nf = nb[axis];
-        T.ncol = nb[cross];
-        T.width = axis == 0 ? 1 : 4;
-        T.na = (T.nf + most - 1) / most;
-        T.len = (T.nf + T.na - 1) / T.na;
-        T.nc = (T.ncol + T.width - 1) / T.width;
-        const dim3 grid((unsigned) ((long long) T.na * T.nc * nb[outer]));
-        switch (axis) {
-            case 0: flux_tile_kernel<LAW, RECON, 0><<<grid, TILE_THREADS, 0, s>>>(P, F, G, pp, C, T, st); break;
-            case 1: flux_tile_kernel<LAW, RECON, 1><<<grid, TILE_THREADS, 0, s>>>(P, F, G, pp, C, T, st); break;
-            default: flux_tile_kernel<LAW, RECON, 2><<<grid, TILE_THREADS, 0, s>>>(P, F, G, pp, C, T, st); break;
-        }
-    } else {
-    FaceSpace X;
-    long long faces = 1;
     for (int a = 0; a < 3; ++a) {
-        if (a == axis) { X.lo[a] = G.g[a]; X.nb[a] = G.n[a] + 1; }
-        else if (G.n[a] > 1) { const int e = G.ct ? 1 : 0; X.lo[a] = G.g[a] - e; X.nb[a] = G.n[a] + 2 * e; }
-        else { X.lo[a] = 0; X.nb[a] = 1; }
-        faces *= X.nb[a];
+        const int e = G.n[a] > 1 && a != axis && G.ct ? 1 : 0;
+        lo[a] = G.g[a] - e;
+        nb[a] = G.n[a] + 2 * e + (a == axis ? 1 : 0);
     }
-    // a run of one forms every zone's reconstruction twice, one of eight 1/8
-    // too many: runs as long as four waves of resident threads remain (KH
-    // 1024^2, four steps: 5.42 ms at 4 faces a run, 5.61 at 8 and 2, 6.28 at 1)
-    X.nf = X.nb[axis];
-    X.run = 1;
-    if (HLLC_FAST<LAW> && RECON != RECON_PCM) {
-        const long long want = 152ll * 1536;
+}
+
+// From this size on a thread per run of faces (KH with PLM, tiles against
+// runs: 128^2, 16 steps 1.09 and 1.25 ms; 256^2, 16 steps 2.21 and 2.25;
+// 400^2, 8 steps 2.28 and 2.15; 1024^2, 4 steps 6.63 and 5.23; with WENO5 the
+// tiles win at all of them, 640^2 by 7.3 to 11.9)
+constexpr long long HLLC_RUN_ZONES = 1ll << 17;
+
+template <int LAW>
+static void flux_runs(const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
+                      double* const* F, DevStatus* st, cudaStream_t s)
+{
+    for (int axis = 0; axis < 3; ++axis) {
+        if (G.n[axis] <= 1) continue;
+        RunSpace X;
+        face_rows(G, axis, X.lo, X.nb);
+        // a run of one forms every zone's slopes twice, one of eight 1/8 too
+        // many: runs as long as four waves of resident threads remain (KH
+        // 1024^2, four steps: 5.42 ms at 4 faces a run, 5.61 at 8 and 2, 6.28 at 1)
+        const long long faces = (long long) X.nb[0] * X.nb[1] * X.nb[2], want = 152ll * 1536;
+        X.nf = X.nb[axis];
         X.run = (int) (faces < 2 * want ? 1 : faces > 8 * want ? 8 : faces / want);
-    }
-    X.nb[axis] = (X.nf + X.run - 1) / X.run;
-    const long long slice = (long long) X.nb[0] * X.nb[1];
-    const int block = block_size(slice * X.nb[2]);
-    const dim3 grid((unsigned) ((slice + block - 1) / block), X.nb[2]);
-    X.axis = axis;
-    if constexpr (!HLLC_FAST<LAW>) {
-        flux_kernel<LAW, RECON, RIEMANN, -1><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st);
-    } else {
+        X.nb[axis] = (X.nf + X.run - 1) / X.run;
+        const long long slice = (long long) X.nb[0] * X.nb[1];
+        const dim3 grid((unsigned) ((slice + 127) / 128), X.nb[2]);
         switch (axis) {
-            case 0: flux_kernel<LAW, RECON, RIEMANN, 0><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
-            case 1: flux_kernel<LAW, RECON, RIEMANN, 1><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
-            default: flux_kernel<LAW, RECON, RIEMANN, 2><<<grid, block, 0, s>>>(P, F, G, pp, C, X, st); break;
+            case 0: flux_run_kernel<0><<<grid, 128, 0, s>>>(P, F[0], G, pp, C, X, st); break;
+            case 1: flux_run_kernel<1><<<grid, 128, 0, s>>>(P, F[1], G, pp, C, X, st); break;
+            default: flux_run_kernel<2><<<grid, 128, 0, s>>>(P, F[2], G, pp, C, X, st); break;
         }
     }
+}
+
+template <int LAW, int RECON, int RIEMANN>
+static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
+                        double* const* F, DevStatus* st, cudaStream_t s)
+{
+    if constexpr (RIEMANN == RIEMANN_HLLC && LAW != LAW_HYDRO) {
+        for (int axis = 0; axis < 3; ++axis) {
+            if (G.n[axis] <= 1) continue;
+            FaceSpace X;
+            face_rows(G, axis, X.lo, X.nb);
+            X.axis = axis;
+            const long long slice = (long long) X.nb[0] * X.nb[1];
+            const int block = block_size(slice * X.nb[2]);
+            const dim3 grid((unsigned) ((slice + block - 1) / block), X.nb[2]);
+            flux_general_kernel<LAW, RECON, RIEMANN><<<grid, block, 0, s>>>(P, F[axis], G, pp, X, st);
+        }
+    } else {
+        if constexpr (LAW == LAW_HYDRO && RIEMANN == RIEMANN_HLLC && RECON == RECON_PLM) {
+            if ((long long) G.n[0] * G.n[1] * G.n[2] >= HLLC_RUN_ZONES) {
+                flux_runs<LAW>(G, pp, C, P, F, st, s);
+                return;
+            }
+        }
+        TileSpaces X;
+        X.first[0] = 0;
+        for (int axis = 0; axis < 3; ++axis) {
+            X.first[axis + 1] = X.first[axis];
+            X.F[axis] = F[axis];
+            if (G.n[axis] <= 1) continue;
+            TileSpace& T = X.axis[axis];
+            int nb[3];
+            face_rows(G, axis, T.lo, nb);
+            // across the tile: rows of y for faces along x, four zones of x (a
+            // 32-byte sector) otherwise; along it, tiles of equal length
+            const int cross = axis == 0 ? 1 : 0, outer = axis == 2 ? 1 : 2;
+            const int most = axis == 0 ? TILE_FACES : TILE_FACES / 4;
+            T.nf = nb[axis];
+            T.ncol = nb[cross];
+            T.width = axis == 0 ? 1 : 4;
+            T.na = (T.nf + most - 1) / most;
+            T.len = (T.nf + T.na - 1) / T.na;
+            T.nc = (T.ncol + T.width - 1) / T.width;
+            X.first[axis + 1] += T.na * T.nc * nb[outer];
+        }
+        flux_tile_kernel<LAW, RECON, RIEMANN><<<X.first[3], TILE_THREADS, 0, s>>>(P, X, G, pp, C, st);
     }
 }
 
 template <int LAW, int RECON>
-static void flux_dispatch_r(int riemann, int axis, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C,
-                            const double* P, double* F, DevStatus* st, cudaStream_t s)
+static void flux_dispatch_r(int riemann, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C,
+                            const double* P, double* const* F, DevStatus* st, cudaStream_t s)
 {
-    if (riemann == RIEMANN_HLLC) flux_launch<LAW, RECON, RIEMANN_HLLC>(axis, G, pp, C, P, F, st, s);
-    else flux_launch<LAW, RECON, RIEMANN_HLLE>(axis, G, pp, C, P, F, st, s);
+    if (riemann == RIEMANN_HLLC) flux_launch<LAW, RECON, RIEMANN_HLLC>(G, pp, C, P, F, st, s);
+    else flux_launch<LAW, RECON, RIEMANN_HLLE>(G, pp, C, P, F, st, s);
 }
 
 template <int LAW>
-void plain_flux_law(int recon, int riemann, int axis, const GridDesc& G, const PhysParamsH& ph, const double* P,
-                    double* F, DevStatus* st, cudaStream_t s)
+void plain_flux_law(int recon, int riemann, const GridDesc& G, const PhysParamsH& ph, const double* P, double* const* F,
+                    DevStatus* st, cudaStream_t s)
 {
     const PhysParams pp = to_dev(ph);
     const fast64::Consts C = to_fast(ph, G);
     switch (recon) {
-        case RECON_PCM: flux_dispatch_r<LAW, RECON_PCM>(riemann, axis, G, pp, C, P, F, st, s); break;
-        case RECON_PLM: flux_dispatch_r<LAW, RECON_PLM>(riemann, axis, G, pp, C, P, F, st, s); break;
-        default: flux_dispatch_r<LAW, RECON_WENO5>(riemann, axis, G, pp, C, P, F, st, s); break;
+        case RECON_PCM: flux_dispatch_r<LAW, RECON_PCM>(riemann, G, pp, C, P, F, st, s); break;
+        case RECON_PLM: flux_dispatch_r<LAW, RECON_PLM>(riemann, G, pp, C, P, F, st, s); break;
+        default: flux_dispatch_r<LAW, RECON_WENO5>(riemann, G, pp, C, P, F, st, s); break;
     }
 }
 
@@ -749,8 +820,8 @@ void plain_courant_law(const GridDesc& G, const PhysParamsH& ph, const double* P
 
 // one translation unit per law instantiates the kernels (plain_*.cu)
 #define MARA_PLAIN_LAW(EXTERN, LAW)                                                                                  \
-    EXTERN template void plain_flux_law<LAW>(int, int, int, const GridDesc&, const PhysParamsH&, const double*,      \
-                                             double*, DevStatus*, cudaStream_t);                                    \
+    EXTERN template void plain_flux_law<LAW>(int, int, const GridDesc&, const PhysParamsH&, const double*,           \
+                                             double* const*, DevStatus*, cudaStream_t);                                    \
     EXTERN template void plain_update_law<LAW>(const GridDesc&, const PhysParamsH&, const double*, double*, double*, \
                                                double*, const double*, const double*, const double*, double, int,   \
                                                const double*, DevStatus*, cudaStream_t, const double*);             \
