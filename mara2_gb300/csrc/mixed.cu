@@ -56,21 +56,28 @@ __device__ __forceinline__ void pdl_chain()
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// the faces of one axis: first face and rows, faces of a z-slice, z-slices
+struct FaceSpaceF {
+    int axis, lo0, lo1, lo2, nb0, nb1, nb2;
+    float* F;
+};
+struct FaceSpacesF {
+    FaceSpaceF a[3];
+};
+
 template <int LAW, int RECON, int RIEMANN, int AXIS>
-__global__ void __launch_bounds__(128) flux_f_kernel(const float* __restrict__ P, float* __restrict__ F, GridF G,
-                                                     int axis, int lo0, int lo1, int lo2, int nb0, int nb1,
-                                                     const int* __restrict__ done, DevStatus* st)
+__device__ __forceinline__ void flux_f_face(const float* __restrict__ P, const GridF& G, const FaceSpaceF& X,
+                                            DevStatus* st)
 {
-    pdl_chain();
-    if constexpr (AXIS >= 0) axis = AXIS;
+    float* __restrict__ F = X.F;
+    const int axis = AXIS >= 0 ? AXIS : X.axis;
+    const int lo0 = X.lo0, lo1 = X.lo1, lo2 = X.lo2, nb0 = X.nb0, nb1 = X.nb1;
     constexpr int NQ = LawInfo<LAW>::NQ;
     constexpr int S = SOf<RECON>::S;
-    if (*done || st->code) return;
-    if (st->failures) { st->halt = 1; return; }
     // the faces of one z-slice as one index space (rows of n + 1 or n + 2
     // faces would leave a nearly empty block per row)
     const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lin >= (unsigned) nb0 * (unsigned) nb1) return;
+    if (lin >= (unsigned) nb0 * (unsigned) nb1 || (int) blockIdx.y >= X.nb2) return;
     const int t = (int) (lin % (unsigned) nb0);
     const int i = lo0 + t, j = lo1 + (int) (lin / (unsigned) nb0), k = lo2 + blockIdx.y;
     const long long stride = axis == 0 ? 1 : axis == 1 ? (long long) G.N[0] : (long long) G.N[0] * G.N[1];
@@ -106,6 +113,29 @@ __global__ void __launch_bounds__(128) flux_f_kernel(const float* __restrict__ P
         // under flux CT nothing reads the flux of the normal magnetic field
         if (AXIS >= 0 && NQ == 8 && q == 5 + AXIS && G.ct) continue;
         F[q * G.sF + f] = Fh[q];
+    }
+}
+
+// The fluxes of every fleshed axis in one launch (blockIdx.z the axis): small
+// grids run their axes side by side, large ones have one last wave instead
+// of three.
+template <int LAW, int RECON, int RIEMANN>
+__global__ void __launch_bounds__(128) flux_f_kernel(const float* __restrict__ P, const __grid_constant__ FaceSpacesF X,
+                                                     const __grid_constant__ GridF G, const int* __restrict__ done,
+                                                     DevStatus* st)
+{
+    pdl_chain();
+    if (*done || st->code) return;
+    if (st->failures) { st->halt = 1; return; }
+    const FaceSpaceF& S = X.a[blockIdx.z];
+    // hydro and MHD fluxes take the axis at compile time; the relativistic
+    // law's cost is its quartic, so it keeps one code for all axes
+    if constexpr (LAW == LAW_RMHD) {
+        flux_f_face<LAW, RECON, RIEMANN, -1>(P, G, S, st);
+    } else {
+        if (S.axis == 0) flux_f_face<LAW, RECON, RIEMANN, 0>(P, G, S, st);
+        else if (S.axis == 1) flux_f_face<LAW, RECON, RIEMANN, 1>(P, G, S, st);
+        else flux_f_face<LAW, RECON, RIEMANN, 2>(P, G, S, st);
     }
 }
 
@@ -1208,45 +1238,41 @@ static void chain_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaSt
 }
 
 template <int LAW, int RECON, int RIEMANN>
-static void flux_f_launch(MixedState* m, int axis, const int* done, DevStatus* st, cudaStream_t s)
+static void flux_f_launch(MixedState* m, const int* done, DevStatus* st, cudaStream_t s)
 {
     const GridF& G = m->GF;
-    int lo[3], nb[3];
-    for (int a = 0; a < 3; ++a) {
-        if (a == axis) { lo[a] = G.g[a]; nb[a] = G.n[a] + 1; }
-        else if (G.n[a] > 1) { const int e = G.ct ? 1 : 0; lo[a] = G.g[a] - e; nb[a] = G.n[a] + 2 * e; }
-        else { lo[a] = 0; nb[a] = 1; }
-    }
-    dim3 grid((unsigned) (((long long) nb[0] * nb[1] + 127) / 128), nb[2]);
-#define MARA_FLUX_ARGS m->Pf, m->F[axis], G, axis, lo[0], lo[1], lo[2], nb[0], nb[1], done, st
-    // hydro and MHD fluxes take the axis at compile time; the relativistic
-    // law's cost is its quartic, so it keeps one kernel for all axes
-    if constexpr (LAW == LAW_RMHD) {
-        chain_launch(flux_f_kernel<LAW, RECON, RIEMANN, -1>, grid, dim3(128), s, MARA_FLUX_ARGS);
-    } else {
-        switch (axis) {
-            case 0: chain_launch(flux_f_kernel<LAW, RECON, RIEMANN, 0>, grid, dim3(128), s, MARA_FLUX_ARGS); break;
-            case 1: chain_launch(flux_f_kernel<LAW, RECON, RIEMANN, 1>, grid, dim3(128), s, MARA_FLUX_ARGS); break;
-            default: chain_launch(flux_f_kernel<LAW, RECON, RIEMANN, 2>, grid, dim3(128), s, MARA_FLUX_ARGS); break;
+    FaceSpacesF X;
+    unsigned axes = 0, blocks = 0, slices = 0;
+    for (int axis = 0; axis < 3; ++axis) {
+        if (G.n[axis] <= 1) continue;
+        int lo[3], nb[3];
+        for (int a = 0; a < 3; ++a) {
+            if (a == axis) { lo[a] = G.g[a]; nb[a] = G.n[a] + 1; }
+            else if (G.n[a] > 1) { const int e = G.ct ? 1 : 0; lo[a] = G.g[a] - e; nb[a] = G.n[a] + 2 * e; }
+            else { lo[a] = 0; nb[a] = 1; }
         }
+        X.a[axes++] = {axis, lo[0], lo[1], lo[2], nb[0], nb[1], nb[2], m->F[axis]};
+        blocks = std::max(blocks, (unsigned) (((long long) nb[0] * nb[1] + 127) / 128));
+        slices = std::max(slices, (unsigned) nb[2]);
     }
-#undef MARA_FLUX_ARGS
+    chain_launch(flux_f_kernel<LAW, RECON, RIEMANN>, dim3(blocks, slices, axes), dim3(128), s, (const float*) m->Pf, X, G,
+                 done, st);
 }
 
 template <int LAW, int RECON>
-static void flux_f_r(MixedState* m, int axis, const int* done, DevStatus* st, cudaStream_t s)
+static void flux_f_r(MixedState* m, const int* done, DevStatus* st, cudaStream_t s)
 {
-    if (m->cfg.riemann == MARA_RIEMANN_HLLC) flux_f_launch<LAW, RECON, RIEMANN_HLLC>(m, axis, done, st, s);
-    else flux_f_launch<LAW, RECON, RIEMANN_HLLE>(m, axis, done, st, s);
+    if (m->cfg.riemann == MARA_RIEMANN_HLLC) flux_f_launch<LAW, RECON, RIEMANN_HLLC>(m, done, st, s);
+    else flux_f_launch<LAW, RECON, RIEMANN_HLLE>(m, done, st, s);
 }
 
 template <int LAW>
-static void flux_f(MixedState* m, int axis, const int* done, DevStatus* st, cudaStream_t s)
+static void flux_f(MixedState* m, const int* done, DevStatus* st, cudaStream_t s)
 {
     switch (m->cfg.recon) {
-        case MARA_RECON_PCM: flux_f_r<LAW, RECON_PCM>(m, axis, done, st, s); break;
-        case MARA_RECON_PLM: flux_f_r<LAW, RECON_PLM>(m, axis, done, st, s); break;
-        default: flux_f_r<LAW, RECON_WENO5>(m, axis, done, st, s); break;
+        case MARA_RECON_PCM: flux_f_r<LAW, RECON_PCM>(m, done, st, s); break;
+        case MARA_RECON_PLM: flux_f_r<LAW, RECON_PLM>(m, done, st, s); break;
+        default: flux_f_r<LAW, RECON_WENO5>(m, done, st, s); break;
     }
 }
 
@@ -1271,16 +1297,13 @@ static void general_stages(MixedState* m, const double* dt, DevStatus* st, cudaS
     const dim3 grid = linear ? dim3((unsigned) (((long long) n0 * m->G.n[1] + 127) / 128), m->G.n[2])
                              : dim3(blocks, m->G.n[1], m->G.n[2]);
     for (int rk = 0; rk < order; ++rk) {
-        for (int a = 0; a < 3; ++a) {
-            if (m->G.n[a] <= 1) continue;
-            timed(m, s, [&] {
-                switch (m->cfg.law) {
-                    case MARA_LAW_HYDRO: flux_f<LAW_HYDRO>(m, a, done, st, s); break;
-                    case MARA_LAW_MHD: flux_f<LAW_MHD>(m, a, done, st, s); break;
-                    default: flux_f<LAW_RMHD>(m, a, done, st, s); break;
-                }
-            });
-        }
+        timed(m, s, [&] {
+            switch (m->cfg.law) {
+                case MARA_LAW_HYDRO: flux_f<LAW_HYDRO>(m, done, st, s); break;
+                case MARA_LAW_MHD: flux_f<LAW_MHD>(m, done, st, s); break;
+                default: flux_f<LAW_RMHD>(m, done, st, s); break;
+            }
+        });
         if (m->E[0]) {
             dim3 eg((unsigned) (((long long) V.M0 * V.M1 + 127) / 128), m->G.N[2] + 1);
             timed(m, s, [&] {
@@ -1873,11 +1896,9 @@ int mixed_launches_per_step(const MixedState* m)
 {
     // fused: the step-begin kernel, one launch per stage, the RK1 rotation
     if (m->fused) return 1 + m->cfg.rk_order + (m->cfg.rk_order == 1 ? 1 : 0);
-    // general: per stage the flux launches, the edge EMFs (flux CT), the
-    // update; per step the Courant slot's reset and commit
-    int axes = 0;
-    for (int a = 0; a < 3; ++a) axes += m->G.n[a] > 1;
-    return m->cfg.rk_order * (axes + 1 + (m->E[0] ? 1 : 0)) + 2;
+    // general: per stage the fluxes, the edge EMFs (flux CT), the update; per
+    // step the Courant slot's reset and commit
+    return m->cfg.rk_order * (2 + (m->E[0] ? 1 : 0)) + 2;
 }
 
 void mixed_enqueue_courant(MixedState* m, DevStatus* st, cudaStream_t s) { k_cfl_publish<<<1, 1, 0, s>>>(m->dcfl, st); }
