@@ -412,17 +412,26 @@ F64_FN double fastest(const Consts& c, const double* P, bool& ok)
     }
 }
 
+// a b on the FP64 pipe, in a branch (the asm keeps the compiler from issuing
+// it for every thread)
+F64_FN double mul_seldom(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+    double r;
+    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+#else
+    return a * b;
+#endif
+}
+
 // a b for any operands: on the FP64 pipe only where the integer product does
-// not hold (the asm keeps the compiler from issuing both)
+// not hold
 F64_FN double mul_any(double a, double b)
 {
     bool ok = true;
     double r = mul(a, b, ok);
-#if defined(__CUDA_ARCH__)
-    if (!ok) asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
-#else
-    if (!ok) r = a * b;
-#endif
+    if (!ok) r = mul_seldom(a, b);
     return r;
 }
 

@@ -119,7 +119,7 @@ F64_FN void rmhd_state(const Consts& c, const double* P, RmhdState& s, bool& ok)
     const double Bv = P[5] * P[1] + P[6] * P[2] + P[7] * P[3];
     s.vn = along<AXIS>(c, P[1], P[2], P[3]);
     s.Bn = along<AXIS>(c, P[5], P[6], P[7]);
-    ok = ok && s.vv < 1.0 && edge_pos(P[0]) && edge_pos(P[4]);
+    ok = ok && less(s.vv, 1.0) && edge_pos(P[0]) && edge_pos(P[4]);
     s.W2 = div(1.0, 1.0 - s.vv, ok);
     s.W0 = sqrt_rn(s.W2, ok);
     s.b0 = s.W0 * Bv;
@@ -297,7 +297,7 @@ F64_FN void rmhd_newton(const Consts& c, const double* U, double* P, bool& ok, d
     }
     double error = 1.0;
     int it = 0;
-    while (ok && error > 1e-12) {
+    while (ok && less(1e-12, error)) {
         const double Z2 = Z * Z, Z3 = Z * Z2, W2 = W * W, W3 = W * W2;
         const Divisor vW2 = ieee64::divisor(W2, ok), vW3 = ieee64::divisor(W3, ok);
         const Divisor vZ2 = ieee64::divisor(Z2, ok), vZ3 = ieee64::divisor(Z3, ok);
@@ -314,10 +314,10 @@ F64_FN void rmhd_newton(const Consts& c, const double* U, double* P, bool& ok, d
         const double dZ = -(G0 * f0 + G1 * f1);
         const double dW = -(G2 * f0 + G3 * f1);
         double Zn = Z + dZ, Wn = W + dW;
-        Zn = (Zn > 0.0) ? Zn : -Zn;
-        Zn = (Zn < 1e20) ? Zn : Z;
-        Wn = (Wn > 1.0) ? Wn : 1.0;
-        Wn = (Wn < 1e12) ? Wn : 1e12;
+        Zn = from_bits(mag(Zn));
+        Zn = less(Zn, 1e20) ? Zn : Z;
+        Wn = less(1.0, Wn) ? Wn : 1.0;
+        Wn = less(Wn, 1e12) ? Wn : 1e12;
         Z = Zn;
         W = Wn;
         error = fabs(div(dZ, Z, ok)) + fabs(div(dW, W, ok));
@@ -335,7 +335,7 @@ F64_FN void rmhd_newton(const Consts& c, const double* U, double* P, bool& ok, d
         P[5 + d] = U[5 + d];
     }
     const double v2 = P[1] * P[1] + P[2] * P[2] + P[3] * P[3];
-    ok = ok && v2 < 1.0 && P[4] > 0.0 && P[0] > 0.0;
+    ok = ok && less(v2, 1.0) && less(0.0, P[4]) && less(0.0, P[0]);
 }
 
 // rmhd_cons (U ordinary), with its closing eigenvalue check along x

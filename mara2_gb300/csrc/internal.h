@@ -63,7 +63,7 @@ void plain_flux(int law, int recon, int riemann, const GridDesc& G, const PhysPa
                 double* const* F, DevStatus* st, cudaStream_t s);
 void plain_update(int law, const GridDesc& G, const PhysParamsH& pp, const double* Pin, double* Pout,
                   double* U0, double* U, const double* Fx, const double* Fy, const double* Fz,
-                  double b, int stage, const double* dt, DevStatus* st, cudaStream_t s,
+                  int order, int stage, const double* dt, DevStatus* st, cudaStream_t s,
                   const double* S = nullptr);
 void plain_courant(int law, const GridDesc& G, const PhysParamsH& pp, const double* P, DevStatus* st,
                    cudaStream_t s);

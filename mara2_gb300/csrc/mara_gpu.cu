@@ -459,11 +459,7 @@ static void make_grid(const MaraGpuConfig* c, GridDesc* G)
 // from st->dt on the device.
 static void enqueue_plain_step(MaraGpuHandle* h)
 {
-    static const double b1[1] = {1.0};
-    static const double b2[2] = {1.0, 0.5};
-    static const double b3[3] = {1.0, 1. / 4, 2. / 3};
     const MaraGpuConfig& c = h->cfg;
-    const double* b = c.rk_order == 1 ? b1 : c.rk_order == 2 ? b2 : b3;
     for (int rk = 0; rk < c.rk_order; ++rk) {
         {
             TimedPair tp;
@@ -494,7 +490,7 @@ static void enqueue_plain_step(MaraGpuHandle* h)
         TimedPair tp;
         timed_begin(h, 1, tp);
         plain_update(kernel_law(&c), h->G, h->pp, h->P[h->cur], h->P[1 - h->cur], h->U0, h->U, h->F[0], h->F[1], h->F[2],
-                     b[rk], rk, &h->st->dt, h->st, h->stream, S);
+                     c.rk_order, rk, &h->st->dt, h->st, h->stream, S);
         timed_end(h, tp);
         h->launches++;
         h->cur = 1 - h->cur;

@@ -87,14 +87,10 @@ static int noalloc_advance(const MaraGpuConfig* config, const GridDesc& G, size_
     launch_aos_to_soa(P_in, P[0], G, s);
 
     // the RK stages of MethodOfLinesTVD::advance (SolutionSchemes.cpp:191-274)
-    static const double b1[1] = {1.0};
-    static const double b2[2] = {1.0, 0.5};
-    static const double b3[3] = {1.0, 1. / 4, 2. / 3};
-    const double* b = config->rk_order == 1 ? b1 : config->rk_order == 2 ? b2 : b3;
     int c = 0;
     for (int rk = 0; rk < config->rk_order; ++rk) {
         plain_flux(law, config->recon, config->riemann, G, pp, P[c], F, st, s);
-        plain_update(law, G, pp, P[c], P[1 - c], U0, U, F[0], F[1], F[2], b[rk], rk, &st->dt, st, s);
+        plain_update(law, G, pp, P[c], P[1 - c], U0, U, F[0], F[1], F[2], config->rk_order, rk, &st->dt, st, s);
         c = 1 - c;
     }
     launch_soa_to_aos(P[c], P_out, G, s);

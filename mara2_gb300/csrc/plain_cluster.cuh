@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
     int par = 0, step = 0;
     for (; step < nsteps; ++step) {
         for (int rk = 0; rk < order; ++rk, par ^= 1, fresh = false) {
-            const double b = order == 1 ? 1.0 : order == 2 ? (rk == 0 ? 1.0 : 0.5) : rk == 0 ? 1.0 : rk == 1 ? 1. / 4 : 2. / 3;
+            const RkWeight w = rk_weight(order, rk);
             double* Ps = Pbuf + par * NQ * W;
             double* Pn = Pbuf + (par ^ 1) * NQ * W;
             cluster.sync();
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
                 const int q = it / mine, z = it - q * mine;
                 const double sum = fast64::add_zero(fast64::mul_any(Fx[q * (m + 1) + z + 1], G.dA[0]) -
                                                     fast64::mul_any(Fx[q * (m + 1) + z], G.dA[0]), false);
-                U[q * m + z] = rk_combine_plain(U0[q * m + z], U[q * m + z], fast64::mul_any(fv, sum), dt, b);
+                U[q * m + z] = rk_combine_plain(U0[q * m + z], U[q * m + z], fast64::mul_any(fv, sum), dt, w);
             }
             __syncthreads();
             for (int z = tid; z < mine; z += nt) {

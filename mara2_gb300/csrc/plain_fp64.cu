@@ -30,13 +30,13 @@ void plain_flux(int law, int recon, int riemann, const GridDesc& G, const PhysPa
 
 void plain_update(int law, const GridDesc& G, const PhysParamsH& ph, const double* Pin, double* Pout,
                   double* U0, double* U, const double* Fx, const double* Fy, const double* Fz,
-                  double b, int stage, const double* dt, DevStatus* st, cudaStream_t s, const double* S)
+                  int order, int stage, const double* dt, DevStatus* st, cudaStream_t s, const double* S)
 {
     switch (law) {
-        case LAW_HYDRO: plain_update_law<LAW_HYDRO>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, b, stage, dt, st, s, S); break;
-        case LAW_MHD: plain_update_law<LAW_MHD>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, b, stage, dt, st, s, S); break;
-        case LAW_MHD_COOL: plain_update_law<LAW_MHD_COOL>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, b, stage, dt, st, s, S); break;
-        default: plain_update_law<LAW_RMHD>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, b, stage, dt, st, s, S); break;
+        case LAW_HYDRO: plain_update_law<LAW_HYDRO>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, order, stage, dt, st, s, S); break;
+        case LAW_MHD: plain_update_law<LAW_MHD>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, order, stage, dt, st, s, S); break;
+        case LAW_MHD_COOL: plain_update_law<LAW_MHD_COOL>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, order, stage, dt, st, s, S); break;
+        default: plain_update_law<LAW_RMHD>(G, ph, Pin, Pout, U0, U, Fx, Fy, Fz, order, stage, dt, st, s, S); break;
     }
 }
 

@@ -417,7 +417,8 @@ __device__ __forceinline__ double times_pow2(double x, int k)
     const unsigned e = fast64::expo(x);
     if (e - 1u < 2046u && e + (unsigned) k - 1u < 2046u)
         return fast64::from_bits(fast64::bits(x) + ((unsigned long long) (long long) k << 52));
-    return fast64::is_zero(x) ? x : x * (k == 1 ? 2.0 : k == -1 ? 0.5 : k == -2 ? 0.25 : 0.125);
+    if (fast64::is_zero(x)) return x;
+    return fast64::mul_seldom(x, k == 1 ? 2.0 : k == -1 ? 0.5 : k == -2 ? 0.25 : 0.125);
 }
 
 // Flux of field q through the face of axis a at flux index (i, j, k), after
@@ -464,15 +465,26 @@ __device__ __forceinline__ double face_flux(const FluxView& V, const GridDesc& G
     return V.at(a, q, i, j, k);
 }
 
+// The weight b of an RK stage (SolutionSchemes.cpp:135-138) and 1 - b.
+struct RkWeight {
+    int kind;        // 0: b = 1, 1: 1/2, 2: 1/4, 3: any
+    double b, rest;
+};
+__host__ __device__ inline RkWeight rk_weight(int order, int stage)
+{
+    const double b = order == 1 || stage == 0 ? 1.0 : order == 2 ? 0.5 : stage == 1 ? 1. / 4 : 2. / 3;
+    return {b == 1.0 ? 0 : b == 0.5 ? 1 : b == 0.25 ? 2 : 3, b, 1 - b};
+}
+
 // U0 (1 - b) + (U + dt L) b
-__device__ __forceinline__ double rk_combine_plain(double Uo, double Up, double L, double dt, double b)
+__device__ __forceinline__ double rk_combine_plain(double Uo, double Up, double L, double dt, const RkWeight& w)
 {
     const double X = Up + fast64::mul_any(dt, L);
-    if (b == 1.0)   // U0 0 + X: a zero plus X (NaN for an infinite U0)
-        return fast64::expo(Uo) == 0x7ffu ? Uo * (1 - b) + X : fast64::add_zero(X, fast64::sign_bit(Uo));
-    if (b == 0.5) return times_pow2(Uo, -1) + times_pow2(X, -1);
-    if (b == 0.25) return Uo * (1 - b) + times_pow2(X, -2);
-    return Uo * (1 - b) + X * b;
+    if (w.kind == 0)   // U0 0 + X: a zero plus X (NaN for an infinite U0)
+        return fast64::expo(Uo) == 0x7ffu ? Uo * w.rest + X : fast64::add_zero(X, fast64::sign_bit(Uo));
+    if (w.kind == 1) return times_pow2(Uo, -1) + times_pow2(X, -1);
+    if (w.kind == 2) return fast64::mul_any(Uo, w.rest) + times_pow2(X, -2);
+    return fast64::mul_any(Uo, w.rest) + fast64::mul_any(X, w.b);
 }
 
 // One RK stage's update of a zone (see the file's comment).  Bound by the
@@ -486,8 +498,8 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
                                                      const __grid_constant__ FluxView V,
                                                      const __grid_constant__ GridDesc G,
                                                      const __grid_constant__ PhysParams pp,
-                                                     const __grid_constant__ fast64::Consts C, double fv, double b,
-                                                     int stage, const double* __restrict__ dtp,
+                                                     const __grid_constant__ fast64::Consts C, double fv,
+                                                     const __grid_constant__ RkWeight w, int stage, const double* __restrict__ dtp,
                                                      DevStatus* __restrict__ st, const double* __restrict__ S)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
@@ -540,7 +552,7 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
             if (q == 8) L += Pc[4] / (pp.gamma - 1.0) * pp.cooling_rate;
         }
         if (S) L += S[q * G.sP + pc];  // the source terms function's array (SolutionSchemes.cpp:219-228)
-        Un[q] = rk_combine_plain(Uo[q], Up[q], L, dt, b);
+        Un[q] = rk_combine_plain(Uo[q], Up[q], L, dt, w);
         U[q * G.sU + uc] = Un[q];
         fine = fine && fast64::ordinary_field(q, Un[q]);
     }
@@ -793,9 +805,10 @@ void plain_flux_law(int recon, int riemann, const GridDesc& G, const PhysParamsH
 
 template <int LAW>
 void plain_update_law(const GridDesc& G, const PhysParamsH& ph, const double* Pin, double* Pout, double* U0, double* U,
-                      const double* Fx, const double* Fy, const double* Fz, double b, int stage, const double* dt,
+                      const double* Fx, const double* Fy, const double* Fz, int order, int stage, const double* dt,
                       DevStatus* st, cudaStream_t s, const double* S)
 {
+    const RkWeight w = rk_weight(order, stage);
     FluxView V;
     V.F[0] = Fx; V.F[1] = Fy; V.F[2] = Fz;
     V.sF = G.sF;
@@ -805,7 +818,7 @@ void plain_update_law(const GridDesc& G, const PhysParamsH& ph, const double* Pi
     const long long slice = (long long) G.n[0] * G.n[1];
     const int block = block_size(slice * G.n[2]);
     const dim3 grid((unsigned) ((slice + block - 1) / block), G.n[2]);
-    update_kernel<LAW><<<grid, block, 0, s>>>(Pin, Pout, U0, U, V, G, to_dev(ph), to_fast(ph, G), factor / G.dV, b,
+    update_kernel<LAW><<<grid, block, 0, s>>>(Pin, Pout, U0, U, V, G, to_dev(ph), to_fast(ph, G), factor / G.dV, w,
                                               stage, dt, st, S);
 }
 
@@ -823,7 +836,7 @@ void plain_courant_law(const GridDesc& G, const PhysParamsH& ph, const double* P
     EXTERN template void plain_flux_law<LAW>(int, int, const GridDesc&, const PhysParamsH&, const double*,           \
                                              double* const*, DevStatus*, cudaStream_t);                                    \
     EXTERN template void plain_update_law<LAW>(const GridDesc&, const PhysParamsH&, const double*, double*, double*, \
-                                               double*, const double*, const double*, const double*, double, int,   \
+                                               double*, const double*, const double*, const double*, int, int,      \
                                                const double*, DevStatus*, cudaStream_t, const double*);             \
     EXTERN template void plain_courant_law<LAW>(const GridDesc&, const PhysParamsH&, const double*, DevStatus*,      \
                                                 cudaStream_t)

@@ -156,7 +156,7 @@ CRM_FN SinCos table(int k)
 CRM_FN double round_checked(double hi, double lo, double err, bool& ok)
 {
     const double r = add(hi, add(lo, err));
-    ok = ok && r == add(hi, sub(lo, err));
+    ok = ok && ieee64::bits(r) == ieee64::bits(add(hi, sub(lo, err)));
     return r;
 }
 
