@@ -412,18 +412,13 @@ F64_FN double fastest(const Consts& c, const double* P, bool& ok)
     }
 }
 
-// a b on the FP64 pipe, in a branch (the asm keeps the compiler from issuing
-// it for every thread)
-F64_FN double mul_seldom(double a, double b)
-{
-#if defined(__CUDA_ARCH__)
-    double r;
-    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
-    return r;
+// a b on the FP64 pipe, as a call: predicated in line it would take its slot
+// of the pipe also where no thread needs it
+#if defined(__CUDACC__)
+static __device__ __noinline__ double mul_seldom(double a, double b) { return __dmul_rn(a, b); }
 #else
-    return a * b;
+static inline double mul_seldom(double a, double b) { return a * b; }
 #endif
-}
 
 // a b for any operands: on the FP64 pipe only where the integer product does
 // not hold

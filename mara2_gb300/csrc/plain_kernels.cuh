@@ -127,7 +127,7 @@ struct TileSpace {
     int lo[3];      // first face (right cell) and rows of each axis
     int nf;         // faces along the axis
     int ncol;       // rows of the axis that runs across the tile
-    int len, width; // faces along and across a tile, at most TILE_FACES in all
+    int len;        // faces along a tile
     int na, nc;     // tiles along and across
 };
 
@@ -177,17 +177,23 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     const int tid = threadIdx.x;
-    const int a0 = (b % X.na) * X.len, c0 = (b / X.na) % X.nc * X.width, o = b / X.na / X.nc;
-    const int len = min(X.len, X.nf - a0), width = min(X.width, X.ncol - c0);
-    const int faces = len * width, zones = faces + width;
+    // across the tile: one row for faces along x, else four zones of x (a
+    // 32-byte sector; at the grid's edge fewer, their items skipped)
+    constexpr int WIDTH = AXIS == 0 ? 1 : 4;
+    const int a0 = (b % X.na) * X.len, c0 = (b / X.na) % X.nc * WIDTH, o = b / X.na / X.nc;
+    const int len = min(X.len, X.nf - a0), width = min(WIDTH, X.ncol - c0);
+    const int faces = len * WIDTH, zones = faces + WIDTH;
     const int i = X.lo[0] + (AXIS == 0 ? a0 : c0);
     const int j = X.lo[1] + (AXIS == 1 ? a0 : AXIS == 0 ? c0 : o);
     const int k = X.lo[2] + (AXIS == 2 ? a0 : o);
     const long long s0 = 1, s1 = G.N[0], s2 = (long long) G.N[0] * G.N[1];
     const long long stride = AXIS == 0 ? s0 : AXIS == 1 ? s1 : s2, cstride = AXIS == 0 ? s1 : s0;
     const double* p = P + ((long long) k * G.N[1] + j) * G.N[0] + i;   // cell on the right of the tile's first face
-    for (int it = tid; it < NQ * zones; it += TILE_THREADS) {
-        const int q = it / zones, z = it - q * zones, s = z / width, w = z - s * width;
+    for (int q = 0, z = tid; q < NQ; z += TILE_THREADS) {
+        for (; z >= zones && q < NQ; z -= zones) ++q;
+        const int s = z / WIDTH, w = z % WIDTH;
+        if (q >= NQ) break;
+        if (w >= width) continue;
         bool ok = true;
         double l, r;
         zone_edges<RECON>(C, p + q * G.sP + (s - 1) * stride + w * cstride, stride, q, l, r, ok);
@@ -196,8 +202,8 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
         if (!ok) sm.odd_zone[z] = 1;
     }
     __syncthreads();
-    if (tid < 2 * faces) {
-        const int s = tid >= faces ? 1 : 0, f = tid - s * faces, z = f + s * width;
+    if (tid < 2 * faces && tid % WIDTH < width) {
+        const int s = tid >= faces ? 1 : 0, f = tid - s * faces, z = f + s * WIDTH;
         double Ps[NQ];
 #pragma unroll
         for (int q = 0; q < NQ; ++q) Ps[q] = sm.edge[1 - s][q][z];
@@ -218,8 +224,11 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
     const long long fstride = AXIS == 0 ? f0 : AXIS == 1 ? f1 : f2, fcstride = AXIS == 0 ? f1 : f0;
     double* out = F + ((long long) k * (G.N[1] + 1) + j) * (G.N[0] + 1) + i;
     if constexpr (RIEMANN == RIEMANN_HLLE) {
-        for (int it = tid; it < NQ * faces; it += TILE_THREADS) {
-            const int q = it / faces, f = it - q * faces, s = f / width, w = f - s * width;
+        for (int q = 0, f = tid; q < NQ; f += TILE_THREADS) {
+            for (; f >= faces && q < NQ; f -= faces) ++q;
+            const int s = f / WIDTH, w = f % WIDTH;
+            if (q >= NQ) break;
+            if (w >= width) continue;
             bool ok = !sm.odd_face[f];
             const double h = fast64::hlle(sm.A[0][0][f], sm.A[1][0][f], sm.A[0][1][f], sm.A[1][1][f], sm.F[0][q][f],
                                           sm.F[1][q][f], sm.U[0][q][f], sm.U[1][q][f], ok);
@@ -227,15 +236,15 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
             if (ok) to[q * G.sF] = h;
             else sm.odd_face[f] = 1;   // every field of the face by the general functions, below
         }
-    } else if (tid < faces) {
+    } else if (tid < faces && tid % WIDTH < width) {
         // HLLC's star state couples the fields: a thread per face
-        const int f = tid, s = f / width, w = f - s * width;
+        const int f = tid, s = f / WIDTH, w = f % WIDTH;
         double Pl[NQ], Pr[NQ], h[NQ];
         fast64::Side<NQ> L, R;
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
             Pl[q] = sm.edge[1][q][f];
-            Pr[q] = sm.edge[0][q][f + width];
+            Pr[q] = sm.edge[0][q][f + WIDTH];
             L.U[q] = sm.U[0][q][f];
             R.U[q] = sm.U[1][q][f];
             L.F[q] = sm.F[0][q][f];
@@ -259,7 +268,7 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
     }
     __syncthreads();
     if (tid < faces && sm.odd_face[tid]) {
-        const int s = tid / width, w = tid - s * width;
+        const int s = tid / WIDTH, w = tid % WIDTH;
         const int e = face_general<LAW, RECON, RIEMANN>(p + s * stride + w * cstride, G.sP, stride,
                                                              G.nrm[AXIS][0], G.nrm[AXIS][1], G.nrm[AXIS][2], &pp,
                                                              out + s * fstride + w * fcstride, G.sF);
@@ -766,16 +775,14 @@ static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::C
             TileSpace& T = X.axis[axis];
             int nb[3];
             face_rows(G, axis, T.lo, nb);
-            // across the tile: rows of y for faces along x, four zones of x (a
-            // 32-byte sector) otherwise; along it, tiles of equal length
+            const int width = axis == 0 ? 1 : 4;
             const int cross = axis == 0 ? 1 : 0, outer = axis == 2 ? 1 : 2;
-            const int most = axis == 0 ? TILE_FACES : TILE_FACES / 4;
+            const int most = TILE_FACES / width;
             T.nf = nb[axis];
             T.ncol = nb[cross];
-            T.width = axis == 0 ? 1 : 4;
             T.na = (T.nf + most - 1) / most;
-            T.len = (T.nf + T.na - 1) / T.na;
-            T.nc = (T.ncol + T.width - 1) / T.width;
+            T.len = (T.nf + T.na - 1) / T.na;   // tiles of equal length
+            T.nc = (T.ncol + width - 1) / width;
             X.first[axis + 1] += T.na * T.nc * nb[outer];
         }
         flux_tile_kernel<LAW, RECON, RIEMANN><<<X.first[3], TILE_THREADS, 0, s>>>(P, X, G, pp, C, st);
