@@ -31,6 +31,7 @@ __global__ void k_courant_init(DevStatus* st)
 // (src/Problems.cpp:181-186); a step at t >= t_final is not taken.
 __global__ void k_dt_from_courant(DevStatus* st, double cfl, double t_final)
 {
+    pdl_chain();
     if (st->done) return;
     const double courant = __longlong_as_double((long long) st->dt_bits);
     double dt = cfl * courant;
@@ -46,6 +47,7 @@ __global__ void k_dt_from_courant(DevStatus* st, double cfl, double t_final)
 // after a driver loop stopped at t_final
 __global__ void k_set_dt(DevStatus* st, double dt)
 {
+    pdl_chain();
     st->dt = dt;
     st->done = 0;
 }
@@ -53,11 +55,16 @@ __global__ void k_set_dt(DevStatus* st, double dt)
 // an advance that ran counts toward the state's ping-pong parity
 __global__ void k_step_taken(DevStatus* st)
 {
+    pdl_chain();
     if (!st->done && !st->code && !st->halt) st->taken += 1;
 }
 
+// the end of a driver-loop step: the clock, and the Courant slot reset for the
+// next step's reduction
 __global__ void k_advance_time(DevStatus* st)
 {
+    pdl_chain();
+    st->dt_bits = (unsigned long long) __double_as_longlong(DBL_MAX);
     if (st->done || st->code) return;
     st->t += st->dt;
     st->steps += 1;
@@ -268,10 +275,10 @@ __global__ void k_assign_b(double* __restrict__ aos, GridDesc G, VecPot V, doubl
 void launch_courant_init(DevStatus* st, cudaStream_t s) { k_courant_init<<<1, 1, 0, s>>>(st); }
 void launch_dt_from_courant(DevStatus* st, double cfl, double t_final, cudaStream_t s)
 {
-    k_dt_from_courant<<<1, 1, 0, s>>>(st, cfl, t_final);
+    chain_launch(k_dt_from_courant, dim3(1), dim3(1), s, st, cfl, t_final);
 }
-void launch_set_dt(DevStatus* st, double dt, cudaStream_t s) { k_set_dt<<<1, 1, 0, s>>>(st, dt); }
-void launch_advance_time(DevStatus* st, cudaStream_t s) { k_advance_time<<<1, 1, 0, s>>>(st); }
+void launch_set_dt(DevStatus* st, double dt, cudaStream_t s) { chain_launch(k_set_dt, dim3(1), dim3(1), s, st, dt); }
+void launch_advance_time(DevStatus* st, cudaStream_t s) { chain_launch(k_advance_time, dim3(1), dim3(1), s, st); }
 void launch_aos_to_soa_range(const double* aos, double* soa, const GridDesc& G, long long c0, long long c1,
                              cudaStream_t s)
 {
@@ -508,15 +515,26 @@ static void enqueue_step(MaraGpuHandle* h)
     }
 }
 
+// the plain path's Courant reduction into dt_bits, which has been reset
+static void enqueue_plain_courant(MaraGpuHandle* h)
+{
+    TimedPair tp;
+    timed_begin(h, 2, tp);
+    plain_courant(kernel_law(&h->cfg), h->G, h->pp, h->P[h->cur], h->st, h->stream);
+    timed_end(h, tp);
+    h->launches++;
+}
+
 static void enqueue_courant(MaraGpuHandle* h)
 {
     launch_courant_init(h->st, h->stream);
+    h->launches++;
+    if (!h->mixed) return enqueue_plain_courant(h);
     TimedPair tp;
     timed_begin(h, 2, tp);
-    if (h->mixed) mixed_enqueue_courant(h->mixed, h->st, h->stream);
-    else plain_courant(kernel_law(&h->cfg), h->G, h->pp, h->P[h->cur], h->st, h->stream);
+    mixed_enqueue_courant(h->mixed, h->st, h->stream);
     timed_end(h, tp);
-    h->launches += 2;
+    h->launches++;
 }
 
 // With the stream idle: the state's buffer parity from the steps that ran
@@ -840,7 +858,7 @@ int mara_gpu_advance(MaraGpuHandle* h, double t0, double dt)
         h->launches++;
         enqueue_step(h);
         if (const int se = take_source_error(h)) return se;
-        k_step_taken<<<1, 1, 0, h->stream>>>(h->st);
+        chain_launch(k_step_taken, dim3(1), dim3(1), h->stream, h->st);
         h->launches++;
     }
     h->steps++;
@@ -893,7 +911,7 @@ static void enqueue_run_step(MaraGpuHandle* h, double cfl, double t_final)
         h->launches += mixed_launches_per_step(h->mixed);
         return;
     }
-    enqueue_courant(h);
+    enqueue_plain_courant(h);
     launch_dt_from_courant(h->st, cfl, t_final, h->stream);
     enqueue_step(h);
     launch_advance_time(h->st, h->stream);
@@ -926,7 +944,7 @@ static int build_run_graph(MaraGpuHandle* h, int which, double cfl, double t_fin
 static int launches_per_run_step(MaraGpuHandle* h)
 {
     if (h->mixed) return mixed_launches_per_step(h->mixed);
-    int n = 2 /* courant init + courant */ + 2 /* dt, time */;
+    const int n = 1 /* courant */ + 2 /* dt, time */;
     return n + h->cfg.rk_order * (plain_flux_launches(kernel_law(&h->cfg), h->cfg.recon, h->cfg.riemann, h->G) + 1);
 }
 
@@ -961,6 +979,10 @@ static int enqueue_run(MaraGpuHandle* h, int max_steps, double cfl, double t_fin
             h->launches++;
         }
         return cuda_status(cudaGetLastError());
+    }
+    if (!h->mixed && max_steps > 0) {
+        launch_courant_init(h->st, h->stream);   // the steps' ends reset it from here on
+        h->launches++;
     }
     const bool use_graph = !h->timing;
     if (use_graph && (h->graph_cfl != cfl || h->graph_tfinal != t_final)) {

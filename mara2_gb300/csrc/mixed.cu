@@ -47,15 +47,6 @@ template <int RECON> struct SOf { static constexpr int S = RECON == RECON_PCM ? 
 // The face fluxes along one axis of the general form.  AXIS >= 0 is the
 // axis at compile time (no multiplications by the zero components of the
 // normal); AXIS < 0 takes it, and the normal, at run time.
-// The general form's kernels run as a chain of programmatic dependent
-// launches: each waits for the kernel before it (whose writes are then
-// visible) and then lets the next one launch, so a launch's start overlaps
-// its predecessor's last wave.  Outside such a chain both are no-ops.
-__device__ __forceinline__ void pdl_chain()
-{
-    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // the faces of one axis: first face and rows, faces of a z-slice, z-slices
 struct FaceSpaceF {
     int axis, lo0, lo1, lo2, nb0, nb1, nb2;
@@ -1221,22 +1212,6 @@ void mixed_volume_diagnostics(MixedState* m, double* partial, int* err, double* 
 }
 
 // ---- general form ------------------------------------------------------------
-// a launch in the general form's chain of programmatic dependents (pdl_chain)
-template <typename... KArgs, typename... Args>
-static void chain_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args)
-{
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = grid;
-    lc.blockDim = block;
-    lc.stream = s;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    cudaLaunchKernelEx(&lc, kernel, std::forward<Args>(args)...);
-}
-
 template <int LAW, int RECON, int RIEMANN>
 static void flux_f_launch(MixedState* m, const int* done, DevStatus* st, cudaStream_t s)
 {

@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(128) flux_general_kernel(const double* __restr
                                                            const __grid_constant__ FaceSpace X,
                                                            DevStatus* __restrict__ st)
 {
+    pdl_wait();
     if (st->code != 0 || st->done) return;
     if (st->failures != 0) { st->halt = 1; return; }  // failures are final once the stage ended
     const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
@@ -290,6 +291,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS)
                      const __grid_constant__ GridDesc G, const __grid_constant__ PhysParams pp,
                      const __grid_constant__ fast64::Consts C, DevStatus* __restrict__ st)
 {
+    pdl_wait();
     __shared__ TileShared<LawInfo<LAW>::NQ> sm;
     const int tid = threadIdx.x;
     for (int z = tid; z < TILE_ZONES; z += TILE_THREADS) sm.odd_zone[z] = 0;
@@ -327,6 +329,7 @@ __global__ void __launch_bounds__(128, 3) flux_run_kernel(const double* __restri
                                                           DevStatus* __restrict__ st)
 {
     constexpr int NQ = LawInfo<LAW_HYDRO>::NQ;
+    pdl_wait();
     if (st->code != 0 || st->done) return;
     if (st->failures != 0) { st->halt = 1; return; }  // failures are final once the stage ended
     const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
@@ -512,6 +515,7 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
                                                      DevStatus* __restrict__ st, const double* __restrict__ S)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
+    pdl_wait();
     if (st->code != 0 || st->halt || st->done) return;
     const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
     if (lin >= (unsigned) G.n[0] * (unsigned) G.n[1]) return;
@@ -624,6 +628,7 @@ __global__ void __launch_bounds__(128) courant_kernel(const double* __restrict__
                                                       DevStatus* __restrict__ st)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
+    pdl_wait();
     // the relativistic law's three normals cost a quartic each: a thread each
     constexpr int AXES = LAW == LAW_RMHD ? 3 : 1;
     const unsigned slice = (unsigned) G.n[0] * (unsigned) G.n[1];
@@ -737,9 +742,9 @@ static void flux_runs(const GridDesc& G, const PhysParams& pp, const fast64::Con
         const long long slice = (long long) X.nb[0] * X.nb[1];
         const dim3 grid((unsigned) ((slice + 127) / 128), X.nb[2]);
         switch (axis) {
-            case 0: flux_run_kernel<0><<<grid, 128, 0, s>>>(P, F[0], G, pp, C, X, st); break;
-            case 1: flux_run_kernel<1><<<grid, 128, 0, s>>>(P, F[1], G, pp, C, X, st); break;
-            default: flux_run_kernel<2><<<grid, 128, 0, s>>>(P, F[2], G, pp, C, X, st); break;
+            case 0: chain_launch(flux_run_kernel<0>, grid, dim3(128), s, P, F[0], G, pp, C, X, st); break;
+            case 1: chain_launch(flux_run_kernel<1>, grid, dim3(128), s, P, F[1], G, pp, C, X, st); break;
+            default: chain_launch(flux_run_kernel<2>, grid, dim3(128), s, P, F[2], G, pp, C, X, st); break;
         }
     }
 }
@@ -757,7 +762,7 @@ static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::C
             const long long slice = (long long) X.nb[0] * X.nb[1];
             const int block = block_size(slice * X.nb[2]);
             const dim3 grid((unsigned) ((slice + block - 1) / block), X.nb[2]);
-            flux_general_kernel<LAW, RECON, RIEMANN><<<grid, block, 0, s>>>(P, F[axis], G, pp, X, st);
+            chain_launch(flux_general_kernel<LAW, RECON, RIEMANN>, grid, dim3(block), s, P, F[axis], G, pp, X, st);
         }
     } else {
         if constexpr (LAW == LAW_HYDRO && RIEMANN == RIEMANN_HLLC && RECON == RECON_PLM) {
@@ -785,7 +790,7 @@ static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::C
             T.nc = (T.ncol + width - 1) / width;
             X.first[axis + 1] += T.na * T.nc * nb[outer];
         }
-        flux_tile_kernel<LAW, RECON, RIEMANN><<<X.first[3], TILE_THREADS, 0, s>>>(P, X, G, pp, C, st);
+        chain_launch(flux_tile_kernel<LAW, RECON, RIEMANN>, dim3(X.first[3]), dim3(TILE_THREADS), s, P, X, G, pp, C, st);
     }
 }
 
@@ -825,8 +830,8 @@ void plain_update_law(const GridDesc& G, const PhysParamsH& ph, const double* Pi
     const long long slice = (long long) G.n[0] * G.n[1];
     const int block = block_size(slice * G.n[2]);
     const dim3 grid((unsigned) ((slice + block - 1) / block), G.n[2]);
-    update_kernel<LAW><<<grid, block, 0, s>>>(Pin, Pout, U0, U, V, G, to_dev(ph), to_fast(ph, G), factor / G.dV, w,
-                                              stage, dt, st, S);
+    chain_launch(update_kernel<LAW>, grid, dim3(block), s, Pin, Pout, U0, U, V, G, to_dev(ph), to_fast(ph, G),
+                 factor / G.dV, w, stage, dt, st, S);
 }
 
 template <int LAW>
@@ -835,7 +840,7 @@ void plain_courant_law(const GridDesc& G, const PhysParamsH& ph, const double* P
     const long long slice = (long long) G.n[0] * G.n[1] * (LAW == LAW_RMHD ? 3 : 1);
     const int block = block_size(slice * G.n[2]);
     const dim3 grid((unsigned) ((slice + block - 1) / block), G.n[2]);
-    courant_kernel<LAW><<<grid, block, 0, s>>>(P, G, to_dev(ph), to_fast(ph, G), st);
+    chain_launch(courant_kernel<LAW>, grid, dim3(block), s, P, G, to_dev(ph), to_fast(ph, G), st);
 }
 
 // one translation unit per law instantiates the kernels (plain_*.cu)
