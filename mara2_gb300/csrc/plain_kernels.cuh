@@ -551,12 +551,14 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
         // the sum over the faces in the reference's order; a flat axis adds
-        // and subtracts a zero, which only makes a -0 a +0
+        // and subtracts a zero, which only makes a -0 a +0.  (These products
+        // in integers too: the two pipes out of balance, KH 1024^2, four
+        // steps, 4.84 -> 5.09 ms.)
         double sum = 0.0;
-        if (fx) sum = fast64::mul_any(face_flux<NQ>(V, G, 0, q, i + 1, j, k), G.dA[0]) - fast64::mul_any(face_flux<NQ>(V, G, 0, q, i, j, k), G.dA[0]);
-        if (fy) sum = sum + fast64::mul_any(face_flux<NQ>(V, G, 1, q, i, j + 1, k), G.dA[1]) - fast64::mul_any(face_flux<NQ>(V, G, 1, q, i, j, k), G.dA[1]);
+        if (fx) sum = face_flux<NQ>(V, G, 0, q, i + 1, j, k) * G.dA[0] - face_flux<NQ>(V, G, 0, q, i, j, k) * G.dA[0];
+        if (fy) sum = sum + face_flux<NQ>(V, G, 1, q, i, j + 1, k) * G.dA[1] - face_flux<NQ>(V, G, 1, q, i, j, k) * G.dA[1];
         else sum = fast64::add_zero(sum, false);
-        if (fz) sum = sum + fast64::mul_any(face_flux<NQ>(V, G, 2, q, i, j, k + 1), G.dA[2]) - fast64::mul_any(face_flux<NQ>(V, G, 2, q, i, j, k), G.dA[2]);
+        if (fz) sum = sum + face_flux<NQ>(V, G, 2, q, i, j, k + 1) * G.dA[2] - face_flux<NQ>(V, G, 2, q, i, j, k) * G.dA[2];
         else sum = fast64::add_zero(sum, false);
         double L = fast64::mul_any(fv, sum);
         if constexpr (LAW == LAW_MHD_COOL) {
