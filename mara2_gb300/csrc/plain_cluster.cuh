@@ -3,7 +3,7 @@
 //
 // A step of a small 1-D grid is a chain of dependent latencies: eight
 // launches, each with a warp or less per scheduler (1024 zones, PLM, HLLE,
-// RK2: 43 us a step).  Here the grid stays in the shared memory of a cluster
+// RK2: 43 us a step, 17 us here).  Here the grid stays in the shared memory of a cluster
 // of up to 16 CTAs, each holding m zones.  Per RK stage the cluster
 // synchronises once, each CTA reads its halo from its neighbours' shared
 // memory (distributed shared memory) or from the boundary images, and its
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
                 const int q = it / (mine + 2), z = it - q * (mine + 2);
                 bool ok = true;
                 double l, h;
-                zone_edges<RECON>(C, Ps + q * W + S + z - 1, 1, q, l, h, ok);
+                zone_edges<LAW_HYDRO, RECON>(C, Ps + q * W + S + z - 1, 1, q, l, h, ok);
                 E[q * (m + 2) + z] = l;
                 E[(NQ + q) * (m + 2) + z] = h;
                 if (!ok) odd_zone[z] = 1;

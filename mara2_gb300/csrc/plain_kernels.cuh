@@ -1,16 +1,22 @@
-// plain_kernels.cuh -- the kernels of the plain FP64 path: one face-flux sweep kernel per
-// fleshed axis, then one fused update kernel per RK stage, plus the Courant
-// reduction.  Compiled with --fmad=false (see mara2_gb300/build.py) so that
-// the arithmetic rounds as the reference's CPU build does.
+// plain_kernels.cuh -- the kernels of the plain FP64 path: one launch of face
+// fluxes over all fleshed axes (runs of faces: one per axis), then one fused
+// update kernel per RK stage, plus the Courant reduction.  Compiled with
+// --fmad=false (see mara2_gb300/build.py) so that the arithmetic rounds as
+// the reference's CPU build does.
 //
 // Per stage (MethodOfLinesTVD::advance, SolutionSchemes.cpp:191-274):
-//   flux_kernel<axis>   MeshOperator::godunov (MeshOperator.cpp:443-525):
-//                       gather the 2s-cell stencil along the axis, intercell
-//                       flux (reconstruction + fromPrimitive x2 + Riemann),
-//                       raw flux stored per face.  Faces are those the
-//                       interior update reads: along the axis the interior
-//                       faces, across it the interior rows plus one guard row
-//                       on each side when flux CT needs transverse neighbours.
+//   flux kernels        MeshOperator::godunov (MeshOperator.cpp:443-525): the
+//                       2s-cell stencil along the axis, intercell flux
+//                       (reconstruction + fromPrimitive x2 + Riemann), raw
+//                       flux stored per face.  Faces are those the interior
+//                       update reads: along the axis the interior faces,
+//                       across it the interior rows plus one guard row on
+//                       each side when flux CT needs transverse neighbours.
+//                       flux_tile_kernel: a block per 32 faces; flux_run_kernel:
+//                       a thread per run of faces (large hydro grids, PLM,
+//                       HLLC); flux_general_kernel: a thread per face (magnetic
+//                       laws with HLLC).  Zones whose values the lean forms of
+//                       fast64.cuh do not cover go to face_general.
 //   update_kernel       per interior zone: CellCenteredFieldCT's flux CT on
 //                       the magnetic fluxes of the zone's six faces
 //                       (CellCenteredFieldCT.cpp:14-134), the divergence
@@ -134,23 +140,38 @@ struct TileSpace {
 
 constexpr int TILE_THREADS = 64, TILE_FACES = TILE_THREADS / 2, TILE_ZONES = TILE_FACES + 4;
 
-template <int RECON>
+static __device__ __noinline__ void weno5_edges_small(const fast64::Consts& C, const double* p, long long s, double& left,
+                                                      double& right, bool* ok)
+{
+    const double w[5] = {p[-2 * s], p[-s], p[0], p[s], p[2 * s]};
+    fast64::weno5_edges<true>(C, &w[2], left, right, *ok);
+}
+
+template <int LAW, int RECON>
 __device__ __forceinline__ void zone_edges(const fast64::Consts& C, const double* p, long long s, int q, double& left,
                                            double& right, bool& ok)
 {
     if constexpr (RECON == RECON_PCM) {
         left = right = p[0];
-        ok = ok && fast64::ordinary_field(q, p[0]);
+        ok = ok && fast64::ordinary_field<LAW>(q, p[0]);
     } else if constexpr (RECON == RECON_PLM) {
         const double l = p[-s], c = p[0], r = p[s];
         const double h = fast64::half_slope(fast64::mul(C.theta, c - l), r - l, fast64::mul(C.theta, r - c));
         left = c - h;
         right = c + h;
-        ok = ok && fast64::ordinary_field(q, l) && fast64::ordinary_field(q, c) && fast64::ordinary_field(q, r);
+        ok = ok && fast64::ordinary_field<LAW>(q, l) && fast64::ordinary_field<LAW>(q, c) && fast64::ordinary_field<LAW>(q, r);
     } else {
         const double w[5] = {p[-2 * s], p[-s], p[0], p[s], p[2 * s]};
 #pragma unroll
         for (int m = 0; m < 5; ++m) ok = ok && fast64::ordinary_field(q, w[m]);
+        if constexpr (LAW == LAW_RMHD) {
+            if (!ok) {
+                ok = true;
+                for (int m = 0; m < 5; ++m) ok = ok && fast64::ordinary_field<LAW>(q, w[m]);
+                if (ok) weno5_edges_small(C, p, s, left, right, &ok);
+                return;
+            }
+        }
         fast64::weno5_edges(C, &w[2], left, right, ok);
     }
 }
@@ -197,7 +218,7 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
         if (w >= width) continue;
         bool ok = true;
         double l, r;
-        zone_edges<RECON>(C, p + q * G.sP + (s - 1) * stride + w * cstride, stride, q, l, r, ok);
+        zone_edges<LAW, RECON>(C, p + q * G.sP + (s - 1) * stride + w * cstride, stride, q, l, r, ok);
         sm.edge[0][q][z] = l;
         sm.edge[1][q][z] = r;
         if (!ok) sm.odd_zone[z] = 1;
@@ -533,7 +554,7 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
     if (stage == 0) {
         bool ok = C.ok;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
+        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field<LAW>(q, Pc[q]);
         if constexpr (LAW == LAW_RMHD) fast64::rmhd_p2u(C, Pc, Uo, ok);
         else fast64::p2u<LAW>(C, Pc, Uo, ok);
         if (!ok) {
@@ -569,7 +590,7 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
         if (S) L += S[q * G.sP + pc];  // the source terms function's array (SolutionSchemes.cpp:219-228)
         Un[q] = rk_combine_plain(Uo[q], Up[q], L, dt, w);
         U[q * G.sU + uc] = Un[q];
-        fine = fine && fast64::ordinary_field(q, Un[q]);
+        fine = fine && fast64::ordinary_field<LAW>(q, Un[q]);
     }
 
     double Pn[NQ];
@@ -647,7 +668,7 @@ __global__ void __launch_bounds__(128) courant_kernel(const double* __restrict__
         double lmax = 0.0;
         bool ok = C.ok;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, Pc[q]);
+        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field<LAW>(q, Pc[q]);
         if constexpr (LAW == LAW_RMHD) lmax = fast64::rmhd_fastest(C, Pc, axis, ok);
         else lmax = fast64::fastest<LAW>(C, Pc, ok);
         if (!ok) {

@@ -66,8 +66,8 @@ static double any()
 
 #ifndef PROBE_IEEE_ONLY
 // A zone's primitives.  kind 0: smooth, 1: zeros and equal values, 2: strong
-// jumps, 3: wide magnitudes, 4: anything; hydro pressure and density positive
-// for kinds 0 to 3
+// jumps, 3: wide magnitudes, 4: anything, 5: small fields and zeros; hydro
+// pressure and density positive for all but kind 4
 static void zone(int law, int kind, int nq, const double* base, double* P)
 {
     for (int q = 0; q < nq; ++q) {
@@ -76,11 +76,19 @@ static void zone(int law, int kind, int nq, const double* base, double* P)
         if (kind == 0) v = base[q] * (1 + 0.1 * (uni() - 0.5));
         else if (kind == 1) v = pos ? (rnd() & 1 ? 1.0 : base[q]) : rnd() % 4 == 0 ? base[q] : rnd() % 3 == 0 ? -0.0 : 0.0;
         else if (kind == 2) v = pos ? exp(8 * (uni() - 0.5)) : 6 * (uni() - 0.5);
+        else if (kind == 5) v = pos || rnd() % 8 ? base[q] * (1 + 0.1 * (uni() - 0.5)) : 0.0;
         else if (kind == 3) v = pos ? fabs(wide(30)) : wide(rnd() % 8 ? 20 : 320);
         else v = any();
         if (law == LAW_RMHD && kind < 4 && !pos && q < 4) v *= kind == 2 ? 0.16 : 0.5;   // mostly below light speed
         P[q] = v;
     }
+}
+
+// some fields down to 2^-930
+static void shrink(int nq, double* base)
+{
+    for (int q = 0; q < nq; ++q)
+        if (q != 0 && q != 4 && rnd() % 2) base[q] *= pow(2.0, -930 * uni());
 }
 
 template <int LAW, int RECON, int RIEMANN, int AXIS>
@@ -91,15 +99,18 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
     for (long m = 0; m < n; ++m) {
         double Z[2 * S][NQ], base[NQ];
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
+        if (kind == 5) shrink(NQ, base);
         for (int s = 0; s < 2 * S; ++s) zone(LAW, kind, NQ, base, Z[s]);
         if (kind == 1 && rnd() % 3 == 0) for (int s = 1; s < 2 * S; ++s) memcpy(Z[s], Z[0], sizeof(Z[0]));
         double PL[NQ], PR[NQ], QL[NQ], QR[NQ];
         bool ok = C.ok;
         for (int q = 0; q < NQ; ++q) {
             double v[2 * S];
+            bool strict = true;
             for (int s = 0; s < 2 * S; ++s) {
                 v[s] = Z[s][q];
-                ok = ok && fast64::ordinary_field(q, v[s]);
+                ok = ok && fast64::ordinary_field<LAW>(q, v[s]);
+                strict = strict && fast64::ordinary_field(q, v[s]);
             }
             if constexpr (RECON == RECON_PCM) { PL[q] = QL[q] = v[0]; PR[q] = QR[q] = v[1]; }
             else if constexpr (RECON == RECON_PLM) {
@@ -112,8 +123,13 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
                 QL[q] = weno5<true>(&v[2], pp.weno_is, pp.shenzha_A);
                 QR[q] = weno5<false>(&v[3], pp.weno_is, pp.shenzha_A);
                 double x;
-                fast64::weno5_edges(C, &v[2], x, PL[q], ok);
-                fast64::weno5_edges(C, &v[3], PR[q], x, ok);
+                if (strict) {
+                    fast64::weno5_edges(C, &v[2], x, PL[q], ok);
+                    fast64::weno5_edges(C, &v[3], PR[q], x, ok);
+                } else {
+                    fast64::weno5_edges<true>(C, &v[2], x, PL[q], ok);
+                    fast64::weno5_edges<true>(C, &v[3], PR[q], x, ok);
+                }
             }
         }
         double F[NQ], H[NQ];
@@ -189,9 +205,10 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
     for (long m = 0; m < n; ++m) {
         double base[NQ], P[NQ];
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
+        if (kind == 5) shrink(NQ, base);
         zone(LAW, kind, NQ, base, P);
         bool ord = C.ok;
-        for (int q = 0; q < NQ; ++q) ord = ord && fast64::ordinary_field(q, P[q]);
+        for (int q = 0; q < NQ; ++q) ord = ord && fast64::ordinary_field<LAW>(q, P[q]);
         double U[NQ], W[NQ];
         bool ok = ord;
         bool wrong = false;
@@ -208,7 +225,7 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
         for (int t = 0; t < 2; ++t) {
             double D[NQ], A[NQ], B[NQ];
             bool o2 = C.ok;
-            for (int q = 0; q < NQ; ++q) { D[q] = t ? U[q] : P[q]; o2 = o2 && fast64::ordinary_field(q, D[q]); A[q] = 0; }
+            for (int q = 0; q < NQ; ++q) { D[q] = t ? U[q] : P[q]; o2 = o2 && fast64::ordinary_field<LAW>(q, D[q]); A[q] = 0; }
             int code = 0;
             const int e = law_cons<LAW>(pp, D, A, &code);
             if constexpr (LAW == LAW_RMHD) fast64::rmhd_cons(C, D, B, o2);

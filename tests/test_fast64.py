@@ -17,7 +17,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 HYDRO, MHD, RMHD, MHD_COOL = 0, 1, 2, 3
-SMOOTH, ZEROS, JUMPS, WIDE, ANY = range(5)
+SMOOTH, ZEROS, JUMPS, WIDE, ANY, SMALL = range(6)
 
 
 def _build(path, ulps, *flags):
@@ -56,19 +56,21 @@ def test_face_flux_has_the_general_forms_bits(lib, law, recon, riemann):
     acc = C.c_long()
     for axis, gamma, theta in ((0, 5.0 / 3, 1.5), (1, 1.4, 1.0), (2, 4.0 / 3, 2.0)):
         for weno in (range(3) if recon == 2 else (2,)):
-            for kind in range(5):
+            for kind in range(6):
                 bad = lib.probe_faces(C.c_long(n), C.c_ulonglong(100 * kind + axis), law, recon, riemann, axis, weno,
                                       C.c_double(gamma), C.c_double(theta), kind, C.byref(acc))
                 assert bad == 0, (axis, weno, kind)
                 if kind in (SMOOTH, ZEROS):
                     assert acc.value == n
+                if kind == SMALL and law == RMHD:
+                    assert acc.value > n / 2
 
 
 @pytest.mark.parametrize("law", [HYDRO, MHD, RMHD, MHD_COOL])
 def test_zone_conversions_and_wave_speeds_have_the_general_forms_bits(lib, law):
     n = 20000
     acc = C.c_long()
-    for kind in range(5):
+    for kind in range(6):
         assert lib.probe_zones(C.c_long(n), C.c_ulonglong(kind), law, C.c_double(5.0 / 3), kind, C.byref(acc)) == 0
         if kind in (SMOOTH, ZEROS, JUMPS):
             assert acc.value == n
