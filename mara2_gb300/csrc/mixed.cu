@@ -5,8 +5,8 @@
 //
 //  * fused tiles (hydro_tile.cuh) for Newtonian hydro on 1-D / 2-D grids:
 //    one kernel per RK stage, primitives and fluxes in shared memory only;
-//  * the general form for every law / reconstruction / dimension: one FP32
-//    face-flux kernel per axis (FP32 fluxes in HBM), then an update kernel
+//  * the general form for every law / reconstruction / dimension: one launch
+//    of FP32 face fluxes over all axes (FP32 fluxes in HBM), then an update kernel
 //    doing FP32 flux CT, divergence, the FP32-pair RK combine and the
 //    primitive recovery (FP32 for hydro and MHD, FP64 Newton for RMHD), and
 //    writing FP32 primitives with their guard images for the next sweep.
@@ -1896,7 +1896,6 @@ int mixed_launches_per_step(const MixedState* m)
 
 void mixed_enqueue_courant(MixedState* m, DevStatus* st, cudaStream_t s) { k_cfl_publish<<<1, 1, 0, s>>>(m->dcfl, st); }
 int mixed_parity(const MixedState* m) { return m->rot & 1; }
-bool mixed_fused(const MixedState* m) { return m->fused; }
 
 // ---- small 1-D grids: many steps per launch on one thread-block cluster -------
 bool mixed_cluster_capable(const MixedState* m)

@@ -36,7 +36,6 @@ bool mixed_host_step_capable(const MixedState* m);
 int mixed_advance_host_step(MixedState* m, double* host_dev, double dt, DevStatus* st, cudaStream_t s,
                             int64_t* launches);
 int mixed_launches_per_step(const MixedState* m);
-bool mixed_fused(const MixedState* m);
 // 1-D hydro grids of up to 8192 zones on the fused form: up to nsteps
 // driver-loop steps in one launch on a thread-block cluster holding the grid
 // in shared memory (hydro_cluster.cuh)
