@@ -57,8 +57,8 @@ F64_FN bool ordinary_field(int q, double x) { return q == 0 || q == 4 ? ordinary
 // the general forms do, so they take fields down to 2^-900: in a medium at
 // rest ahead of a wave, WENO leaves transverse fields of 1e-200 to 1e-99
 // behind for good (blast 512^2 after 43 steps: in a third of the zones).
-// Their faces and zones went to the general functions: 45 steps about 590 ms, with
-// the lean ones 322.
+// Their faces and zones went to the general functions: 45 steps 631 ms; with
+// the lean ones, and rmhd_roots_certain's second point, 321.
 // Only the product with y's normal is formed without a check; its factors are
 // steep() or zero.
 F64_FN bool steep(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) >= (68u << 20) || is_zero(x); }   // 2^-955
