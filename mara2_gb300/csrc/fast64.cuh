@@ -47,8 +47,11 @@ F64_FN u32 expo(double x) { return (u32) (bits(x) >> 52) & 0x7ffu; }
 
 // Ordinary operands: a density or pressure of 2^-100 to 2^101, another field
 // zero or of magnitude 2^-330 to 2^101.  An edge value then is at least
-// 2^-153 and 2^-383 (or zero), and the products that the functions below form
-// without a check stay normal: the smallest is rho v v above 2^-920.
+// 2^-154 (edge_pos) and 2^-383 (or zero), and the products that the functions
+// below form without a check stay normal: the smallest is rho v v above 2^-974,
+// its v_n along y a difference of two such values.  PLM gives no smaller
+// edges (the last place of 2^-331); WENO's weighted sum cancels a second time,
+// down to 2^-436 found, so weno5_edges checks (edge()).
 F64_FN bool ordinary_pos(double x) { return (u32) (bits(x) >> 32) - (923u << 20) <= (200u << 20); }
 F64_FN bool ordinary(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (693u << 20) <= (430u << 20) || is_zero(x); }
 // field q of a primitive (or conserved: density and energy) state
@@ -68,6 +71,8 @@ F64_FN bool ordinary_field(int q, double x)
     if (LAW != LAW_RMHD || q == 0 || q == 4) return ordinary_field(q, x);
     return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (123u << 20) <= (1000u << 20) || is_zero(x);
 }
+// a reconstructed value of ordinary ones
+F64_FN bool edge(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) >= (640u << 20) || is_zero(x); }
 // a reconstructed density or pressure
 F64_FN bool edge_pos(double x) { return (u32) (bits(x) >> 32) - (869u << 20) <= (256u << 20); }
 
@@ -209,7 +214,7 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
     const double l0 = e0 - gp + tp2, l1 = tm + c0 - sp, l2 = -sm2 + cm + t0;
     right = div(mul(wr[0], r0) + mul(wr[1], r1) + mul(wr[2], r2), wr[0] + wr[1] + wr[2], ok);
     left = div(mul(wl[0], l0) + mul(wl[1], l1) + mul(wl[2], l2), wl[0] + wl[1] + wl[2], ok);
-    if (SMALL) ok = ok && steep(left) && steep(right);
+    ok = ok && (SMALL ? steep(left) && steep(right) : edge(left) && edge(right));
 }
 
 // ---------------------------------------------------------------------------

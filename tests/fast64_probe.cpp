@@ -197,6 +197,42 @@ extern "C" long probe_faces(long n, u64 seed, int law, int recon, int riemann, i
     RECONS(LAW_MHD_COOL, RIEMANN_HLLE);
 }
 
+// The hydro WENO5 HLLE flux along x of the face between zones 2 and 3 of
+// Z[6][5]: 1 where the lean form took it with other bits, 0 where it took it
+// with the same, -1 where it refused.
+extern "C" int probe_hydro_weno_face(const double* Z, int weno)
+{
+    PhysParams pp;
+    fast64::Consts C;
+    double nrm[3][3];
+    constants(pp, C, nrm, weno, 5.0 / 3, 1.5);
+    double PL[5], PR[5], QL[5], QR[5], x;
+    bool ok = C.ok;
+    for (int q = 0; q < 5; ++q) {
+        double v[6];
+        for (int s = 0; s < 6; ++s) {
+            v[s] = Z[s * 5 + q];
+            ok = ok && fast64::ordinary_field(q, v[s]);
+        }
+        QL[q] = weno5<true>(&v[2], pp.weno_is, pp.shenzha_A);
+        QR[q] = weno5<false>(&v[3], pp.weno_is, pp.shenzha_A);
+        fast64::weno5_edges(C, &v[2], x, PL[q], ok);
+        fast64::weno5_edges(C, &v[3], PR[q], x, ok);
+    }
+    StateD<5> L, R;
+    law_prim<LAW_HYDRO>(pp, QL, nrm[0], L);
+    law_prim<LAW_HYDRO>(pp, QR, nrm[0], R);
+    double H[5];
+    hlle<5>(L, R, H);
+    fast64::Side<5> l, r;
+    fast64::side<LAW_HYDRO, 0>(C, PL, l, ok);
+    fast64::side<LAW_HYDRO, 0>(C, PR, r, ok);
+    bool wrong = false;
+    for (int q = 0; q < 5; ++q)
+        wrong = wrong || !same(H[q], fast64::hlle(l.ap, r.ap, l.am, r.am, l.F[q], r.F[q], l.U[q], r.U[q], ok));
+    return !ok ? -1 : wrong;
+}
+
 template <int LAW>
 static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const double (*nrm)[3], int kind, long* accepted)
 {

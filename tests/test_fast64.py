@@ -81,3 +81,20 @@ def test_two_phase_functions_round_as_the_accurate_ones(lib):
     acc = C.c_long()
     assert lib.probe_ziv(C.c_long(n), C.c_ulonglong(3), C.byref(acc)) == 0
     assert acc.value > 2.9 * n
+
+
+# Density (and pressure) and velocity of five zones of ordinary magnitudes
+# whose WENO5 value at the right edge of the middle one nearly vanishes
+# (2^-153 and 2^-436), so that the density of kinetic energy there is subnormal.
+EDGE_RHO = "0x1.845f67b9a7b48p-99 0x1.8f7b8e6bad8bcp-98 0x1.1ac7f23636d4bp-100 0x1.0e9e382c71194p-100 0x1.cb435c8e74616p-100"
+EDGE_V = "-0x1.49592ff5d47c9p-328 -0x1.8b37d326fefbep-329 -0x1.077a8cc4a9fd4p-330 0x1.077a8cc4a9fd4p-330 0x1.8b37d326fefcp-329"
+
+
+def test_weno_edges_that_nearly_vanish_are_refused_or_right(lib):
+    rho, v = ([float.fromhex(x) for x in line.split()] for line in (EDGE_RHO, EDGE_V))
+    Z = [(rho[min(s, 4)],) + 3 * (v[min(s, 4)],) + (rho[min(s, 4)],) for s in range(6)]
+    flat = (C.c_double * 30)(*[x for z in Z for x in z])
+    assert lib.probe_hydro_weno_face(flat, 2) <= 0
+    # the same zones of magnitude one are taken
+    flat = (C.c_double * 30)(*[x * 2.0 ** (330 if 0 < q < 4 else 100) for z in Z for q, x in enumerate(z)])
+    assert lib.probe_hydro_weno_face(flat, 2) == 0
