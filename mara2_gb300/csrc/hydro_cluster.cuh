@@ -300,9 +300,7 @@ inline cudaError_t cluster1d_config(int cluster_count, int C, int m, cudaStream_
     const size_t smem = cluster1d_smem_bytes(m, G);
     const int threads = m + 1 < 1024 ? ((m + 1 + 31) / 32) * 32 : 1024;  // one thread per face
     auto k = hydro_cluster1d_kernel<RECON, RIEMANN, ACC64>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    if (e == cudaSuccess && C > CLUSTER1D_MAX_CTAS)
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    const cudaError_t e = allow_cluster(k, smem, C > CLUSTER1D_MAX_CTAS);
     if (e != cudaSuccess) return e;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned) C;

@@ -88,6 +88,30 @@ inline void chain_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaSt
     lc.numAttrs = 1;
     cudaLaunchKernelEx(&lc, kernel, std::forward<Args>(args)...);
 }
+
+// Lets a cluster kernel take smem bytes of dynamic shared memory.  The limit
+// belongs to the kernel, which handles of all sizes launch from any thread,
+// so it is only ever raised, and at once to all that the kernel's static
+// arrays leave: a limit of one grid's size, set by another thread between
+// this call and its launch, had refused the larger grid's launch.
+template <typename... KArgs>
+inline cudaError_t allow_cluster(void (*kernel)(KArgs...), size_t smem, bool non_portable)
+{
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess && (size_t) fa.maxDynamicSharedSizeBytes < smem) {
+        int device = 0, most = 0;
+        e = cudaGetDevice(&device);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        if (e != cudaSuccess) return e;
+        const size_t limit = (size_t) most - fa.sharedSizeBytes;
+        if (smem > limit) return cudaErrorInvalidValue;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) limit);
+    }
+    if (e == cudaSuccess && non_portable)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
 #endif
 
 // ---- plain FP64 path (plain_*.cu) --------------------------------------------

@@ -310,8 +310,7 @@ static cudaError_t plain_cluster_config(int n, int ctas, cudaStream_t s, cudaLau
     const int m = (n + ctas - 1) / ctas;
     const size_t smem = sizeof(double) * plain_cluster_doubles(m, ReconInfo<RECON>::S);
     auto k = plain_cluster_kernel<RECON, RIEMANN>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    if (e == cudaSuccess && ctas > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    const cudaError_t e = allow_cluster(k, smem, ctas > 8);
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned) ctas;
     at[0].val.clusterDim.y = 1;
