@@ -51,7 +51,7 @@ F64_FN u32 expo(double x) { return (u32) (bits(x) >> 52) & 0x7ffu; }
 // below form without a check stay normal: the smallest is rho v v above 2^-974,
 // its v_n along y a difference of two such values.  PLM gives no smaller
 // edges (the last place of 2^-331); WENO's weighted sum cancels a second time,
-// down to 2^-436 found, so weno5_edges checks (edge()).
+// down to 2^-436 found, so weno5_edges checks (EDGE).
 F64_FN bool ordinary_pos(double x) { return (u32) (bits(x) >> 32) - (923u << 20) <= (200u << 20); }
 F64_FN bool ordinary(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (693u << 20) <= (430u << 20) || is_zero(x); }
 // field q of a primitive (or conserved: density and energy) state
@@ -64,15 +64,15 @@ F64_FN bool ordinary_field(int q, double x) { return q == 0 || q == 4 ? ordinary
 // the lean ones, and rmhd_roots_certain's second point, 321.
 // Only the product with y's normal is formed without a check; its factors are
 // steep() or zero.
-F64_FN bool steep(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) >= (68u << 20) || is_zero(x); }   // 2^-955
+constexpr int STEEP = 68;   // exponent field of 2^-955
+F64_FN bool steep(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) >= (u32) STEEP << 20 || is_zero(x); }
 template <int LAW>
 F64_FN bool ordinary_field(int q, double x)
 {
     if (LAW != LAW_RMHD || q == 0 || q == 4) return ordinary_field(q, x);
     return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (123u << 20) <= (1000u << 20) || is_zero(x);
 }
-// a reconstructed value of ordinary ones
-F64_FN bool edge(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) >= (640u << 20) || is_zero(x); }
+constexpr int EDGE = 640;   // exponent field of 2^-383
 // a reconstructed density or pressure
 F64_FN bool edge_pos(double x) { return (u32) (bits(x) >> 32) - (869u << 20) <= (256u << 20); }
 
@@ -212,9 +212,11 @@ F64_FN void weno5_edges(const Consts& c, const double* v, double& left, double& 
     const double cp = mul(a56, v[1]), cm = mul(a56, v[-1]), gp = mul(a76, v[1]), gm = mul(a76, v[-1]);
     const double r0 = t0 + cp - sp2, r1 = -sm + c0 + tp, r2 = tm2 - gm + e0;
     const double l0 = e0 - gp + tp2, l1 = tm + c0 - sp, l2 = -sm2 + cm + t0;
-    right = div(mul(wr[0], r0) + mul(wr[1], r1) + mul(wr[2], r2), wr[0] + wr[1] + wr[2], ok);
-    left = div(mul(wl[0], l0) + mul(wl[1], l1) + mul(wl[2], l2), wl[0] + wl[1] + wl[2], ok);
-    ok = ok && (SMALL ? steep(left) && steep(right) : edge(left) && edge(right));
+    // (the quotient's own range check, raised: no edge between zero and what
+    // the functions below assume)
+    constexpr int LOW = SMALL ? STEEP : EDGE;
+    right = div<LOW>(mul(wr[0], r0) + mul(wr[1], r1) + mul(wr[2], r2), wr[0] + wr[1] + wr[2], ok);
+    left = div<LOW>(mul(wl[0], l0) + mul(wl[1], l1) + mul(wl[2], l2), wl[0] + wl[1] + wl[2], ok);
 }
 
 // ---------------------------------------------------------------------------

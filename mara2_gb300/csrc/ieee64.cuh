@@ -165,8 +165,8 @@ IEEE64_FN Divisor divisor(double d, bool& ok)
     return v;
 }
 
-// RN(x / d)
-IEEE64_FN double div(double x, const Divisor& v, bool& ok)
+// RN(x / d).  LOW: a quotient below 2^(LOW - 1023) clears ok.
+template <int LOW = 1> IEEE64_FN double div(double x, const Divisor& v, bool& ok)
 {
     const u64 b = bits(x);
     const u32 xhi = (u32) (b >> 32);
@@ -177,7 +177,7 @@ IEEE64_FN double div(double x, const Divisor& v, bool& ok)
     const bool less = X < v.D;
     X <<= less ? 1 : 0;                                    // X / D in [1, 2)
     const int e = (int) ex - (int) ed + 1023 - (less ? 1 : 0);
-    ok = ok && (zero || (ex - 1u < 2046u && (u32) (e - 1) < 2046u));
+    ok = ok && (zero || (ex - 1u < 2046u && (u32) (e - LOW) < 2047u - LOW));
     const u32 q1 = mulhi((u32) (X >> 22), v.R);            // X / D 2^30, at most 9 units low
     const u64 rem = (X << 30) - (u64) q1 * v.D;            // in [0, 9 D), below 2^57
     const u32 q2 = mulhi((u32) (rem >> 25), v.R);          // rem / D 2^27, at most 6 units low
@@ -191,7 +191,7 @@ IEEE64_FN double div(double x, const Divisor& v, bool& ok)
     return from_bits(q | ((u64) sign << 32));
 }
 
-IEEE64_FN double div(double x, double d, bool& ok) { return div(x, divisor(d, ok), ok); }
+template <int LOW = 1> IEEE64_FN double div(double x, double d, bool& ok) { return div<LOW>(x, divisor(d, ok), ok); }
 
 // RN(sqrt(a)) for a >= 0 (zero or normal)
 IEEE64_FN double sqrt_rn(double a, bool& ok)
