@@ -56,20 +56,25 @@ F64_FN bool ordinary_pos(double x) { return (u32) (bits(x) >> 32) - (923u << 20)
 F64_FN bool ordinary(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (693u << 20) <= (430u << 20) || is_zero(x); }
 // field q of a primitive (or conserved: density and energy) state
 F64_FN bool ordinary_field(int q, double x) { return q == 0 || q == 4 ? ordinary_pos(x) : ordinary(x); }
-// The relativistic forms multiply with FP64 instructions, which underflow as
-// the general forms do, so they take fields down to 2^-900: in a medium at
-// rest ahead of a wave, WENO leaves transverse fields of 1e-200 to 1e-99
-// behind for good (blast 512^2 after 43 steps: in a third of the zones).
-// Their faces and zones went to the general functions: 45 steps 631 ms; with
-// the lean ones, and rmhd_roots_certain's second point, 321.
-// Only the product with y's normal is formed without a check; its factors are
-// steep() or zero.
+// Ahead of a wave into a medium at rest, transverse fields fall by orders of
+// magnitude from zone to zone and stay behind for good, at 1e-99 to 1e-270
+// (magnetic laws, field along x or y: the transverse field in 49 % of the zones
+// of 256^2 after 40 steps with WENO5 and 39 % with PLM, a velocity in 37 % of
+// 64^3 after 20; in a third of a relativistic blast 512^2 after 43; never in
+// hydro).  The magnetic laws take fields down to 2^-900 for it.  Relativistic
+// forms multiply with FP64 instructions, which underflow as the general forms
+// do; mhd_side does so where an operand is below 2^-330 (SMALL), p2u, cons and
+// fastest use mul_any and times_pow2.  Products without a check remain with y's
+// normal, whose factors are steep() or zero, and with pressures.  Against the
+// general functions for these zones: relativistic blast, 45 steps, 631 -> 321 ms
+// (with rmhd_roots_certain's second point); hot region in MHD at rest, 64^3 PLM,
+// 6 steps, 16.7 -> 7.0 ms, 256^2 WENO5, 20 steps, 43.8 -> 17.1.
 constexpr int STEEP = 68;   // exponent field of 2^-955
 F64_FN bool steep(double x) { return ((u32) (bits(x) >> 32) & 0x7fffffffu) >= (u32) STEEP << 20 || is_zero(x); }
 template <int LAW>
 F64_FN bool ordinary_field(int q, double x)
 {
-    if (LAW != LAW_RMHD || q == 0 || q == 4) return ordinary_field(q, x);
+    if (LAW == LAW_HYDRO || q == 0 || q == 4) return ordinary_field(q, x);
     return ((u32) (bits(x) >> 32) & 0x7fffffffu) - (123u << 20) <= (1000u << 20) || is_zero(x);
 }
 constexpr int EDGE = 640;   // exponent field of 2^-383
@@ -86,6 +91,33 @@ F64_FN double scale(double x, int k)
     return is_zero(x) ? x : from_bits(bits(x) + ((u64) (ieee64::i64) k << 52));
 }
 F64_FN double half(double x) { return scale(x, -1); }
+
+// a b on the FP64 pipe, as a call: predicated in line it would take its slot
+// of the pipe also where no thread needs it
+#if defined(__CUDACC__)
+static __device__ __noinline__ double mul_seldom(double a, double b) { return __dmul_rn(a, b); }
+#else
+static inline double mul_seldom(double a, double b) { return a * b; }
+#endif
+
+// a b for any operands: on the FP64 pipe only where the integer product does
+// not hold
+F64_FN double mul_any(double a, double b)
+{
+    bool ok = true;
+    double r = mul(a, b, ok);
+    if (!ok) r = mul_seldom(a, b);
+    return r;
+}
+
+// x 2^k, -3 <= k <= 1: on the exponent where x and the result are normal
+F64_FN double times_pow2(double x, int k)
+{
+    const u32 e = expo(x);
+    if (e - 1u < 2046u && e + (u32) k - 1u < 2046u) return from_bits(bits(x) + ((u64) (ieee64::i64) k << 52));
+    if (is_zero(x)) return x;
+    return mul_seldom(x, k == 1 ? 2.0 : k == -1 ? 0.5 : k == -2 ? 0.25 : 0.125);
+}
 
 // x + z for a zero z of the given sign: x, or the zero the addition gives
 F64_FN double add_zero(double x, bool z_negative)
@@ -282,8 +314,12 @@ F64_FN void hydro_side(const Consts& c, const double* P, Side<5>& S, bool& ok)
     S.am = clamp_neg(vn - cs);
 }
 
-// mhd_prim; an auxiliary field (index 8) is carried without a flux
-template <int AXIS, int NQ>
+// mhd_prim; an auxiliary field (index 8) is carried without a flux.  SMALL:
+// from fields whose products may underflow.
+template <bool SMALL> F64_FN double prod(double a, double b) { return SMALL ? a * b : mul(a, b); }
+template <bool SMALL> F64_FN double halved(double x) { return SMALL ? 0.5 * x : half(x); }
+
+template <int AXIS, bool SMALL, int NQ>
 F64_FN void mhd_side(const Consts& c, const double* P, Side<NQ>& S, bool& ok)
 {
     ok = ok && edge_pos(P[0]) && edge_pos(P[4]);
@@ -294,34 +330,34 @@ F64_FN void mhd_side(const Consts& c, const double* P, Side<NQ>& S, bool& ok)
     const double Bv = dot(P[5], P[6], P[7], P[1], P[2], P[3]);
     const double vn = along<AXIS>(c, P[1], P[2], P[3]);
     const double Bn = along<AXIS>(c, P[5], P[6], P[7]);
-    const double ps = P[4] + half(BB);
+    const double ps = P[4] + halved<SMALL>(BB);
     S.vn = vn;
     S.U[0] = P[0];
 #pragma unroll
-    for (int d = 1; d < 4; ++d) S.U[d] = mul(P[0], P[d]);
-    S.U[4] = half(mul(P[0], vv)) + half(BB) + div(P[4], c.gm1_div, ok);
+    for (int d = 1; d < 4; ++d) S.U[d] = prod<SMALL>(P[0], P[d]);
+    S.U[4] = halved<SMALL>(prod<SMALL>(P[0], vv)) + halved<SMALL>(BB) + div(P[4], c.gm1_div, ok);
 #pragma unroll
     for (int d = 5; d < NQ; ++d) S.U[d] = P[d];
-    S.F[0] = times_along<AXIS>(vn, S.U[0], S.U[1 + AXIS]);
+    S.F[0] = SMALL ? vn * S.U[0] : times_along<AXIS>(vn, S.U[0], S.U[1 + AXIS]);
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-        S.F[1 + d] = add_normal<AXIS>(c, d, mul(vn, S.U[1 + d]) - mul(Bn, P[5 + d]), ps);
-    S.F[4] = mul(vn, S.U[4]) - Bn * Bv + mul(ps, vn);
+        S.F[1 + d] = add_normal<AXIS>(c, d, prod<SMALL>(vn, S.U[1 + d]) - prod<SMALL>(Bn, P[5 + d]), ps);
+    S.F[4] = prod<SMALL>(vn, S.U[4]) - Bn * Bv + prod<SMALL>(ps, vn);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        if (AXIS != 1 && d == AXIS) {
+        if (!SMALL && AXIS != 1 && d == AXIS) {
             // v_n B_n - B_n v_n: +0, or the difference of two zeros
             const bool zero = is_zero(vn) || is_zero(Bn);
             const bool p = sign_bit(vn) != sign_bit(P[5 + d]), q = sign_bit(Bn) != sign_bit(P[1 + d]);
             S.F[5 + d] = from_bits(zero && p && !q ? SIGN : 0ull);
         } else {
-            S.F[5 + d] = mul(vn, S.U[5 + d]) - mul(Bn, P[1 + d]);
+            S.F[5 + d] = prod<SMALL>(vn, S.U[5 + d]) - prod<SMALL>(Bn, P[1 + d]);
         }
     }
     if constexpr (NQ > 8) S.F[8] = 0.0;
     // the fast speed; an Alfven speed that rounding puts above it wins
     const double ca2 = div(BB, rho, ok);
-    const double cn2 = div(mul(Bn, Bn), rho, ok);
+    const double cn2 = div(prod<SMALL>(Bn, Bn), rho, ok);
     const double s = cs2 + ca2;
     const double cF2 = half(s + sqrt_rn(mul(s, s) - scale(cs2, 2) * cn2, ok));
     const double cf = sqrt_rn(max_pos(cF2, cn2), ok);
@@ -329,11 +365,11 @@ F64_FN void mhd_side(const Consts& c, const double* P, Side<NQ>& S, bool& ok)
     S.am = clamp_neg(vn - cf);
 }
 
-template <int LAW, int AXIS>
+template <int LAW, int AXIS, bool SMALL = false>
 F64_FN void side(const Consts& c, const double* P, Side<LawInfo<LAW>::NQ>& S, bool& ok)
 {
     if constexpr (LAW == LAW_HYDRO) hydro_side<AXIS>(c, P, S, ok);
-    else mhd_side<AXIS, LawInfo<LAW>::NQ>(c, P, S, ok);
+    else mhd_side<AXIS, SMALL>(c, P, S, ok);
 }
 
 // ---------------------------------------------------------------------------
@@ -384,9 +420,10 @@ F64_FN void cons(const Consts& c, const double* U, double* P, bool& ok)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     const Divisor rho = ieee64::divisor(U[0], ok);
-    double e = U[4] - div(half(dot(U[1], U[2], U[3], U[1], U[2], U[3])), rho, ok);
+    const double pp = dot(U[1], U[2], U[3], U[1], U[2], U[3]);
+    double e = U[4] - div(LAW == LAW_HYDRO ? half(pp) : times_pow2(pp, -1), rho, ok);
     if constexpr (LAW != LAW_HYDRO) {
-        e = e - half(dot(U[5], U[6], U[7], U[5], U[6], U[7]));
+        e = e - times_pow2(dot(U[5], U[6], U[7], U[5], U[6], U[7]), -1);
 #pragma unroll
         for (int q = 5; q < NQ; ++q) P[q] = U[q];
         ok = ok && !sign_bit(e);
@@ -402,12 +439,17 @@ template <int LAW>
 F64_FN void p2u(const Consts& c, const double* P, double* U, bool& ok)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
+    const double vv = dot(P[1], P[2], P[3], P[1], P[2], P[3]);
+    double e;
     U[0] = P[0];
+    if constexpr (LAW == LAW_HYDRO) {
 #pragma unroll
-    for (int d = 1; d < 4; ++d) U[d] = mul(P[0], P[d]);
-    double e = half(mul(P[0], dot(P[1], P[2], P[3], P[1], P[2], P[3])));
-    if constexpr (LAW != LAW_HYDRO) {
-        e = e + half(dot(P[5], P[6], P[7], P[5], P[6], P[7]));
+        for (int d = 1; d < 4; ++d) U[d] = mul(P[0], P[d]);
+        e = half(mul(P[0], vv));
+    } else {
+#pragma unroll
+        for (int d = 1; d < 4; ++d) U[d] = mul_any(P[0], P[d]);
+        e = times_pow2(mul_any(P[0], vv), -1) + times_pow2(dot(P[5], P[6], P[7], P[5], P[6], P[7]), -1);
 #pragma unroll
         for (int q = 5; q < NQ; ++q) U[q] = P[q];
     }
@@ -434,30 +476,12 @@ F64_FN double fastest(const Consts& c, const double* P, bool& ok)
         double m = 0.0;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const double cn2 = div(mul(B[a], B[a], ok), rho, ok);
+            const double cn2 = div(mul_any(B[a], B[a]), rho, ok);
             const double cF2 = half(s + sqrt_rn(s2 - scale(cs2, 2) * cn2, ok));
             m = max_pos(m, from_bits(mag(v[a])) + sqrt_rn(max_pos(cF2, cn2), ok));
         }
         return m;
     }
-}
-
-// a b on the FP64 pipe, as a call: predicated in line it would take its slot
-// of the pipe also where no thread needs it
-#if defined(__CUDACC__)
-static __device__ __noinline__ double mul_seldom(double a, double b) { return __dmul_rn(a, b); }
-#else
-static inline double mul_seldom(double a, double b) { return a * b; }
-#endif
-
-// a b for any operands: on the FP64 pipe only where the integer product does
-// not hold
-F64_FN double mul_any(double a, double b)
-{
-    bool ok = true;
-    double r = mul(a, b, ok);
-    if (!ok) r = mul_seldom(a, b);
-    return r;
 }
 
 } // namespace fast64

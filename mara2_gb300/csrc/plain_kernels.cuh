@@ -39,6 +39,8 @@
 
 namespace mara {
 
+using fast64::times_pow2;
+
 template <int RECON> struct ReconInfo;
 template <> struct ReconInfo<RECON_PCM> { static constexpr int S = 1; };
 template <> struct ReconInfo<RECON_PLM> { static constexpr int S = 2; };
@@ -147,19 +149,29 @@ static __device__ __noinline__ void weno5_edges_small(const fast64::Consts& C, c
     fast64::weno5_edges<true>(C, &w[2], left, right, *ok);
 }
 
+template <int LAW> constexpr bool NEWTONIAN_MHD = LAW == LAW_MHD || LAW == LAW_MHD_COOL;
+
+// whether zone_edges takes a field: for Newtonian MHD only large ones, small
+// ones are left to odd_sides
+template <int LAW> __device__ __forceinline__ bool lean_field(int q, double x)
+{
+    if constexpr (LAW == LAW_RMHD) return fast64::ordinary_field<LAW>(q, x);
+    else return fast64::ordinary_field(q, x);
+}
+
 template <int LAW, int RECON>
 __device__ __forceinline__ void zone_edges(const fast64::Consts& C, const double* p, long long s, int q, double& left,
                                            double& right, bool& ok)
 {
     if constexpr (RECON == RECON_PCM) {
         left = right = p[0];
-        ok = ok && fast64::ordinary_field<LAW>(q, p[0]);
+        ok = ok && lean_field<LAW>(q, p[0]);
     } else if constexpr (RECON == RECON_PLM) {
         const double l = p[-s], c = p[0], r = p[s];
         const double h = fast64::half_slope(fast64::mul(C.theta, c - l), r - l, fast64::mul(C.theta, r - c));
         left = c - h;
         right = c + h;
-        ok = ok && fast64::ordinary_field<LAW>(q, l) && fast64::ordinary_field<LAW>(q, c) && fast64::ordinary_field<LAW>(q, r);
+        ok = ok && lean_field<LAW>(q, l) && lean_field<LAW>(q, c) && lean_field<LAW>(q, r);
     } else {
         const double w[5] = {p[-2 * s], p[-s], p[0], p[s], p[2 * s]};
 #pragma unroll
@@ -176,20 +188,74 @@ __device__ __forceinline__ void zone_edges(const fast64::Consts& C, const double
     }
 }
 
-template <int LAW, int AXIS>
-__device__ __forceinline__ void face_side(const fast64::Consts& C, const double* P, fast64::Side<LawInfo<LAW>::NQ>& S,
-                                          bool& ok)
-{
-    if constexpr (LAW == LAW_RMHD) fast64::rmhd_side<AXIS>(C, P, S, ok);
-    else fast64::side<LAW, AXIS>(C, P, S, ok);
-}
-
 // a block's shared memory
 template <int NQ> struct TileShared {
     double edge[2][NQ][TILE_ZONES];           // left and right edge of each zone
     double U[2][NQ][TILE_FACES], F[2][NQ][TILE_FACES], A[2][2][TILE_FACES];   // states by side; ap, am
     unsigned char odd_zone[TILE_ZONES], odd_face[TILE_FACES];                 // operands out of the ordinary
+    alignas(4) unsigned char odd_field[NQ][TILE_ZONES];                       // Newtonian MHD: the zone's fields not taken by zone_edges
 };
+
+// the state on side s of face f, from zone z's edge
+template <int LAW, int AXIS, bool SMALL>
+__device__ __forceinline__ void face_side(const fast64::Consts& C, TileShared<LawInfo<LAW>::NQ>& sm, int s, int f, int z)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ;
+    double P[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) P[q] = sm.edge[1 - s][q][z];
+    fast64::Side<NQ> S;
+    bool ok = C.ok && !sm.odd_zone[z];
+    if constexpr (LAW == LAW_RMHD) fast64::rmhd_side<AXIS>(C, P, S, ok);
+    else fast64::side<LAW, AXIS, SMALL>(C, P, S, ok);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        sm.U[s][q][f] = S.U[q];
+        sm.F[s][q][f] = S.F[q];
+    }
+    sm.A[s][0][f] = S.ap;
+    sm.A[s][1][f] = S.am;
+    if (!ok) sm.odd_face[f] = 1;
+}
+// The states of a tile of Newtonian MHD with fields that zone_edges did not
+// take: their edges first, then the states, all by the SMALL form (of two forms
+// a warp would run both).
+// As a call for the whole block, so that other tiles do not pay for it: with a
+// call and a branch per item they took 1 to 2 % longer, with the flags as bits
+// set by atomics 1 %.
+template <int LAW, int RECON, int AXIS>
+__device__ __noinline__ void odd_sides(const fast64::Consts& C, TileShared<LawInfo<LAW>::NQ>& sm, const double* p,
+                                       long long sP, long long stride, long long cstride, int faces, int width)
+{
+    constexpr int NQ = LawInfo<LAW>::NQ, WIDTH = AXIS == 0 ? 1 : 4;
+    constexpr int S = ReconInfo<RECON>::S - 1;   // zones on either side
+    const int zones = faces + WIDTH;
+    for (int it = threadIdx.x; it < NQ * zones; it += TILE_THREADS) {
+        const int q = it / zones, z = it - q * zones;
+        if (!sm.odd_field[q][z]) continue;
+        const double* v = p + q * sP + (z / WIDTH - 1) * stride + z % WIDTH * cstride;
+        bool ok = true;
+        for (int m = -S; m <= S; ++m) ok = ok && fast64::ordinary_field<LAW>(q, v[m * stride]);
+        double left = v[0], right = v[0];
+        if constexpr (RECON == RECON_PLM) {
+            const double l = v[-stride], r = v[stride];
+            const double h = fast64::half_slope(fast64::mul(C.theta, left - l), r - l, fast64::mul(C.theta, r - left));
+            left -= h;
+            right += h;
+        } else if constexpr (RECON == RECON_WENO5) {
+            if (ok) weno5_edges_small(C, v, stride, left, right, &ok);
+        }
+        sm.edge[0][q][z] = left;
+        sm.edge[1][q][z] = right;
+        if (!ok) sm.odd_zone[z] = 1;
+    }
+    __syncthreads();
+    const int tid = threadIdx.x;
+    if (tid < 2 * faces && tid % WIDTH < width) {
+        const int s = tid >= faces ? 1 : 0, f = tid - s * faces, z = f + s * WIDTH;
+        face_side<LAW, AXIS, true>(C, sm, s, f, z);
+    }
+}
 
 // tile b of the faces along AXIS
 template <int LAW, int RECON, int RIEMANN, int AXIS>
@@ -211,6 +277,7 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
     const long long s0 = 1, s1 = G.N[0], s2 = (long long) G.N[0] * G.N[1];
     const long long stride = AXIS == 0 ? s0 : AXIS == 1 ? s1 : s2, cstride = AXIS == 0 ? s1 : s0;
     const double* p = P + ((long long) k * G.N[1] + j) * G.N[0] + i;   // cell on the right of the tile's first face
+    bool odd = false;
     for (int q = 0, z = tid; q < NQ; z += TILE_THREADS) {
         for (; z >= zones && q < NQ; z -= zones) ++q;
         const int s = z / WIDTH, w = z % WIDTH;
@@ -221,25 +288,17 @@ __device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, cons
         zone_edges<LAW, RECON>(C, p + q * G.sP + (s - 1) * stride + w * cstride, stride, q, l, r, ok);
         sm.edge[0][q][z] = l;
         sm.edge[1][q][z] = r;
-        if (!ok) sm.odd_zone[z] = 1;
-    }
-    __syncthreads();
-    if (tid < 2 * faces && tid % WIDTH < width) {
-        const int s = tid >= faces ? 1 : 0, f = tid - s * faces, z = f + s * WIDTH;
-        double Ps[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) Ps[q] = sm.edge[1 - s][q][z];
-        fast64::Side<NQ> S;
-        bool ok = C.ok && !sm.odd_zone[z];
-        face_side<LAW, AXIS>(C, Ps, S, ok);
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            sm.U[s][q][f] = S.U[q];
-            sm.F[s][q][f] = S.F[q];
+        if (!ok) {
+            if constexpr (NEWTONIAN_MHD<LAW>) sm.odd_field[q][z] = 1;
+            else sm.odd_zone[z] = 1;
+            odd = true;
         }
-        sm.A[s][0][f] = S.ap;
-        sm.A[s][1][f] = S.am;
-        if (!ok) sm.odd_face[f] = 1;
+    }
+    if (__syncthreads_or(odd) && NEWTONIAN_MHD<LAW>) {
+        odd_sides<LAW, RECON, AXIS>(C, sm, p, G.sP, stride, cstride, faces, width);
+    } else if (tid < 2 * faces && tid % WIDTH < width) {
+        const int s = tid >= faces ? 1 : 0, f = tid - s * faces;
+        face_side<LAW, AXIS, false>(C, sm, s, f, f + s * WIDTH);
     }
     __syncthreads();
     const long long f0 = 1, f1 = G.N[0] + 1, f2 = (long long) (G.N[0] + 1) * (G.N[1] + 1);
@@ -316,6 +375,8 @@ __global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS)
     __shared__ TileShared<LawInfo<LAW>::NQ> sm;
     const int tid = threadIdx.x;
     for (int z = tid; z < TILE_ZONES; z += TILE_THREADS) sm.odd_zone[z] = 0;
+    if constexpr (NEWTONIAN_MHD<LAW>)
+        for (int w = tid; w < (int) sizeof(sm.odd_field) / 4; w += TILE_THREADS) ((unsigned*) sm.odd_field)[w] = 0;
     if (tid < TILE_FACES) sm.odd_face[tid] = 0;
     const int code = st->code, failures = st->failures;
     if (__syncthreads_or(code != 0 || st->done || failures != 0)) {
@@ -443,16 +504,6 @@ struct FluxView {
         return F[a][q * sF + ((long long) k * M1 + j) * M0 + i];
     }
 };
-
-// x 2^k, on the exponent where x and the result are normal
-__device__ __forceinline__ double times_pow2(double x, int k)
-{
-    const unsigned e = fast64::expo(x);
-    if (e - 1u < 2046u && e + (unsigned) k - 1u < 2046u)
-        return fast64::from_bits(fast64::bits(x) + ((unsigned long long) (long long) k << 52));
-    if (fast64::is_zero(x)) return x;
-    return fast64::mul_seldom(x, k == 1 ? 2.0 : k == -1 ? 0.5 : k == -2 ? 0.25 : 0.125);
-}
 
 // Flux of field q through the face of axis a at flux index (i, j, k), after
 // CellCenteredFieldCT::correctGodunovFluxes when ct is on (magnetic index 5):

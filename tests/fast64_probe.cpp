@@ -66,7 +66,8 @@ static double any()
 
 #ifndef PROBE_IEEE_ONLY
 // A zone's primitives.  kind 0: smooth, 1: zeros and equal values, 2: strong
-// jumps, 3: wide magnitudes, 4: anything, 5: small fields and zeros; hydro
+// jumps, 3: wide magnitudes, 4: anything, 5: small fields and zeros, 6: small
+// magnetic fields and zeros; hydro
 // pressure and density positive for all but kind 4
 static void zone(int law, int kind, int nq, const double* base, double* P)
 {
@@ -76,7 +77,7 @@ static void zone(int law, int kind, int nq, const double* base, double* P)
         if (kind == 0) v = base[q] * (1 + 0.1 * (uni() - 0.5));
         else if (kind == 1) v = pos ? (rnd() & 1 ? 1.0 : base[q]) : rnd() % 4 == 0 ? base[q] : rnd() % 3 == 0 ? -0.0 : 0.0;
         else if (kind == 2) v = pos ? exp(8 * (uni() - 0.5)) : 6 * (uni() - 0.5);
-        else if (kind == 5) v = pos || rnd() % 8 ? base[q] * (1 + 0.1 * (uni() - 0.5)) : 0.0;
+        else if (kind == 5 || kind == 6) v = pos || rnd() % 8 ? base[q] * (1 + 0.1 * (uni() - 0.5)) : 0.0;
         else if (kind == 3) v = pos ? fabs(wide(30)) : wide(rnd() % 8 ? 20 : 320);
         else v = any();
         if (law == LAW_RMHD && kind < 4 && !pos && q < 4) v *= kind == 2 ? 0.16 : 0.5;   // mostly below light speed
@@ -84,10 +85,10 @@ static void zone(int law, int kind, int nq, const double* base, double* P)
     }
 }
 
-// some fields down to 2^-930
-static void shrink(int nq, double* base)
+// some fields (kind 6: from the magnetic ones on) down to 2^-930
+static void shrink(int nq, double* base, int kind)
 {
-    for (int q = 0; q < nq; ++q)
+    for (int q = kind == 6 ? 5 : 0; q < nq; ++q)
         if (q != 0 && q != 4 && rnd() % 2) base[q] *= pow(2.0, -930 * uni());
 }
 
@@ -99,11 +100,11 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
     for (long m = 0; m < n; ++m) {
         double Z[2 * S][NQ], base[NQ];
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
-        if (kind == 5) shrink(NQ, base);
+        if (kind >= 5) shrink(NQ, base, kind);
         for (int s = 0; s < 2 * S; ++s) zone(LAW, kind, NQ, base, Z[s]);
         if (kind == 1 && rnd() % 3 == 0) for (int s = 1; s < 2 * S; ++s) memcpy(Z[s], Z[0], sizeof(Z[0]));
         double PL[NQ], PR[NQ], QL[NQ], QR[NQ];
-        bool ok = C.ok;
+        bool ok = C.ok, all = true;   // all: every field of every zone is large
         for (int q = 0; q < NQ; ++q) {
             double v[2 * S];
             bool strict = true;
@@ -112,6 +113,7 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
                 ok = ok && fast64::ordinary_field<LAW>(q, v[s]);
                 strict = strict && fast64::ordinary_field(q, v[s]);
             }
+            all = all && strict;
             if constexpr (RECON == RECON_PCM) { PL[q] = QL[q] = v[0]; PR[q] = QR[q] = v[1]; }
             else if constexpr (RECON == RECON_PLM) {
                 QL[q] = v[1] + +1.0 * 0.5 * minmod(pp.plm_theta, v[0], v[1], v[2]);
@@ -139,9 +141,12 @@ static long faces(long n, const PhysParams& pp, const fast64::Consts& C, const d
         if constexpr (LAW == LAW_RMHD) {
             fast64::rmhd_side<AXIS>(C, PL, l, ok);
             fast64::rmhd_side<AXIS>(C, PR, r, ok);
-        } else {
+        } else if (all) {
             fast64::side<LAW, AXIS>(C, PL, l, ok);
             fast64::side<LAW, AXIS>(C, PR, r, ok);
+        } else {
+            fast64::side<LAW, AXIS, true>(C, PL, l, ok);
+            fast64::side<LAW, AXIS, true>(C, PR, r, ok);
         }
         if constexpr (RIEMANN == RIEMANN_HLLC) {
             hllc<NQ>(L, R, nrm[AXIS], H);
@@ -241,7 +246,7 @@ static long zones(long n, const PhysParams& pp, const fast64::Consts& C, const d
     for (long m = 0; m < n; ++m) {
         double base[NQ], P[NQ];
         for (int q = 0; q < NQ; ++q) base[q] = q == 0 || q == 4 ? exp(2 * (uni() - 0.5)) : 2 * (uni() - 0.5);
-        if (kind == 5) shrink(NQ, base);
+        if (kind >= 5) shrink(NQ, base, kind);
         zone(LAW, kind, NQ, base, P);
         bool ord = C.ok;
         for (int q = 0; q < NQ; ++q) ord = ord && fast64::ordinary_field<LAW>(q, P[q]);

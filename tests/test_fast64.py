@@ -18,6 +18,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 HYDRO, MHD, RMHD, MHD_COOL = 0, 1, 2, 3
 SMOOTH, ZEROS, JUMPS, WIDE, ANY, SMALL = range(6)
+SMALL_MAGNETIC = 6
 
 
 def _build(path, ulps, *flags):
@@ -98,3 +99,21 @@ def test_weno_edges_that_nearly_vanish_are_refused_or_right(lib):
     # the same zones of magnitude one are taken
     flat = (C.c_double * 30)(*[x * 2.0 ** (330 if 0 < q < 4 else 100) for z in Z for q, x in enumerate(z)])
     assert lib.probe_hydro_weno_face(flat, 2) == 0
+
+
+@pytest.mark.parametrize("kind", [SMALL, SMALL_MAGNETIC])
+@pytest.mark.parametrize("law", [MHD, MHD_COOL])
+@pytest.mark.parametrize("recon", range(3))
+def test_small_fields_of_mhd_take_the_lean_forms(lib, law, recon, kind):
+    """Ahead of a wave into a medium at rest, transverse fields and velocities
+    fall to 1e-270 and stay: the lean forms have to take such faces and zones,
+    with the general bits."""
+    n = 6000
+    acc = C.c_long()
+    for axis in range(3):
+        for weno in (range(3) if recon == 2 else (2,)):
+            assert lib.probe_faces(C.c_long(n), C.c_ulonglong(7 + axis), law, recon, 0, axis, weno, C.c_double(5.0 / 3),
+                                   C.c_double(1.5), kind, C.byref(acc)) == 0
+            assert acc.value > 0.6 * n
+    assert lib.probe_zones(C.c_long(20000), C.c_ulonglong(11), law, C.c_double(5.0 / 3), kind, C.byref(acc)) == 0
+    assert acc.value > 0.6 * 20000

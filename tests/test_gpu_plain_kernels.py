@@ -140,3 +140,37 @@ def test_mixed_general_update_ragged_rows(gpu_lib, port, law, shape, precision):
         out = g.download()
     # the mixed path's contract: 1e-5 of each field's L1 norm
     assert np.all(rel_l1_max(out[s.interior()], ref[s.interior()]) <= 1e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,recon,rk,cooling", [((70, 33, 1), "plm", 2, -1.0), ((33, 40, 1), "weno5", 3, -1.0),
+                                                    ((9, 10, 12), "pcm", 1, -1.0), ((17, 9, 11), "plm", 2, 0.1),
+                                                    ((40, 1, 1), "weno5", 2, -1.0)])
+def test_plain_mhd_in_a_medium_with_small_fields_matches_oracle(gpu_lib, port, shape, recon, rk, cooling):
+    """A hot region in a medium at rest with a field along x, whose transverse
+    fields and velocities are of 1e-100 to 1e-300 (and some subnormal or zero),
+    as a wave leaves them ahead of it."""
+    s = Scheme(law="mhd", recon=recon, riemann="hlle", bc="outflow", rk_order=rk, shape=shape, cfl=0.3,
+               cooling_rate=cooling)
+    rng = np.random.default_rng(sum(shape) + rk)
+    P = W.empty_state(s)
+    Q = np.zeros(shape + (P.shape[-1],))
+    Q[..., 0] = 1.0
+    Q[..., 4] = np.where(rng.random(shape) < 0.1, 10.0, 0.1)
+    Q[..., 5] = 0.5
+    for q in (2, 3, 6, 7):
+        Q[..., q] = 10.0 ** -rng.uniform(100, 300, shape) * rng.choice([-1.0, 1.0], shape)
+        Q[..., q] = np.where(rng.random(shape) < 0.1, rng.choice([0.0, -0.0, 3e-310, 1e-30], shape), Q[..., q])
+    P[s.interior()] = Q
+    P = W.apply_bc_numpy(s, P)
+    ref = P.copy()
+    status, _, dts = port.run(oracle_config(s), ref, 3, s.cfl, s.t_final)
+    assert status == 0
+    with Solver(s, "fp64") as g:
+        g.upload(P.copy())
+        for dt in dts:
+            assert s.cfl * g.courant() == dt
+            g.advance(dt)
+        g.synchronize()
+        out = g.download()
+    assert np.array_equal(out[s.interior()].view(np.uint64), ref[s.interior()].view(np.uint64))
