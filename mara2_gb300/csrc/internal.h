@@ -115,10 +115,11 @@ inline cudaError_t allow_cluster(void (*kernel)(KArgs...), size_t smem, bool non
 #endif
 
 // ---- plain FP64 path (plain_*.cu) --------------------------------------------
-// the face fluxes of every fleshed axis (F[a]), and its number of launches
+// the face fluxes of every fleshed axis (F[a]): the number of launches, and
+// the launches one by one, so that a caller can time each
 int plain_flux_launches(int law, int recon, int riemann, const GridDesc& G);
-void plain_flux(int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& pp, const double* P,
-                double* const* F, DevStatus* st, cudaStream_t s);
+void plain_flux(int launch, int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& pp,
+                const double* P, double* const* F, DevStatus* st, cudaStream_t s);
 void plain_update(int law, const GridDesc& G, const PhysParamsH& pp, const double* Pin, double* Pout,
                   double* U0, double* U, const double* Fx, const double* Fy, const double* Fz,
                   int order, int stage, const double* dt, DevStatus* st, cudaStream_t s,

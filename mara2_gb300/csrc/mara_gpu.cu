@@ -468,12 +468,12 @@ static void enqueue_plain_step(MaraGpuHandle* h)
 {
     const MaraGpuConfig& c = h->cfg;
     for (int rk = 0; rk < c.rk_order; ++rk) {
-        {
+        for (int l = 0; l < plain_flux_launches(kernel_law(&c), c.recon, c.riemann, h->G); ++l) {
             TimedPair tp;
             timed_begin(h, 0, tp);
-            plain_flux(kernel_law(&c), c.recon, c.riemann, h->G, h->pp, h->P[h->cur], h->F, h->st, h->stream);
+            plain_flux(l, kernel_law(&c), c.recon, c.riemann, h->G, h->pp, h->P[h->cur], h->F, h->st, h->stream);
             timed_end(h, tp);
-            h->launches += plain_flux_launches(kernel_law(&h->cfg), h->cfg.recon, h->cfg.riemann, h->G);
+            h->launches++;
         }
         const double* S = nullptr;
         if (h->src_fn) {

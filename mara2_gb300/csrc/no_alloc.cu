@@ -89,7 +89,8 @@ static int noalloc_advance(const MaraGpuConfig* config, const GridDesc& G, size_
     // the RK stages of MethodOfLinesTVD::advance (SolutionSchemes.cpp:191-274)
     int c = 0;
     for (int rk = 0; rk < config->rk_order; ++rk) {
-        plain_flux(law, config->recon, config->riemann, G, pp, P[c], F, st, s);
+        for (int l = 0; l < plain_flux_launches(law, config->recon, config->riemann, G); ++l)
+            plain_flux(l, law, config->recon, config->riemann, G, pp, P[c], F, st, s);
         plain_update(law, G, pp, P[c], P[1 - c], U0, U, F[0], F[1], F[2], config->rk_order, rk, &st->dt, st, s);
         c = 1 - c;
     }

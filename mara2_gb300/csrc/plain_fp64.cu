@@ -17,14 +17,14 @@ int plain_flux_launches(int law, int recon, int riemann, const GridDesc& G)
     return riemann == RIEMANN_HLLC && (law != LAW_HYDRO || runs) ? axes : 1;
 }
 
-void plain_flux(int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& ph, const double* P,
-                double* const* F, DevStatus* st, cudaStream_t s)
+void plain_flux(int launch, int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& ph,
+                const double* P, double* const* F, DevStatus* st, cudaStream_t s)
 {
     switch (law) {
-        case LAW_HYDRO: plain_flux_law<LAW_HYDRO>(recon, riemann, G, ph, P, F, st, s); break;
-        case LAW_MHD: plain_flux_law<LAW_MHD>(recon, riemann, G, ph, P, F, st, s); break;
-        case LAW_MHD_COOL: plain_flux_law<LAW_MHD_COOL>(recon, riemann, G, ph, P, F, st, s); break;
-        default: plain_flux_law<LAW_RMHD>(recon, riemann, G, ph, P, F, st, s); break;
+        case LAW_HYDRO: plain_flux_law<LAW_HYDRO>(launch, recon, riemann, G, ph, P, F, st, s); break;
+        case LAW_MHD: plain_flux_law<LAW_MHD>(launch, recon, riemann, G, ph, P, F, st, s); break;
+        case LAW_MHD_COOL: plain_flux_law<LAW_MHD_COOL>(launch, recon, riemann, G, ph, P, F, st, s); break;
+        default: plain_flux_law<LAW_RMHD>(launch, recon, riemann, G, ph, P, F, st, s); break;
     }
 }
 

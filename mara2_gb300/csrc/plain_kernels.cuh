@@ -799,11 +799,11 @@ static void face_rows(const GridDesc& G, int axis, int* lo, int* nb)
 constexpr long long HLLC_RUN_ZONES = 1ll << 17;
 
 template <int LAW>
-static void flux_runs(const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
+static void flux_runs(int launch, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
                       double* const* F, DevStatus* st, cudaStream_t s)
 {
     for (int axis = 0; axis < 3; ++axis) {
-        if (G.n[axis] <= 1) continue;
+        if (G.n[axis] <= 1 || launch-- != 0) continue;
         RunSpace X;
         face_rows(G, axis, X.lo, X.nb);
         // a run of one forms every zone's slopes twice, one of eight 1/8 too
@@ -824,12 +824,12 @@ static void flux_runs(const GridDesc& G, const PhysParams& pp, const fast64::Con
 }
 
 template <int LAW, int RECON, int RIEMANN>
-static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
+static void flux_launch(int launch, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
                         double* const* F, DevStatus* st, cudaStream_t s)
 {
     if constexpr (RIEMANN == RIEMANN_HLLC && LAW != LAW_HYDRO) {
         for (int axis = 0; axis < 3; ++axis) {
-            if (G.n[axis] <= 1) continue;
+            if (G.n[axis] <= 1 || launch-- != 0) continue;
             FaceSpace X;
             face_rows(G, axis, X.lo, X.nb);
             X.axis = axis;
@@ -841,7 +841,7 @@ static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::C
     } else {
         if constexpr (LAW == LAW_HYDRO && RIEMANN == RIEMANN_HLLC && RECON == RECON_PLM) {
             if ((long long) G.n[0] * G.n[1] * G.n[2] >= HLLC_RUN_ZONES) {
-                flux_runs<LAW>(G, pp, C, P, F, st, s);
+                flux_runs<LAW>(launch, G, pp, C, P, F, st, s);
                 return;
             }
         }
@@ -869,23 +869,23 @@ static void flux_launch(const GridDesc& G, const PhysParams& pp, const fast64::C
 }
 
 template <int LAW, int RECON>
-static void flux_dispatch_r(int riemann, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C,
+static void flux_dispatch_r(int launch, int riemann, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C,
                             const double* P, double* const* F, DevStatus* st, cudaStream_t s)
 {
-    if (riemann == RIEMANN_HLLC) flux_launch<LAW, RECON, RIEMANN_HLLC>(G, pp, C, P, F, st, s);
-    else flux_launch<LAW, RECON, RIEMANN_HLLE>(G, pp, C, P, F, st, s);
+    if (riemann == RIEMANN_HLLC) flux_launch<LAW, RECON, RIEMANN_HLLC>(launch, G, pp, C, P, F, st, s);
+    else flux_launch<LAW, RECON, RIEMANN_HLLE>(launch, G, pp, C, P, F, st, s);
 }
 
 template <int LAW>
-void plain_flux_law(int recon, int riemann, const GridDesc& G, const PhysParamsH& ph, const double* P, double* const* F,
-                    DevStatus* st, cudaStream_t s)
+void plain_flux_law(int launch, int recon, int riemann, const GridDesc& G, const PhysParamsH& ph, const double* P,
+                    double* const* F, DevStatus* st, cudaStream_t s)
 {
     const PhysParams pp = to_dev(ph);
     const fast64::Consts C = to_fast(ph, G);
     switch (recon) {
-        case RECON_PCM: flux_dispatch_r<LAW, RECON_PCM>(riemann, G, pp, C, P, F, st, s); break;
-        case RECON_PLM: flux_dispatch_r<LAW, RECON_PLM>(riemann, G, pp, C, P, F, st, s); break;
-        default: flux_dispatch_r<LAW, RECON_WENO5>(riemann, G, pp, C, P, F, st, s); break;
+        case RECON_PCM: flux_dispatch_r<LAW, RECON_PCM>(launch, riemann, G, pp, C, P, F, st, s); break;
+        case RECON_PLM: flux_dispatch_r<LAW, RECON_PLM>(launch, riemann, G, pp, C, P, F, st, s); break;
+        default: flux_dispatch_r<LAW, RECON_WENO5>(launch, riemann, G, pp, C, P, F, st, s); break;
     }
 }
 
@@ -919,8 +919,8 @@ void plain_courant_law(const GridDesc& G, const PhysParamsH& ph, const double* P
 
 // one translation unit per law instantiates the kernels (plain_*.cu)
 #define MARA_PLAIN_LAW(EXTERN, LAW)                                                                                  \
-    EXTERN template void plain_flux_law<LAW>(int, int, const GridDesc&, const PhysParamsH&, const double*,           \
-                                             double* const*, DevStatus*, cudaStream_t);                                    \
+    EXTERN template void plain_flux_law<LAW>(int, int, int, const GridDesc&, const PhysParamsH&, const double*,      \
+                                             double* const*, DevStatus*, cudaStream_t);                              \
     EXTERN template void plain_update_law<LAW>(const GridDesc&, const PhysParamsH&, const double*, double*, double*, \
                                                double*, const double*, const double*, const double*, int, int,      \
                                                const double*, DevStatus*, cudaStream_t, const double*);             \

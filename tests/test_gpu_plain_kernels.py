@@ -174,3 +174,28 @@ def test_plain_mhd_in_a_medium_with_small_fields_matches_oracle(gpu_lib, port, s
         g.synchronize()
         out = g.download()
     assert np.array_equal(out[s.interior()].view(np.uint64), ref[s.interior()].view(np.uint64))
+
+
+# tiles: one launch of fluxes a stage for all axes; face runs (hydro, PLM, HLLC
+# from 2^17 zones) and magnetic HLLC: one per axis
+@pytest.mark.gpu
+@pytest.mark.parametrize("law,shape,recon,riemann,launches", [("hydro", (40, 30, 1), "plm", "hllc", 1),
+                                                              ("hydro", (400, 400, 1), "plm", "hllc", 2),
+                                                              ("hydro", (60, 50, 50), "plm", "hllc", 3),
+                                                              ("mhd", (8, 9, 10), "pcm", "hllc", 3),
+                                                              ("mhd", (24, 20, 1), "weno5", "hlle", 1)])
+def test_kernel_timing_counts_every_plain_launch(gpu_lib, law, shape, recon, riemann, launches):
+    s, P = _state(law, shape, recon, riemann, "periodic", 2, False)
+    with Solver(s, "fp64") as g:
+        g.upload(P.copy())
+        dt = 0.1 * s.cfl * g.courant()
+        g.set_kernel_timing(True)
+        before = g.stats().kernel_launches
+        g.advance(dt)
+        g.advance(dt)
+        enqueued = g.stats().kernel_launches - before
+        ms, n = g.kernel_times()
+        g.set_kernel_timing(False)
+    assert n[0] == 2 * s.rk_order * launches and n[1] == 2 * s.rk_order, n
+    assert n[0] + n[1] + 4 == enqueued      # and dt and the step count, once a step each
+    assert ms[0] > 0.0 and ms[1] > 0.0
