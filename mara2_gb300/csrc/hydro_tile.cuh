@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(NT, (TileForm<DIM, RECON, TX, TY, NT, ACC64, O
     hydro_tile_kernel(const HGrid* __restrict__ grids, const TileRef* __restrict__ tiles,
                       const int* __restrict__ ntiles_p,
                       const int* __restrict__ rot,  // per grid: state buffer s
-                      const double* __restrict__ dtg, int dt_stride, const int* __restrict__ done, int done_stride,
+                      const double* dtg, int dt_stride, const int* done, int done_stride,
                       int stage, float b, float omb, int last, unsigned long long* __restrict__ cfl, int cfl_stride,
                       int after_begin)
 {

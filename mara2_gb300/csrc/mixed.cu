@@ -57,7 +57,7 @@ struct FaceSpacesF {
 };
 
 template <int LAW, int RECON, int RIEMANN, int AXIS>
-__device__ __forceinline__ void flux_f_face(const float* __restrict__ P, const GridF& G, const FaceSpaceF& X,
+__device__ __forceinline__ void flux_f_face(const float* P, const GridF& G, const FaceSpaceF& X,
                                             DevStatus* st)
 {
     float* __restrict__ F = X.F;
@@ -111,8 +111,8 @@ __device__ __forceinline__ void flux_f_face(const float* __restrict__ P, const G
 // grids run their axes side by side, large ones have one last wave instead
 // of three.
 template <int LAW, int RECON, int RIEMANN>
-__global__ void __launch_bounds__(128) flux_f_kernel(const float* __restrict__ P, const __grid_constant__ FaceSpacesF X,
-                                                     const __grid_constant__ GridF G, const int* __restrict__ done,
+__global__ void __launch_bounds__(128) flux_f_kernel(const float* P, const __grid_constant__ FaceSpacesF X,
+                                                     const __grid_constant__ GridF G, const int* done,
                                                      DevStatus* st)
 {
     pdl_chain();
@@ -135,10 +135,15 @@ struct FluxViewF {
     const float* E[3];   // edge EMFs of the flux CT (pairs x-y, x-z, y-z), or null
     long long sF;
     int M0, M1;
-    template <bool RO = false> __device__ __forceinline__ float at(int a, int q, int i, int j, int k) const
+    // CA: as ld.global.ca, which in the hydro update takes the time of a
+    // read-only load (112x90x75, 16 steps, 2.98 ms; plain loads 3.06, 128^3 7.94
+    // and 8.82), but such a load must not be used here: it promises data that
+    // nothing writes while the kernel exists, and the update is launched while
+    // the fluxes are still being written
+    template <bool CA = false> __device__ __forceinline__ float at(int a, int q, int i, int j, int k) const
     {
         const float* p = F[a] + q * sF + ((long long) k * M1 + j) * M0 + i;
-        if constexpr (RO) return __ldg(p);
+        if constexpr (CA) return __ldca(p);
         else return *p;
     }
     __device__ __forceinline__ float emf(int e, int i, int j, int k) const
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(128) ct_emf_kernel(FluxViewF V, float* E01, fl
 // flux CT of CellCenteredFieldCT::correctGodunovFluxes on one face (FP32):
 // the normal field's flux is zero, a tangential field's the mean of the edge
 // EMFs (ct_emf_kernel) on the face's two edges along the other axis
-template <int NQ, bool RO>
+template <int NQ, bool CA>
 __device__ __forceinline__ float face_flux_f(const FluxViewF& V, const GridF& G, int a, int q, int i, int j, int k)
 {
     if (NQ == 8 && G.ct && q >= 5) {
@@ -194,7 +199,7 @@ __device__ __forceinline__ float face_flux_f(const FluxViewF& V, const GridF& G,
             if (q == B1 && fy) return -0.5f * (V.emf(2, i, j + 1, k) + V.emf(2, i, j, k));
         }
     }
-    return V.template at<RO>(a, q, i, j, k);
+    return V.template at<CA>(a, q, i, j, k);
 }
 
 // The 2-D (Z, W) Newton iteration of ConsToPrimRMHD (rm_anton2dzw, after
@@ -551,8 +556,8 @@ template <int LAW, bool ACC64, bool LINEAR>
 __global__ void __launch_bounds__(128, 8) update_f_kernel(float* __restrict__ Pf, const float* U0h, const float* U0l,
                                                        const float* Uph, const float* Upl, float* Unh, float* Unl,
                                                        FluxViewF V, GridF G,
-                                                       const double* __restrict__ dtp, float b, float omb,
-                                                       const int* __restrict__ done, DevStatus* st,
+                                                       const double* dtp, float b, float omb,
+                                                       const int* done, DevStatus* st,
                                                        unsigned long long* cfl)
 {
     // hydro gains (112x90x75, 16 steps 3.44 -> 3.12 ms; 40^3 to 180^3 0 to 7 %),

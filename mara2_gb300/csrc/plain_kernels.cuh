@@ -100,7 +100,7 @@ struct FaceSpace {
 };
 
 template <int LAW, int RECON, int RIEMANN>
-__global__ void __launch_bounds__(128) flux_general_kernel(const double* __restrict__ P, double* __restrict__ F,
+__global__ void __launch_bounds__(128) flux_general_kernel(const double* P, double* __restrict__ F,
                                                            const __grid_constant__ GridDesc G,
                                                            const __grid_constant__ PhysParams pp,
                                                            const __grid_constant__ FaceSpace X,
@@ -259,7 +259,7 @@ __device__ __noinline__ void odd_sides(const fast64::Consts& C, TileShared<LawIn
 
 // tile b of the faces along AXIS
 template <int LAW, int RECON, int RIEMANN, int AXIS>
-__device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, const double* __restrict__ P,
+__device__ __forceinline__ void flux_tile(TileShared<LawInfo<LAW>::NQ>& sm, const double* P,
                                           double* __restrict__ F, const GridDesc& G, const PhysParams& pp,
                                           const fast64::Consts& C, const TileSpace& X, int b, DevStatus* st)
 {
@@ -367,7 +367,7 @@ struct TileSpaces {
 
 template <int LAW, int RECON, int RIEMANN>
 __global__ void __launch_bounds__(TILE_THREADS, 512 / TILE_THREADS)
-    flux_tile_kernel(const double* __restrict__ P, const __grid_constant__ TileSpaces X,
+    flux_tile_kernel(const double* P, const __grid_constant__ TileSpaces X,
                      const __grid_constant__ GridDesc G, const __grid_constant__ PhysParams pp,
                      const __grid_constant__ fast64::Consts C, DevStatus* __restrict__ st)
 {
@@ -403,7 +403,7 @@ struct RunSpace {
 
 // Three blocks per SM (168 registers): 4, 5 and 6 lose 1, 6 and 11 % to spills.
 template <int AXIS>
-__global__ void __launch_bounds__(128, 3) flux_run_kernel(const double* __restrict__ P, double* __restrict__ F,
+__global__ void __launch_bounds__(128, 3) flux_run_kernel(const double* P, double* __restrict__ F,
                                                           const __grid_constant__ GridDesc G,
                                                           const __grid_constant__ PhysParams pp,
                                                           const __grid_constant__ fast64::Consts C,
@@ -577,14 +577,14 @@ __device__ __forceinline__ double rk_combine_plain(double Uo, double Up, double 
 // Resident blocks: hydro 1 to 5 a SM 5.60 ms, 8 5.39 (KH 1024^2, four steps);
 // MHD 1 3.94, 4 3.66, 5 3.57, 8 3.67 (64x56x48).
 template <int LAW>
-__global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 1 : 5) update_kernel(const double* __restrict__ Pin, double* __restrict__ Pout,
+__global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 1 : 5) update_kernel(const double* Pin, double* __restrict__ Pout,
                                                      double* __restrict__ U0, double* __restrict__ U,
                                                      const __grid_constant__ FluxView V,
                                                      const __grid_constant__ GridDesc G,
                                                      const __grid_constant__ PhysParams pp,
                                                      const __grid_constant__ fast64::Consts C, double fv,
-                                                     const __grid_constant__ RkWeight w, int stage, const double* __restrict__ dtp,
-                                                     DevStatus* __restrict__ st, const double* __restrict__ S)
+                                                     const __grid_constant__ RkWeight w, int stage, const double* dtp,
+                                                     DevStatus* __restrict__ st, const double* S)
 {
     constexpr int NQ = LawInfo<LAW>::NQ;
     pdl_wait();
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(128, LAW == LAW_HYDRO ? 8 : LAW == LAW_RMHD ? 
 // lmin / lambda falls with lambda, also after rounding, so a block divides
 // once, by its largest eigenvalue.
 template <int LAW>
-__global__ void __launch_bounds__(128) courant_kernel(const double* __restrict__ P,
+__global__ void __launch_bounds__(128) courant_kernel(const double* P,
                                                       const __grid_constant__ GridDesc G,
                                                       const __grid_constant__ PhysParams pp,
                                                       const __grid_constant__ fast64::Consts C,
