@@ -801,16 +801,19 @@ __device__ __forceinline__ void store_cell(const float* Uh, const float* Ul, lon
         // from its own start
         bool ok = C->ok;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, U[q]);
+        for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field<LAW>(q, U[q]);
         const long long pc = ((long long) (kk + G.g[2]) * G.N[1] + (jj + G.g[1])) * G.N[0] + (ii + G.g[0]);
         const float rho = Pf[pc], v1 = Pf[G.sP + pc], v2 = Pf[2 * G.sP + pc], v3 = Pf[3 * G.sP + pc], pre = Pf[4 * G.sP + pc];
         const float V2 = v1 * v1 + v2 * v2 + v3 * v3;
         const float W2 = 1.0f / (1.0f - V2), Z = (rho + pre * G.rm_hcoef) * W2;
         ok = ok && V2 < 1.0f && rho > 0.0f && pre > 0.0f && Z > 0.0f && Z < 1e30f;
         fast64::rmhd_newton(*C, U, P, ok, (double) Z, (double) sqrtf(W2));
-        if (!ok) {
-            int code = 0;
-            law_cons<LAW>(pp, U, P, &code);
+        // a zone that cannot be recovered kept its primitives (fromConserved's
+        // closing check of the wave speeds is not made here: a zone that it
+        // refuses is recovered all the same)
+        if (!ok && rmhd_recover(pp, U, P) != ST_OK) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) P[q] = (double) Pf[q * G.sP + pc];
         }
     } else {
         int code = 0;

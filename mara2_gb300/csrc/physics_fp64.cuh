@@ -579,11 +579,9 @@ __device__ __forceinline__ int rm_noble1dw(const C2pRmhd& s, double* P)
     return rm_reconstruct(s, Z, W, P);
 }
 
-// RelativisticMHD::fromConserved (ConservationLaws.cpp:627-657).  *code gets
-// the Newton failure status when both solvers fail; the eigenvalue check of
-// the reference's closing fromPrimitive call is kept (it can raise "bad
-// eigenvalues").
-__device__ __forceinline__ int rmhd_cons(const PhysParams& pp, const double* U, double* P, int* code)
+// The recovery of RelativisticMHD::fromConserved (ConservationLaws.cpp:
+// 627-657): the Newton status if both solvers fail; P is then not written.
+__device__ __forceinline__ int rmhd_recover(const PhysParams& pp, const double* U, double* P)
 {
     C2pRmhd s;
     s.gamf = (pp.gamma - 1.0) / pp.gamma;
@@ -598,9 +596,19 @@ __device__ __forceinline__ int rmhd_cons(const PhysParams& pp, const double* U, 
     for (int q = 0; q < 8; ++q) s.Cons[q] = U[q];
     s.Z_start = sqrt(s.S2 + s.D * s.D);
     s.W_start = s.Z_start / s.D;
+    int err = rm_anton2dzw(s, P);
+    if (err != ST_OK) err = rm_noble1dw(s, P);
+    return err;
+}
+
+// RelativisticMHD::fromConserved.  *code gets the Newton failure status when
+// both solvers fail; the eigenvalue check of the reference's closing
+// fromPrimitive call is kept (it can raise "bad eigenvalues").  P is written
+// only where neither fails.
+__device__ __forceinline__ int rmhd_cons(const PhysParams& pp, const double* U, double* P, int* code)
+{
     double Q[8];
-    int err = rm_anton2dzw(s, Q);
-    if (err != ST_OK) err = rm_noble1dw(s, Q);
+    const int err = rmhd_recover(pp, U, Q);
     if (err != ST_OK) { *code = err; return ST_INVERSION_FAILURE; }
     {
         const double xhat[3] = {1.0, 0.0, 0.0};
