@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(CONV_BLOCK) load_kernel(const double* __restri
                 // (RMHD 512^2 with general functions: 811 us, FP64-bound)
                 bool ok = C.ok;
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field(q, P[q]);
+                for (int q = 0; q < NQ; ++q) ok = ok && fast64::ordinary_field<LAW>(q, P[q]);
                 fast64::rmhd_p2u(C, P, U, ok);
                 if (!ok) {
                     const int e = law_p2u<LAW>(pp, P, U);
