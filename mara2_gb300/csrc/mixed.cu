@@ -1417,19 +1417,18 @@ void mixed_enqueue_step(MixedState* m, const double* dt, DevStatus* st, cudaStre
     if (m->fused && m->cfg.rk_order == 1) m->rot ^= 1;
 }
 
-bool mixed_enqueue_run_step(MixedState* m, double cfl, double t_final, DevStatus* st, cudaStream_t s)
+void mixed_enqueue_run_step(MixedState* m, double cfl, double t_final, DevStatus* st, cudaStream_t s)
 {
     if (!m->fused) {
         chain_launch(k_general_begin, dim3(1), dim3(1), s, (const unsigned long long*) m->dcfl, m->dcfl_next, st, cfl,
                      t_final);
         general_stages(m, &st->dt, st, s);
         chain_launch(k_general_end, dim3(1), dim3(1), s, m->dcfl, (const unsigned long long*) m->dcfl_next, st);
-        return true;
+        return;
     }
     k_fused_run_begin<<<1, 1, 0, s>>>(m->dcfl, st, cfl, t_final);
     fused_step(m, &st->dt, st, s);
     if (m->cfg.rk_order == 1) m->rot ^= 1;
-    return true;
 }
 
 bool mixed_enqueue_advance(MixedState* m, double dt, DevStatus* st, cudaStream_t s)

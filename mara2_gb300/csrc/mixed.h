@@ -20,10 +20,10 @@ void mixed_load_finish(MixedState* m, DevStatus* st, cudaStream_t s);
 void mixed_store_aos_range(MixedState* m, double* aos, long long c0, long long c1, cudaStream_t s);
 void mixed_enqueue_step(MixedState* m, const double* dt, DevStatus* st, cudaStream_t s, int64_t* timed);
 void mixed_enqueue_courant(MixedState* m, DevStatus* st, cudaStream_t s);
-// One whole driver-loop step (dt from the Courant step, stages, clock) or one
-// advance with a given dt, when the fused hydro kernels apply; false (nothing
-// enqueued) otherwise.
-bool mixed_enqueue_run_step(MixedState* m, double cfl, double t_final, DevStatus* st, cudaStream_t s);
+// One whole driver-loop step: dt from the Courant step, stages, clock.  Of one
+// advance with a given dt the same when the fused hydro kernels apply; false
+// (nothing enqueued) otherwise.
+void mixed_enqueue_run_step(MixedState* m, double cfl, double t_final, DevStatus* st, cudaStream_t s);
 bool mixed_enqueue_advance(MixedState* m, double dt, DevStatus* st, cudaStream_t s);
 void mixed_sync_rotation(MixedState* m, cudaStream_t s);
 // one advance of a page-locked host MeshData::P in place (host_dev: its

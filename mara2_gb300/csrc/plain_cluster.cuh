@@ -302,7 +302,11 @@ __global__ void __launch_bounds__(512) plain_cluster_kernel(double* __restrict__
     }
 }
 
-constexpr int PLAIN_CLUSTER_MAX = 4096;   // zones
+// Zones.  A chosen limit, not the shared memory's (16 CTAs hold about 7500) nor
+// where the step kernels catch up: a step on the cluster at 4096 zones and by
+// step kernels at 4097 takes 35.6 and 37.4 us (PLM, HLLE, RK2), 36.1 and 39.4
+// (PLM, HLLC, RK2), but 115 and 83 (WENO5, HLLC, RK3).
+constexpr int PLAIN_CLUSTER_MAX = 4096;
 
 template <int RECON, int RIEMANN>
 static cudaError_t plain_cluster_config(int n, int ctas, cudaStream_t s, cudaLaunchAttribute* at, cudaLaunchConfig_t& lc)

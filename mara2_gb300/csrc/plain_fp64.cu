@@ -13,8 +13,7 @@ int plain_flux_launches(int law, int recon, int riemann, const GridDesc& G)
 {
     int axes = 0;
     for (int a = 0; a < 3; ++a) axes += G.n[a] > 1;
-    const bool runs = law == LAW_HYDRO && recon == RECON_PLM && (long long) G.n[0] * G.n[1] * G.n[2] >= HLLC_RUN_ZONES;
-    return riemann == RIEMANN_HLLC && (law != LAW_HYDRO || runs) ? axes : 1;
+    return in_face_runs(law, recon, riemann, G) || (riemann == RIEMANN_HLLC && law != LAW_HYDRO) ? axes : 1;
 }
 
 void plain_flux(int launch, int law, int recon, int riemann, const GridDesc& G, const PhysParamsH& ph,

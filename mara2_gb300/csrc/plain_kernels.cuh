@@ -797,6 +797,11 @@ static void face_rows(const GridDesc& G, int axis, int* lo, int* nb)
 // 400^2, 8 steps 2.28 and 2.15; 1024^2, 4 steps 6.63 and 5.23; with WENO5 the
 // tiles win at all of them, 640^2 by 7.3 to 11.9)
 constexpr long long HLLC_RUN_ZONES = 1ll << 17;
+inline bool in_face_runs(int law, int recon, int riemann, const GridDesc& G)
+{
+    return law == LAW_HYDRO && recon == RECON_PLM && riemann == RIEMANN_HLLC &&
+           (long long) G.n[0] * G.n[1] * G.n[2] >= HLLC_RUN_ZONES;
+}
 
 template <int LAW>
 static void flux_runs(int launch, const GridDesc& G, const PhysParams& pp, const fast64::Consts& C, const double* P,
@@ -840,7 +845,7 @@ static void flux_launch(int launch, const GridDesc& G, const PhysParams& pp, con
         }
     } else {
         if constexpr (LAW == LAW_HYDRO && RIEMANN == RIEMANN_HLLC && RECON == RECON_PLM) {
-            if ((long long) G.n[0] * G.n[1] * G.n[2] >= HLLC_RUN_ZONES) {
+            if (in_face_runs(LAW, RECON, RIEMANN, G)) {
                 flux_runs<LAW>(launch, G, pp, C, P, F, st, s);
                 return;
             }
