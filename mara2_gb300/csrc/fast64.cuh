@@ -167,8 +167,11 @@ static inline Consts make_consts(double gamma, double theta, double shenzha_A, i
     c.d6 = ieee64::divisor(6.0, c.ok);
     c.d9 = ieee64::divisor(9.0, c.ok);
     c.d27 = ieee64::divisor(27.0, c.ok);
+    // gamma - 1 only divides, or multiplies with a check: nearly isothermal
+    // gases (1.001) would otherwise pay the lean forms and then the general
+    // ones (MHD 192^2, 6 steps, 2.18 ms against 1.75 by the general ones alone)
     const double small = 1e-3, large = 1e3;
-    c.ok = c.ok && gamma > small && gamma < large && c.gm1 > small && theta > small && theta < large &&
+    c.ok = c.ok && gamma < large && c.gm1 > 1e-8 && (theta == 0.0 || theta > small) && theta < large &&
            shenzha_A >= 0.0 && shenzha_A < 1e9 && ny0 > 1e-20 && ny0 < small;
     return c;
 }

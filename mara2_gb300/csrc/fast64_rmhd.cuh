@@ -224,7 +224,7 @@ F64_FN bool rmhd_roots_certain(const Consts& c, const double* P)
     const float BB = p[5] * p[5] + p[6] * p[6] + p[7] * p[7], Bv = p[5] * p[1] + p[6] * p[2] + p[7] * p[3];
     if (!(vv < 0.999f)) return false;
     const float W2 = 1.0f / (1.0f - vv), W = sqrtf(W2), b0 = W * Bv, bb = BB / W2 + Bv * Bv, bn = p[5] / W + b0 * p[1];
-    const float rh = p[0] + p[4] * (g / (g - 1.0f)), cs2 = g * p[4] / rh, v = p[1];
+    const float rh = p[0] + p[4] / (float) c.gamf, cs2 = g * p[4] / rh, v = p[1];
     if (BB == 0.0f) return P[5] == 0.0 && P[6] == 0.0 && P[7] == 0.0;   // no quartic then
     const float K = W2 * W2 * rh * (1.0f / cs2 - 1.0f), L = -W2 * (rh + bb / cs2);
     const float y0 = b0 * v - bn, d1 = sqrtf(-L * (1.0f - v * v) / (2.0f * K));

@@ -117,3 +117,25 @@ def test_small_fields_of_mhd_take_the_lean_forms(lib, law, recon, kind):
             assert acc.value > 0.6 * n
     assert lib.probe_zones(C.c_long(20000), C.c_ulonglong(11), law, C.c_double(5.0 / 3), kind, C.byref(acc)) == 0
     assert acc.value > 0.6 * 20000
+
+
+@pytest.mark.parametrize("law", [HYDRO, MHD, RMHD, MHD_COOL])
+@pytest.mark.parametrize("gamma,theta", [(1.001, 1.5), (1.0 + 1e-6, 2.0), (5.0 / 3, 0.0)])
+def test_nearly_isothermal_gases_and_unlimited_slopes_take_the_lean_forms(lib, law, gamma, theta):
+    n = 3000
+    acc = C.c_long()
+    # (the relativistic law loses a third of these states' wave speeds to
+    # rounding at gamma - 1 = 1e-6, by the general functions too)
+    most = 0.9 if law != RMHD or gamma > 1.0001 else 0.0
+    for recon in range(3):
+        for axis in range(3):
+            for kind in (SMOOTH, ZEROS, JUMPS, WIDE, ANY):
+                for riemann in ((0, 1) if law == HYDRO else (0,)):
+                    assert lib.probe_faces(C.c_long(n), C.c_ulonglong(50 * kind + axis), law, recon, riemann, axis, 2,
+                                           C.c_double(gamma), C.c_double(theta), kind, C.byref(acc)) == 0
+                    if kind == SMOOTH:
+                        assert acc.value > most * n
+    for kind in (SMOOTH, JUMPS, WIDE, ANY):
+        assert lib.probe_zones(C.c_long(10000), C.c_ulonglong(kind), law, C.c_double(gamma), kind, C.byref(acc)) == 0
+        if kind == SMOOTH:
+            assert acc.value > most * 10000
