@@ -215,6 +215,10 @@ F64_FN void rmhd_side(const Consts& c, const double* P, Side<8>& S, bool& ok)
 // not to drown in FP64's rounding of the quartic.  With the first point alone
 // nearly every zone of such a medium needed its roots (mixed 512^2 blast,
 // 16 steps 4.19 -> 4.09 ms; plain 160x131, 2 steps 1.64 -> 1.44).
+// The thousandth covers the rounding of value and terms (1.2e-4 of the terms at
+// most in 32 M random states); of 96 M states with v^2 up to 0.999, p / rho of
+// 1e-6 to 1e4 and gamma of 1.0001 to 5/3, the general functions refused none
+// of the 70 % certified here.
 F64_FN bool rmhd_roots_certain(const Consts& c, const double* P)
 {
     float p[8];
